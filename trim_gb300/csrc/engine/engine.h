@@ -438,7 +438,12 @@ void launch_tc_slices(int ns, const TcSector* secs, int nsec, const int64_t* a_t
                       const int64_t* b_ts, int64_t b_tiles, const double* A, const double* B,
                       const unsigned long long* amax, const unsigned long long* bmax, uint8_t* images, int num_sms,
                       cudaStream_t s);
-size_t tc_gemm_smem(int ns);
+// the fast modes' GEMM (ns = 1: BF16, 2: TF32) and the split mode's, on images
+// of kSplitDigits digits per operand tile (part: FP64 partial tiles of K-split sectors)
+constexpr int kSplitDigits = 6;
+void launch_tc_gemm_split(const TcSector* secs, const int4* items, int nitems, const uint8_t* ws,
+                          const unsigned long long* ea, const unsigned long long* eb, double* C, double* part,
+                          int* err, int grid, cudaStream_t s);
 void launch_tc_gemm(int ns, const TcSector* secs, const int4* items, int nitems, const uint8_t* ws,
                     const unsigned long long* ea, const unsigned long long* eb, double* C, double* part, int* err,
                     int grid, cudaStream_t s);

@@ -390,8 +390,8 @@ static GemmRoute static_route(const Ctx& ctx, int mode, const std::vector<tn_sec
   return GemmRoute::Tiled;
 }
 
-// digit images per 64-k operand tile: 7 slices (split), one BF16 slice, or
-// the two 128-byte halves of a TF32 tile
+// digit images per 64-k operand tile: 7 slices (split, fused form), one BF16
+// slice, or the two 128-byte halves of a TF32 tile
 static int mode_ns(int mode) {
   const int m = mode & ~kModeFlags;
   return m == TN_MODE_SPLIT ? 7 : (m == TN_MODE_FAST_TF32 ? 2 : 1);
@@ -560,7 +560,7 @@ void run_sector_gemms(Ctx& ctx, int mode, const std::vector<tn_sector_gemm>& lis
     std::vector<tn_sector_gemm> tc, f64;
     for (const auto& g : list) (!tc_only && thin_sector(g) ? f64 : tc).push_back(g);
     if (!f64.empty()) run_fp64(ctx, f64, A, B, C);
-    if (!tc.empty()) run_tc_gemms(ctx, ns, tc, A, B, C);
+    if (!tc.empty()) run_tc_gemms(ctx, ns == 7 ? kSplitDigits : ns, tc, A, B, C);
   };
   const GemmRoute route = tune_route(
       ctx, mode, list, [&] { run_tc_fused(ctx, ns, list, A, B, C); }, [&] { run_fp64(ctx, list, A, B, C); }, &tiled);

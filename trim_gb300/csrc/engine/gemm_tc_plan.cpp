@@ -13,13 +13,13 @@ namespace tn {
 
 namespace {
 constexpr int kTM = 128, kTN = 64, kTK = 64;
-constexpr int kChunkTiles = 9;  // 64-k tiles per exact-accumulation chunk of the split kernel
+constexpr int kChunkTiles = 9;  // 64-k tiles of the shortest K range of a split sector
 int64_t cdiv(int64_t a, int64_t b) { return (a + b - 1) / b; }
 }  // namespace
 
 struct TcPlan {
   std::vector<tn_sector_gemm> list;
-  int ns = 7;
+  int ns = kSplitDigits;
   DevBufP meta;
   size_t off_secs = 0, off_rb = 0, off_cb = 0, off_at = 0, off_bt = 0, off_it = 0, off_rit = 0;
   int nsec = 0, nitems = 0, nred = 0;
@@ -85,8 +85,8 @@ static std::shared_ptr<TcPlan> build_tc_plan(Ctx& ctx, const std::vector<tn_sect
     P->in_bytes += 8.0 * ((double)g.M * g.K + (double)g.K * g.N);
   }
   // K split: with fewer than two output tiles per SM, long-K sectors are cut
-  // into K ranges of whole 576-k chunks (the exact-accumulation unit); each
-  // range writes an FP64 partial tile and a reduction sums them in order.
+  // into K ranges of whole 576-k chunks; each range writes an FP64 partial
+  // tile and a reduction sums them in order.
   int64_t tiles = 0;
   for (const auto& s : secs) tiles += (int64_t)s.nmt * s.nnt;
   const int64_t want = 2 * (int64_t)ctx.num_sms;
@@ -203,10 +203,14 @@ void run_tc_gemms(Ctx& ctx, int ns, const std::vector<tn_sector_gemm>& list, con
     ctx.launched();
   }
   {
-    ProfScope ps(ctx, ns == 7 ? "tc_gemm_split" : (ns == 2 ? "tc_gemm_tf32" : "tc_gemm_bf16"), 0, P->flops);
+    ProfScope ps(ctx, ns == kSplitDigits ? "tc_gemm_split" : (ns == 2 ? "tc_gemm_tf32" : "tc_gemm_bf16"), 0, P->flops);
     int grid = (int)std::min<int64_t>((int64_t)P->nitems, (int64_t)ctx.num_sms);
-    launch_tc_gemm(ns, dsecs, (const int4*)(mb + P->off_it), P->nitems, images, ea, eb, C, part, err, grid,
-                   ctx.stream);
+    if (ns == kSplitDigits)
+      launch_tc_gemm_split(dsecs, (const int4*)(mb + P->off_it), P->nitems, images, ea, eb, C, part, err, grid,
+                           ctx.stream);
+    else
+      launch_tc_gemm(ns, dsecs, (const int4*)(mb + P->off_it), P->nitems, images, ea, eb, C, part, err, grid,
+                     ctx.stream);
     ctx.launched();
   }
   if (P->nred > 0) {

@@ -1,26 +1,9 @@
-// Tensor-core sector GEMMs for sm_103a (tcgen05 + TMEM + bulk copies).
+// Tensor-core sector GEMMs for sm_103a (tcgen05 + TMEM + bulk copies): the
+// operand maxima and digit images of every tensor-core mode, and the GEMM of
+// the fast modes (the split-precision GEMM is gemm_tc_split.cu).
 //
-// Split precision (TN_MODE_SPLIT): every FP64 operand element is written in
-// fixed point against its row's (A) or column's (B) power-of-two scale,
-// rounded to 49 bits, and cut into NS = 7 balanced signed digits of 7 bits
-// (d_0 in [-129, 129], d_1..d_6 in [-64, 63]); digit s is stored as the BF16
-// value d * 2^-7s, exact.  C = 2^(ea+eb-14) * sum_{s+t<=7} A_s B_t (34 of the
-// 49 digit products).  The products of one level l = s+t are integers times
-// 2^-7l; per k their magnitudes sum to at most 2*129*64 + 3*64*64 = 28800
-// for levels 0..4, so those accumulate exactly in FP32 over a chunk of 576 k
-// (576 * 28800 < 2^24).  Every level 0..7 has its own 64-column TMEM
-// accumulator (all 512 columns), drained into a double-float (hi, lo) FP32
-// sum per chunk; the FP32 rounding of levels 5..7 is far below 2^-53 of the
-// result.  The dropped levels 8..12 and the operand rounding bound the error
-// near 2^-50 relative to row/column maxima.
-//
-// With level l at columns 64 l, the products of A digit s with B digits
-// t0..t0+n-1 land in the contiguous columns 64 (s+t0) .. 64 (s+t0+n) - 1, and
-// the n B digit tiles lie back to back in shared memory with the same
-// 8-row stride: one MMA with N = 64 n (n <= 4) issues them all and reads the
-// A tile once.  A k-step takes 11 MMAs instead of 34, and runs at the full
-// tensor rate (N = 64 MMAs are bound by their shared-memory operand reads:
-// 48 clocks for 32 of work).
+// Split precision (TN_MODE_SPLIT): six BF16 digit images per operand tile
+// (tc_digits.cuh).
 // Fast BF16 (TN_MODE_FAST_BF16): one slice, the BF16 rounding of each scaled
 // element, FP32 accumulation over the whole K.
 // Fast TF32 (TN_MODE_FAST_TF32, NS = 2 below): the TF32 rounding of each
@@ -37,8 +20,8 @@
 //
 // GEMM CTA (576 threads): warp 0 = loads (bulk copies), warp 1 = MMA issue +
 // TMEM allocation, warps 2..17 = epilogue: warp w drains TMEM lane quadrant
-// w & 3 and columns 16 * ((w - 2) >> 2) .. +15 of every accumulator, so a
-// chunk's drain -- during which the MMAs wait -- is spread over 16 warps.
+// w & 3 and columns 16 * ((w - 2) >> 2) .. +15 of the accumulator, so the
+// drain -- during which the MMAs wait -- is spread over 16 warps.
 #include <cuda_bf16.h>
 
 #include <cstdint>
@@ -56,9 +39,6 @@ constexpr int kTM = 128, kTN = 64, kTK = 64;
 constexpr int kATile = kTM * kTK * 2;  // bytes of one A slice tile
 constexpr int kBTile = kTN * kTK * 2;  // bytes of one B slice tile
 constexpr int kARing = 6, kBRing = 2;
-constexpr int kChunkTiles = 9;  // 576 k per exact-accumulation chunk
-constexpr int kLevels = 8;      // one accumulator per level 0..7
-constexpr int kMaxLevel = 7;    // digit products with s + t <= 7 are kept
 constexpr int kEpiWarps = 16;
 constexpr int kThreadsTc = 64 + 32 * kEpiWarps;
 constexpr int kEpiCols = kTN * 4 / kEpiWarps;  // accumulator columns per epilogue warp
@@ -267,13 +247,6 @@ __device__ __forceinline__ void raise_timeout(TcShared& sh, int* err) {
   atomicExch(err, TN_ERR_TIMEOUT);
 }
 
-__device__ __forceinline__ void two_sum_add(float& hi, float& lo, float v) {
-  const float s = hi + v;
-  const float bb = s - hi;
-  lo += (hi - (s - bb)) + (v - bb);
-  hi = s;
-}
-
 template <int NS>
 __global__ void __launch_bounds__(kThreadsTc, 1) tc_gemm(const TcSector* __restrict__ secs,
                                                          const int4* __restrict__ items, int nitems,
@@ -282,16 +255,15 @@ __global__ void __launch_bounds__(kThreadsTc, 1) tc_gemm(const TcSector* __restr
                                                          const unsigned long long* __restrict__ eb,
                                                          double* __restrict__ C, double* __restrict__ part,
                                                          int* __restrict__ err) {
-  constexpr bool kFast = NS != 7;  // BF16 (NS = 1) or TF32 (NS = 2): one FP32 accumulator
-  constexpr int LV = kFast ? 1 : kLevels;
-  constexpr int kChunk = kFast ? 1 << 20 : kChunkTiles;  // fast modes: one chunk over all of K
+  // BF16 (NS = 1) or TF32 (NS = 2): one FP32 accumulator over all of K
   extern __shared__ uint8_t dyn[];
   __shared__ TcShared sh;
   // 1024-byte aligned operand buffers (the swizzle is anchored to 1024 B)
   uint8_t* base = (uint8_t*)(((uintptr_t)dyn + 1023) & ~(uintptr_t)1023);
   uint8_t* abuf = base;                                    // kARing x 16 KB
   uint8_t* bbuf = base + kARing * kATile;                  // kBRing x NS x 8 KB
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  // read from lane 0, so the compiler knows the warp's role to be warp-uniform
+  const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
 
   if (threadIdx.x == 0) {
     for (int i = 0; i < kARing; i++) {
@@ -358,86 +330,51 @@ __global__ void __launch_bounds__(kThreadsTc, 1) tc_gemm(const TcSector* __restr
     // ------------------------------------------------ MMA issue
     // The whole warp runs the loop (every lane waits on the barriers and the
     // outcome is made warp-uniform); one elected lane issues the MMAs and commits.
-    // instruction descriptor for N = 64: N = 64 n adds (n - 1) * 8 to its N >> 3 field (bit 17)
-    const uint32_t idesc1 = idesc_bf16_f32(kTM, kTN);
-    static_assert(idesc_bf16_f32(kTM, 4 * kTN) == idesc_bf16_f32(kTM, kTN) + ((3u * (kTN >> 3)) << 17), "N field");
+    constexpr uint32_t idesc = NS == 2 ? idesc_tf32_f32(kTM, kTN) : idesc_bf16_f32(kTM, kTN);
     uint32_t na = 0, nb = 0, nchunk = 0;
     bool ok = true;
     for (int it = blockIdx.x; it < nitems && ok; it += gridDim.x) {
       const int4 w = items[it];
       const TcSector& S = secs[w.x];
       const int kb = w.w * S.kts, ke = min(S.nkt, kb + S.kts);
-      for (int k0 = kb; k0 < ke && ok; k0 += kChunk) {
-        const int k1 = min(ke, k0 + kChunk);
-        if (!__all_sync(0xffffffffu, mbar_wait(&sh.acc_empty, (nchunk & 1) ^ 1, &sh.abort))) { ok = false; break; }
+      if (!__all_sync(0xffffffffu, mbar_wait(&sh.acc_empty, (nchunk & 1) ^ 1, &sh.abort))) { ok = false; break; }
+      tc_fence_after();
+      uint32_t touched = 0;
+      for (int kt = kb; kt < ke && ok; kt++) {
+        const int sb = nb % kBRing;
+        if (!__all_sync(0xffffffffu, mbar_wait(&sh.fullB[sb], (nb / kBRing) & 1, &sh.abort))) { ok = false; break; }
         tc_fence_after();
-        uint32_t touched = 0;
-        for (int kt = k0; kt < k1 && ok; kt++) {
-          const int sb = nb % kBRing;
-          const int nks = min(kTK, S.K - kt * kTK + 15) >> 4;  // 16-k steps of this tile holding data
-          if (!__all_sync(0xffffffffu, mbar_wait(&sh.fullB[sb], (nb / kBRing) & 1, &sh.abort))) { ok = false; break; }
-          tc_fence_after();
-          const uint32_t b_addr = smem_u32(bbuf + sb * NS * kBTile);
-          for (int s = 0; s < NS; s++) {
-            const int sa = na % kARing;
-            if (!__all_sync(0xffffffffu, mbar_wait(&sh.fullA[sa], (na / kARing) & 1, &sh.abort))) {
-              ok = false;
-              break;
-            }
-            tc_fence_after();
-            const uint64_t adesc = desc_sw128(smem_u32(abuf + sa * kATile));
-            if constexpr (NS == 2) {
-              // TF32: image s holds k 32 s .. 32 s + 31 of A and of B; steps of 8 k
-              const int kdat = S.K - kt * kTK - 32 * s;  // k of this image holding data
-              const int nk8 = kdat <= 0 ? 0 : min(4, (kdat + 7) >> 3);
-              const uint64_t bdesc = desc_sw128(b_addr + s * kBTile);
-              const uint32_t idesc = idesc_tf32_f32(kTM, kTN);
-              for (int kk = 0; kk < nk8; kk++) {
-                mma_tf32_elect(tmem, adesc + 2 * kk, bdesc + 2 * kk, idesc, (touched | kk) ? 1u : 0u);
-                touched = 1;
-              }
-              mma_commit_elect(&sh.emptyA[sa]);
-              na++;
-              continue;
-            }
-            // B digits t = 0 .. T-1 pair with A digit s (s + t <= 7), in
-            // groups of at most 4 (7 -> 4 + 3, 6 -> 3 + 3, 5 -> 3 + 2)
-            const int T = NS == 1 ? 1 : min(NS, kMaxLevel + 1 - s);
-            for (int t0 = 0; t0 < T;) {
-              int tn = T - t0 > 4 ? (T - t0 + 1) >> 1 : T - t0;
-              const int l0 = s + t0;
-              // one accumulate flag per MMA: cut the group where a level is
-              // written for the first time in this chunk (level 7, by s = 1)
-              const uint32_t acc = (touched >> l0) & 1;
-              for (int k = 1; k < tn; k++)
-                if (((touched >> (l0 + k)) & 1) != acc) {
-                  tn = k;
-                  break;
-                }
-              const uint32_t d = tmem + l0 * kTN;
-              const uint64_t bdesc = desc_sw128(b_addr + t0 * kBTile);
-              const uint32_t idesc = idesc1 + ((uint32_t)(tn - 1) * (kTN >> 3) << 17);
-              if (nks == kTK / 16) {  // a full 64-k tile: no per-step guard in the issue stream
-                mma_bf16_elect(d, adesc, bdesc, idesc, acc);
-#pragma unroll
-                for (int kk = 1; kk < kTK / 16; kk++)
-                  // advancing K by 16 bf16 = 32 bytes inside the swizzle atom: +2 in the address field
-                  mma_bf16_elect(d, adesc + 2 * kk, bdesc + 2 * kk, idesc, 1);
-              } else {  // the last tile of a ragged K: only the 16-k steps that hold data
-                for (int kk = 0; kk < nks; kk++) mma_bf16_elect(d, adesc + 2 * kk, bdesc + 2 * kk, idesc, kk ? 1 : acc);
-              }
-              touched |= ((1u << tn) - 1) << l0;
-              t0 += tn;
-            }
-            mma_commit_elect(&sh.emptyA[sa]);
-            na++;
+        const uint32_t b_addr = smem_u32(bbuf + sb * NS * kBTile);
+        for (int s = 0; s < NS; s++) {
+          const int sa = na % kARing;
+          if (!__all_sync(0xffffffffu, mbar_wait(&sh.fullA[sa], (na / kARing) & 1, &sh.abort))) {
+            ok = false;
+            break;
           }
-          mma_commit_elect(&sh.emptyB[sb]);
-          nb++;
+          tc_fence_after();
+          const uint64_t adesc = desc_sw128(smem_u32(abuf + sa * kATile));
+          const uint64_t bdesc = desc_sw128(b_addr + s * kBTile);
+          // 32 bytes of each operand row per step: 16 k (BF16) or 8 k (TF32: image s
+          // holds k 32 s .. 32 s + 31); only the steps that hold data
+          const int kdat = S.K - kt * kTK - (NS == 2 ? 32 * s : 0);
+          const int nstep = NS == 2 ? (kdat <= 0 ? 0 : min(4, (kdat + 7) >> 3)) : min(kTK, kdat + 15) >> 4;
+#pragma unroll
+          for (int kk = 0; kk < 4; kk++) {
+            if (kk >= nstep) break;
+            if constexpr (NS == 2)
+              mma_tf32_elect(tmem, adesc + 2 * kk, bdesc + 2 * kk, idesc, touched);
+            else
+              mma_bf16_elect(tmem, adesc + 2 * kk, bdesc + 2 * kk, idesc, touched);
+            touched = 1;
+          }
+          mma_commit_elect(&sh.emptyA[sa]);
+          na++;
         }
-        mma_commit_elect(&sh.acc_full);
-        nchunk++;
+        mma_commit_elect(&sh.emptyB[sb]);
+        nb++;
       }
+      mma_commit_elect(&sh.acc_full);
+      nchunk++;
     }
     if (!ok && lane == 0) raise_timeout(sh, err);
     // every MMA issued must complete before the tensor memory is released
@@ -453,29 +390,15 @@ __global__ void __launch_bounds__(kThreadsTc, 1) tc_gemm(const TcSector* __restr
     for (int it = blockIdx.x; it < nitems && ok; it += gridDim.x) {
       const int4 w = items[it];
       const TcSector& S = secs[w.x];
-      float hi[kEpiCols], lo[kEpiCols];
-#pragma unroll
-      for (int j = 0; j < kEpiCols; j++) hi[j] = lo[j] = 0.f;
-      const int kb = w.w * S.kts, ke = min(S.nkt, kb + S.kts);
-      for (int k0 = kb; k0 < ke; k0 += kChunk) {
-        if (!mbar_wait(&sh.acc_full, nchunk & 1, &sh.abort)) { ok = false; break; }
-        tc_fence_after();
-#pragma unroll
-        for (int l = 0; l < LV; l++) {
-#pragma unroll
-          for (int cg = 0; cg < kEpiCols / 16; cg++) {
-            float v[16];
-            tmem_ld16(lane_addr + l * kTN + cg * 16, v);
-#pragma unroll
-            for (int q = 0; q < 16; q++) two_sum_add(hi[cg * 16 + q], lo[cg * 16 + q], v[q]);
-          }
-        }
-        tc_fence_before();
-        __syncwarp();
-        if (lane == 0) mbar_arrive(&sh.acc_empty);
-        nchunk++;
-      }
-      if (!ok) break;
+      if (!mbar_wait(&sh.acc_full, nchunk & 1, &sh.abort)) { ok = false; break; }
+      tc_fence_after();
+      float v[kEpiCols];
+      static_assert(kEpiCols == 16, "one tcgen05.ld per tile and warp");
+      tmem_ld16(lane_addr, v);
+      tc_fence_before();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&sh.acc_empty);
+      nchunk++;
       const int64_t i = (int64_t)w.y * kTM + quad * 32 + lane;
       if (i < S.M) {
         const int e_i = exp_of(ea[S.ea_off + i]);
@@ -487,11 +410,9 @@ __global__ void __launch_bounds__(kThreadsTc, 1) tc_gemm(const TcSector* __restr
 #pragma unroll
         for (int j = 0; j < kEpiCols; j++) {
           const int64_t jj = (int64_t)w.z * kTN + half * kEpiCols + j;
-          // three FP64-pipe operations per output (two conversions, one add),
-          // the power-of-two scale on the exponent field: the epilogue warps
-          // share their schedulers with the MMA and load warps, so a long
-          // integer sequence here would slow the MMA issue instead
-          if (jj < S.N) crow[jj] = scale_pow2((double)hi[j] + (double)lo[j], e_i + exp_of(eb[S.eb_off + jj]) - 14);
+          // one FP64-pipe operation per output (the conversion), the power-of-two
+          // scale on the exponent field
+          if (jj < S.N) crow[jj] = scale_pow2((double)v[j], e_i + exp_of(eb[S.eb_off + jj]) - 14);
         }
       }
     }
@@ -537,8 +458,8 @@ void launch_tc_slices(int ns, const TcSector* secs, int nsec, const int64_t* a_t
                       const unsigned long long* amax, const unsigned long long* bmax, uint8_t* images, int num_sms,
                       cudaStream_t s) {
   int g2 = (int)std::min<int64_t>(a_tiles + b_tiles, (int64_t)num_sms * 8);
-  if (ns == 7)
-    tc_slices<7><<<g2, 256, 0, s>>>(secs, a_ts, b_ts, nsec, a_tiles, b_tiles, A, B, amax, bmax, images);
+  if (ns == kSplitDigits)
+    tc_slices<kSplitDigits><<<g2, 256, 0, s>>>(secs, a_ts, b_ts, nsec, a_tiles, b_tiles, A, B, amax, bmax, images);
   else if (ns == 2)
     tc_slices<2><<<g2, 256, 0, s>>>(secs, a_ts, b_ts, nsec, a_tiles, b_tiles, A, B, amax, bmax, images);
   else
@@ -546,20 +467,13 @@ void launch_tc_slices(int ns, const TcSector* secs, int nsec, const int64_t* a_t
   TN_CUDA(cudaGetLastError());
 }
 
-size_t tc_gemm_smem(int ns) { return (size_t)kARing * kATile + (size_t)kBRing * ns * kBTile + 1024; }
+static size_t tc_gemm_smem(int ns) { return (size_t)kARing * kATile + (size_t)kBRing * ns * kBTile + 1024; }
 
 void launch_tc_gemm(int ns, const TcSector* secs, const int4* items, int nitems, const uint8_t* ws,
                     const unsigned long long* ea, const unsigned long long* eb, double* C, double* part, int* err,
                     int grid, cudaStream_t s) {
   const size_t smem = tc_gemm_smem(ns);
-  if (ns == 7) {
-    static bool attr = false;
-    if (!attr) {
-      TN_CUDA(cudaFuncSetAttribute(tc_gemm<7>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-      attr = true;
-    }
-    tc_gemm<7><<<grid, kThreadsTc, smem, s>>>(secs, items, nitems, ws, ea, eb, C, part, err);
-  } else if (ns == 2) {
+  if (ns == 2) {
     static bool attr = false;
     if (!attr) {
       TN_CUDA(cudaFuncSetAttribute(tc_gemm<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));

@@ -1,7 +1,8 @@
 // Digit slicing shared by the tensor-core GEMM kernels: the power-of-two
-// row/column scale, the 7 balanced signed 7-bit digits of an FP64 value as
-// exact BF16 values, and the 128-byte swizzled K-major operand layout of
-// tcgen05 shared-memory descriptors.
+// row/column scale, the balanced signed digits of an FP64 value as exact BF16
+// values (6 of 9 bits in the tiled form, 7 of 7 bits in the fused form), and
+// the 128-byte swizzled K-major operand layout of tcgen05 shared-memory
+// descriptors.
 #pragma once
 #include <cuda_bf16.h>
 
@@ -35,11 +36,16 @@ __device__ __forceinline__ int exp_of(uint64_t maxbits) {
 // FP32 from the bit pattern of 1.5 * 2^(23-7s) + d * 2^-7s (integer add into
 // the mantissa, one exact subtraction); it has at most 8 significant bits, so
 // its BF16 pattern is the top half of the FP32 pattern.
+// NS = 6: X = |x| * 2^(52 - e) rounded to the nearest integer (X <= 2^52), V =
+// +-X and its balanced base-512 digits (d_1..d_5 in [-256, 255], |d_0| <= 128)
+// read out of Y = V + 256 * (1 + 512 + ... + 512^4) the same way.  They are
+// stored as plain integers (BF16 holds every integer up to 256), so one magic
+// number, 1.5 * 2^23, serves all of them.
 // NS = 1 (fast mode): the BF16 rounding of the FP32 rounding of x * 2^(7-e),
 // the scaling done on the exponent field.
 template <int NS>
 __device__ __forceinline__ void make_slices(const double (&x)[8], int e, uint4 (&out)[NS]) {
-  static_assert(NS == 1 || NS == 7, "7 digits (split) or one BF16 slice (fast)");
+  static_assert(NS == 1 || NS == 6 || NS == 7, "6 or 7 digits (split) or one BF16 slice (fast)");
   uint32_t hbits[NS][8];
 #pragma unroll
   for (int i = 0; i < 8; i++) {
@@ -61,23 +67,39 @@ __device__ __forceinline__ void make_slices(const double (&x)[8], int e, uint4 (
         mant |= 1ull << 52;
         E = ef - 1023;
       }
-      const int sh = 3 + e - E;  // X = mant * 2^(E - 52) * 2^(49 - e)
+      const int sh = (NS == 7 ? 3 : 0) + e - E;  // X = mant * 2^(E - 52) * 2^(49 - e), or 2^(52 - e) for 6 digits
       const uint64_t X = (sh >= 64) ? 0ull : (sh > 0 ? ((mant + (1ull << (sh - 1))) >> sh) : (mant << (-sh)));
       const long long V = (bits >> 63) ? -(long long)X : (long long)X;
-      const uint64_t Y = (uint64_t)(V + 2216338399296ll);  // + 64 * (128^6 - 1) / 127
-      const uint32_t lo = (uint32_t)Y, hi = (uint32_t)(Y >> 32);
-      int d[7];
-      d[6] = (int)(lo & 127u) - 64;
-      d[5] = (int)((lo >> 7) & 127u) - 64;
-      d[4] = (int)((lo >> 14) & 127u) - 64;
-      d[3] = (int)((lo >> 21) & 127u) - 64;
-      d[2] = (int)(__funnelshift_r(lo, hi, 28) & 127u) - 64;
-      d[1] = (int)((hi >> 3) & 127u) - 64;
-      d[0] = (int)hi >> 10;
+      if constexpr (NS == 6) {
+        const uint64_t Y = (uint64_t)(V + 17626613022976ll);  // + 256 * (512^5 - 1) / 511
+        const uint32_t lo = (uint32_t)Y, hi = (uint32_t)(Y >> 32);
+        // the five lower digits plus 256, in the low bits
+        const uint32_t d[6] = {(uint32_t)((int)hi >> 13),
+                               (hi >> 4) & 511u,
+                               __funnelshift_r(lo, hi, 27) & 511u,
+                               (lo >> 18) & 511u,
+                               (lo >> 9) & 511u,
+                               lo & 511u};
+        const float magic = __uint_as_float(0x4B400000u);  // 1.5 * 2^23
 #pragma unroll
-      for (int s = 0; s < 7; s++) {
-        const float magic = __uint_as_float(0x4B400000u - ((uint32_t)(7 * s) << 23));  // 1.5 * 2^(23-7s)
-        hbits[s][i] = __float_as_uint(__uint_as_float(__float_as_uint(magic) + (uint32_t)d[s]) - magic);
+        for (int s = 0; s < 6; s++)
+          hbits[s][i] = __float_as_uint(__uint_as_float(0x4B400000u + d[s]) - (s ? magic + 256.f : magic));
+      } else if constexpr (NS == 7) {
+        const uint64_t Y = (uint64_t)(V + 2216338399296ll);  // + 64 * (128^6 - 1) / 127
+        const uint32_t lo = (uint32_t)Y, hi = (uint32_t)(Y >> 32);
+        int d[7];
+        d[6] = (int)(lo & 127u) - 64;
+        d[5] = (int)((lo >> 7) & 127u) - 64;
+        d[4] = (int)((lo >> 14) & 127u) - 64;
+        d[3] = (int)((lo >> 21) & 127u) - 64;
+        d[2] = (int)(__funnelshift_r(lo, hi, 28) & 127u) - 64;
+        d[1] = (int)((hi >> 3) & 127u) - 64;
+        d[0] = (int)hi >> 10;
+#pragma unroll
+        for (int s = 0; s < 7; s++) {
+          const float magic = __uint_as_float(0x4B400000u - ((uint32_t)(7 * s) << 23));  // 1.5 * 2^(23-7s)
+          hbits[s][i] = __float_as_uint(__uint_as_float(__float_as_uint(magic) + (uint32_t)d[s]) - magic);
+        }
       }
     }
   }
@@ -126,6 +148,22 @@ __device__ __forceinline__ double fixed_to_double(long long S, int q) {
   return __longlong_as_double((long long)(sign | (((uint64_t)(E + 1022) << 52) + r)));
 }
 
+// The same for q within +-1000, where no result leaves the normal range: about
+// 25 integer instructions
+__device__ __forceinline__ double fixed_to_double_inrange(long long S, int q) {
+  const uint32_t neg = (uint32_t)((uint64_t)S >> 32) & 0x80000000u;
+  const uint64_t mag = S < 0 ? 0ull - (uint64_t)S : (uint64_t)S;
+  const uint32_t mh = (uint32_t)(mag >> 32), ml = (uint32_t)mag;
+  const uint32_t h = mh ? mh : ml, l = mh ? ml : 0u;
+  const int z = __clz((int)h);
+  const uint32_t H = __funnelshift_l(l, h, z), L = l << z;   // leading one at bit 31 of H
+  const uint32_t up = ((L & 0x7FFu) + ((L >> 11) & 1u) + 0x3FFu) >> 11;  // round to nearest even
+  const uint32_t e = (uint32_t)((mh ? 1022 + 63 : 1022 + 31) - z + q);
+  uint64_t r = ((uint64_t)(H >> 11) << 32) | __funnelshift_r(L, H, 11);
+  r += ((uint64_t)(e << 20) << 32) + up;  // the hidden bit adds one to the exponent field
+  r |= (uint64_t)neg << 32;
+  return __longlong_as_double((long long)(h ? r : 0ull));
+}
 
 // d * 2^q for a finite double d, the exponent field adjusted as an integer
 // when the result stays normal (else ldexp)
