@@ -65,8 +65,18 @@ void choose_tile(PermSub& ps, int es) {
   } else {
     ps.tx = (int32_t)std::min<int64_t>(ps.dims[x], kTile);
     if (n >= 2) {
+      // y: the next destination dim; with rows of 32 elements and more, where
+      // the order of whole rows costs nothing, the dim that fills the tile
+      // best.  (A physical bond of 2 next to a virtual one made tiles of two
+      // rows, each a pipeline latency: the U(1) regroup (v, p | p', v) ->
+      // (v, p' | p, v) of 4.2e6 complex elements, v = 1500 over 7 charges,
+      // took 71 us, now 31.)
+      const int64_t rows = std::max<int64_t>(1, kTile / ps.tx);
       ps.ydim = n - 2;
-      ps.ty = (int32_t)std::min<int64_t>(ps.dims[n - 2], std::max<int64_t>(1, kTile / ps.tx));
+      if (ps.tx >= 32)
+        for (int i = n - 3; i >= 0; i--)
+          if (std::min<int64_t>(ps.dims[i], rows) > std::min<int64_t>(ps.dims[ps.ydim], rows)) ps.ydim = i;
+      ps.ty = (int32_t)std::min<int64_t>(ps.dims[ps.ydim], rows);
     } else {
       ps.ty = 1;
     }
@@ -77,7 +87,8 @@ void choose_tile(PermSub& ps, int es) {
   if (ps.mode == 0 && n >= 3 && (int64_t)ps.tx * ps.ty <= kTile / 16) {
     int z = -1;
     int64_t best = 0;
-    for (int i = 0; i < n - 2; i++) {
+    for (int i = 0; i < n - 1; i++) {
+      if (i == ps.ydim) continue;
       const int64_t c = std::min(ps.sstride[i], ps.dstride[i]);
       if (z < 0 || c < best) {
         z = i;
