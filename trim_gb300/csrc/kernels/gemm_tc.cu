@@ -181,6 +181,17 @@ __device__ __forceinline__ void slice_a_tile(const TcSector* __restrict__ secs, 
   }
 }
 
+// The column that row r of a B image holds.  The split kernel's epilogue reads
+// its accumulators in the tcgen05 16 x 256b fragment order, where a thread of a
+// group of four has columns 2 p, 2 p + 1, 8 + 2 p and 9 + 2 p of 16: with the
+// columns in this order they are 4 p .. 4 p + 3, and it stores 32 bytes, four
+// threads the 128 bytes of a row.
+template <int NS>
+__device__ __forceinline__ int image_column(int r) {
+  if (NS != kSplitDigits) return r;
+  return (r & ~15) | ((r & 6) << 1) | ((r & 8) >> 2) | (r & 1);
+}
+
 // B tile t: (sector, nt, kt) -> NS images of 64 columns (rows of the image) x 64 k.
 // The FP64 block is first staged in shared memory with flat coalesced loads,
 // then each thread slices 8 consecutive k of one column.
@@ -208,12 +219,12 @@ __device__ __forceinline__ void slice_b_tile(const TcSector* __restrict__ secs, 
   __syncthreads();
   uint8_t* img = ws + S.b_img + (int64_t)local * NS * kBTile;
   for (int u = threadIdx.x; u < kTN * 8; u += blockDim.x) {
-    const int r = u % kTN, c = u / kTN;
+    const int r = u % kTN, c = u / kTN, n = image_column<NS>(r);
     int e = 0;
-    if (r < w) e = exp_of(eb[S.eb_off + n0 + r]);
+    if (n < w) e = exp_of(eb[S.eb_off + n0 + n]);
     double x[8];
 #pragma unroll
-    for (int q = 0; q < 8; q++) x[q] = stage[c * 8 + q][r];
+    for (int q = 0; q < 8; q++) x[q] = stage[c * 8 + q][n];
     store_chunk<NS>(img, kBTile, r, c, x, e);
   }
 }

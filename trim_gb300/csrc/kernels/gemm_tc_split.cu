@@ -46,12 +46,14 @@
 // columns 16 ((w - 2) >> 2) .. +15 of each level.
 //
 // Measured (GB300, all of a call's launches): the left MERA diagram at chi = 24
-// (K = 576, 6.7e11 FP64-equivalent flop) 16.0 -> 9.7 ms, the iPEPS quadrant at
-// chi = 128, D = 8 (K = 4096, 1.4e11) 3.41 -> 1.77 ms, against the 34-product
+// (K = 576, 6.7e11 FP64-equivalent flop) 16.0 -> 9.5 ms, the iPEPS quadrant at
+// chi = 128, D = 8 (K = 4096, 1.4e11) 3.41 -> 1.76 ms, against the 34-product
 // kernel.  21 products per FP64 multiply-add: 80 TFLOP/s FP64-equivalent at
 // K = 4096 is 1 690 of BF16, and the tensor pipe alone (no loads, no drain, no
-// output) takes 1.51 ms; at K = 576 the FP64 output of every ninth tile costs
-// as much again as what is left of the drain.
+// output) takes 1.51 ms; at K = 576 the FP64 output of every ninth tile (64 KB at
+// the 30 B per clock that an SM stores, whatever the pattern, as long as a row's
+// 128 bytes go together: 17 B per clock with a row per lane) stalls the drain
+// and, through the ring, the MMAs for 1.4 ms of the 9.5.
 #include <cstdint>
 
 #include "../engine/engine.h"
@@ -209,19 +211,23 @@ __device__ __forceinline__ int split_tile(MmaState& st) {
   return 1;
 }
 
-// warp: 32 lanes x 16 columns at a and at b; the data is in the registers on return
-__device__ __forceinline__ void tmem_ld16x2(uint32_t a, uint32_t b, float (&v)[16], float (&w)[16]) {
+// warp: 32 TMEM lanes x 16 columns at a and at b, as four 16-lane x 16-column
+// loads in the accumulator fragment order: with r = lane / 4 and p = lane % 4,
+// value 8 h + 4 g + 2 u + i is row 16 h + 8 u + r, column 8 g + 2 p + i.  The
+// data is in the registers on return.
+__device__ __forceinline__ void tmem_ld32x16x2(uint32_t a, uint32_t b, float (&v)[16], float (&w)[16]) {
   uint32_t r[16], s[16];
   asm volatile(
-      "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%32];\n"
-      "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31}, "
-      "[%33];\n"
+      "tcgen05.ld.sync.aligned.16x256b.x2.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%32];\n"
+      "tcgen05.ld.sync.aligned.16x256b.x2.b32 {%8,%9,%10,%11,%12,%13,%14,%15}, [%33];\n"
+      "tcgen05.ld.sync.aligned.16x256b.x2.b32 {%16,%17,%18,%19,%20,%21,%22,%23}, [%34];\n"
+      "tcgen05.ld.sync.aligned.16x256b.x2.b32 {%24,%25,%26,%27,%28,%29,%30,%31}, [%35];\n"
       "tcgen05.wait::ld.sync.aligned;"
       : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]),
         "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15]), "=r"(s[0]),
         "=r"(s[1]), "=r"(s[2]), "=r"(s[3]), "=r"(s[4]), "=r"(s[5]), "=r"(s[6]), "=r"(s[7]), "=r"(s[8]), "=r"(s[9]),
         "=r"(s[10]), "=r"(s[11]), "=r"(s[12]), "=r"(s[13]), "=r"(s[14]), "=r"(s[15])
-      : "r"(a), "r"(b)
+      : "r"(a), "r"(a + (16u << 16)), "r"(b), "r"(b + (16u << 16))
       : "memory");
 #pragma unroll
   for (int i = 0; i < 16; i++) {
@@ -234,7 +240,7 @@ __device__ __forceinline__ void prefetch_l1(const void* p) {
   asm volatile("prefetch.global.L1 [%0];" ::"l"(__cvta_generic_to_global(p)));
 }
 
-// 32 bytes in one store (sm_100 and up): a full L2 sector per thread
+// 32 bytes in one store (sm_100 and up); four lanes write a row's 128 bytes
 __device__ __forceinline__ void store4(double* p, const double* v) {
   asm volatile("st.global.v4.f64 [%0], {%1, %2, %3, %4};" ::"l"(__cvta_generic_to_global(p)), "d"(v[0]), "d"(v[1]),
                "d"(v[2]), "d"(v[3])
@@ -371,10 +377,10 @@ __global__ void __launch_bounds__(kThreadsSplit, 1) tc_gemm_split(const TcSector
       prefetch_l1(items + next);
       const TcSector& S = secs[w.x];
       const int kb = w.w * S.kts, ke = min(S.nkt, kb + S.kts);
-      const int64_t i = (int64_t)w.y * kTM + quad * 32 + lane;
-      const int64_t j0 = (int64_t)w.z * kTN + half * kEpiCols;  // first column of this thread
+      const int64_t i0 = (int64_t)w.y * kTM + quad * 32, i = i0 + lane;
+      const int64_t j0 = (int64_t)w.z * kTN + half * kEpiCols;  // first column of this warp
       const int nc = (int)max((int64_t)0, min((int64_t)kEpiCols, S.N - j0));
-      // the row's maximum, and lane q the one of column j0 + q
+      // lane l: the maximum of row i0 + l, and of column j0 + (l & 15)
       const unsigned long long row_max = i < S.M ? __ldg(ea + S.ea_off + i) : 0;
       const unsigned long long col_max = (lane & 15) < nc ? __ldg(eb + S.eb_off + j0 + (lane & 15)) : 0;
       for (int k0 = kb; k0 < ke && ok; k0 += kSegTiles) {
@@ -392,7 +398,7 @@ __global__ void __launch_bounds__(kThreadsSplit, 1) tc_gemm_split(const TcSector
             }
             tc_fence_after();
             float a[kEpiCols], b[kEpiCols];  // levels 2j and 2j + 1
-            tmem_ld16x2(lane_addr + slot * kSlotCols, lane_addr + slot * kSlotCols + kTN, a, b);
+            tmem_ld32x16x2(lane_addr + slot * kSlotCols, lane_addr + slot * kSlotCols + kTN, a, b);
             tc_fence_before();
             __syncwarp();
             if (lane == 0) mbar_arrive(&sh.emptyT[slot]);
@@ -411,33 +417,40 @@ __global__ void __launch_bounds__(kThreadsSplit, 1) tc_gemm_split(const TcSector
         }
         if (!ok) break;
         if (nc > 0) {
-          const int e_i = exp_of(row_max) - kUnit, e_j = exp_of(col_max);
-          // one K range of a split sector: its FP64 partial tile, [128][64]
-          double* crow = S.nsplit > 1
-                             ? part + S.p_off + (((int64_t)w.y * S.nnt + w.z) * S.nsplit + w.w) * (kTM * kTN) +
-                                   (quad * 32 + lane) * kTN + half * kEpiCols
-                             : C + S.c_off + i * S.N + j0;
-          const bool live = i < S.M;
+          const int e_row = exp_of(row_max) - kUnit, e_col = exp_of(col_max);
           // every scale of the warp well inside the exponent range: no output can leave it
-          const bool plain = abs(e_i) < 400 && abs(e_j) < 400;
-          if (__all_sync(0xffffffffu, plain && (!live || ((uintptr_t)crow & 31) == 0)) && nc == kEpiCols && k0 == kb) {
+          const bool plain = __all_sync(0xffffffffu, abs(e_row) < 400 && abs(e_col) < 400);
+          // the images of B hold the columns of a group of 16 in the order that gives a
+          // thread four consecutive ones: columns j0 + 4 p .. + 3 of rows r, r + 8, ..
+          const int r = lane >> 2, p4 = 4 * (lane & 3);
+          int ej[4];
 #pragma unroll
-            for (int q = 0; q < kEpiCols; q += 4) {
-              double v[4];
+          for (int c = 0; c < 4; c++) ej[c] = __shfl_sync(0xffffffffu, e_col, p4 + c);
+          // one K range of a split sector: its FP64 partial tile, [128][64]
+          double* out = S.nsplit > 1 ? part + S.p_off +
+                                           (((int64_t)w.y * S.nnt + w.z) * S.nsplit + w.w) * (kTM * kTN) +
+                                           quad * 32 * kTN + half * kEpiCols + p4
+                                     : C + S.c_off + i0 * S.N + j0 + p4;
+          const int64_t ld = S.nsplit > 1 ? kTN : S.N;
+          const int rows = (int)min((int64_t)32, S.M - i0);
+          const bool wide = plain && nc == kEpiCols && k0 == kb && (((uintptr_t)out | (uintptr_t)(8 * ld)) & 31) == 0;
 #pragma unroll
-              for (int p = 0; p < 4; p++)
-                v[p] = fixed_to_double_inrange(acc[q + p], e_i + __shfl_sync(0xffffffffu, e_j, q + p));
-              if (live) store4(crow + q, v);
+          for (int t = 0; t < 4; t++) {  // row r + 8 t: values 8 (t / 2) + 2 (t % 2) + {0, 1, 4, 5}
+            const int e_i = __shfl_sync(0xffffffffu, e_row, r + 8 * t);
+            double* crow = out + (r + 8 * t) * ld;
+            const bool live = r + 8 * t < rows;
+            double v[4];
+#pragma unroll
+            for (int c = 0; c < 4; c++) {
+              const long long x = acc[8 * (t >> 1) + 2 * (t & 1) + 4 * (c >> 1) + (c & 1)];
+              v[c] = plain ? fixed_to_double_inrange(x, e_i + ej[c]) : fixed_to_double(x, e_i + ej[c]);
             }
-          } else {
+            if (wide) {
+              if (live) store4(crow, v);
+            } else {
 #pragma unroll
-            for (int q = 0; q < kEpiCols; q++) {
-              const int e = e_i + __shfl_sync(0xffffffffu, e_j, q);
-              if (live && q < nc) {
-                double v = fixed_to_double(acc[q], e);
-                if (k0 > kb) v += crow[q];  // the segments of a long K, in order
-                crow[q] = v;
-              }
+              for (int c = 0; c < 4; c++)
+                if (live && p4 + c < nc) crow[c] = k0 > kb ? crow[c] + v[c] : v[c];  // the segments of a long K, in order
             }
           }
         }
