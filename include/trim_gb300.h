@@ -175,11 +175,12 @@ int tn_contract_sectors_loop(tn_ctx_t ctx, int mode, int n, const tn_sector_gemm
 /* Autotuner of the FP64 grouped GEMM (no counterpart in the reference): when
  * on, the first contraction with a new sector-size histogram (the number of
  * sectors per (log2 M, log2 N, log2 K) bucket) times each candidate plan --
- * tile width rule (narrowest of 4/8/16/32 columns that covers N, or always
- * 32) x K-split target (4, 8, 16 work items per SM) -- once with CUDA events
+ * the default (outputs dealt to lanes one after another), or output tiles with
+ * a width rule (narrowest of 4/8/16/32 columns that covers N, or always 32) x
+ * K-split target (2, 8, 16 work items per SM) -- once with CUDA events
  * and keeps the fastest for that histogram; that call is synchronous.  Later
  * contractions with the same histogram use the kept choice, so they stay
- * deterministic.  Off by default (the narrowest-width rule, 8 items per SM).
+ * deterministic.  Off by default.
  * entries (may be NULL) receives the number of histograms tuned so far. */
 int tn_autotune(tn_ctx_t ctx, int on, int64_t* entries);
 

@@ -157,15 +157,36 @@ struct GemmTile {
   int64_t ws_off;               // partial-tile slot in the workspace (elements), -1 if nsplit==1
 };
 
+// Work item of the flat FP64 grouped GEMM (gemm_fp64_flat.cu): entries v0 ..
+// v0 + nv - 1 (at most 128) of a sector's list of (K range, output) pairs, the
+// outputs of one range after another; entry v is output v % mn of K range
+// v / mn (kc long).  Items whose outputs have several ranges belong to a group
+// (outputs o0 .. o0 + go - 1, cnt items) that the last of them sums.
+struct FlatItem {
+  int64_t a_off, b_off, c_off;
+  int64_t ws_off;          // the group's partial sums: range q of output o0 + i at ws_off + q * gs + i
+  int32_t N, K, mn;        // mn = M * N
+  int32_t v0, nv, kc;
+  int32_t nsplit, o0, go, gs;
+  int32_t grp, cnt;        // group (-1: one K range, written directly) and its number of items
+  int32_t rows;            // 1: entries are rows of a sector of N <= 2 columns, lanes along K
+  int32_t a_vw, b_vw;      // operand views (ViewHdr index), -1: contiguous row-major
+  int32_t pad;
+};
+constexpr int kFlatWarps = 4, kFlatCtasPerSm = 5;  // warps per CTA, CTAs an SM holds (registers)
+constexpr int kFlatSlots = 4, kFlatViewSlots = 2;  // slots per item, and with a view
+
 // Planning choices of the FP64 grouped GEMM (the autotuner's search space):
-// tile width rule (0: the narrowest of 4/8/16/32 that covers N; 1: always 32)
-// and the K-split target (work items per SM).
+// flat items, or tiles with a width rule (0: the
+// narrowest of 4/8/16/32 that covers N; 1: always 32) and a K-split target
+// (work items per SM).
 struct Fp64Policy {
+  bool flat = true;
   int tn_rule = 0;
   int items_per_sm = 8;
   int spread = 4;  // with fewer than spread x SMs tiles, K is split until there are about that many items (0: never)
   bool operator==(const Fp64Policy& o) const {
-    return tn_rule == o.tn_rule && items_per_sm == o.items_per_sm && spread == o.spread;
+    return flat == o.flat && tn_rule == o.tn_rule && items_per_sm == o.items_per_sm && spread == o.spread;
   }
 };
 
@@ -402,6 +423,11 @@ void run_sector_gemms_views(Ctx& ctx, int mode, const std::vector<tn_sector_gemm
 std::vector<GemmTile> plan_fp64(const std::vector<tn_sector_gemm>& list, int num_sms, int64_t ws_cap_elems,
                                 int64_t* ws_elems, const Fp64Policy& pol = Fp64Policy());
 
+// Flat work list: ws_elems / ngroups receive the partial sums' workspace and
+// the number of split groups; vw (may be null): (A view, B view) per sector.
+std::vector<FlatItem> plan_fp64_flat(const std::vector<tn_sector_gemm>& list, int num_sms, int64_t* ws_elems,
+                                     int64_t* ngroups, const std::vector<std::pair<int, int>>* vw = nullptr);
+
 // kernel launchers (defined in the .cu files)
 void launch_permute_kernel(const PermSub* subs, const int64_t* tile_start, int nsub, int64_t ntiles, int esz,
                            bool conj, const void* src, void* dst, int grid, cudaStream_t s);
@@ -414,6 +440,8 @@ void launch_permute_kernel(const PermSub* subs, const int64_t* tile_start, int n
 void launch_gemm_fp64(const GemmTile* tiles, int ntiles, const double* A, const double* B, double* C,
                       double* ws, int* counters, const ViewHdr* views, const int64_t* pool, int grid,
                       cudaStream_t s, bool dependent_launch = true);
+void launch_gemm_fp64_flat(const FlatItem* items, int nitems, const double* A, const double* B, double* C, double* ws,
+                           int* counters, const ViewHdr* views, const int64_t* pool, int grid, cudaStream_t s);
 void launch_splitk_reduce(const GemmTile* tiles, int ntiles, const double* ws, double* C, int grid,
                           cudaStream_t s);
 void launch_negate_blocks(const int64_t* tab, int n, double* elem, cudaStream_t s);

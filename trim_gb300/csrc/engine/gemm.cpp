@@ -149,7 +149,130 @@ std::vector<GemmTile> plan_fp64(const std::vector<tn_sector_gemm>& list, int num
   return t;
 }
 
+// Flat items.  Cost is counted in warp FMAs (slots x K): an SM sub-partition
+// runs one at a time, so items are cut to about a sixteenth of its share (at
+// least 64 warp FMAs, below which an item's own latency shows; at most 4096).
+// Sectors of at least 128 outputs are cut into chunks of at most 4 slots (one
+// slot while an item is small: K ranges, with their partial sums, are the
+// second choice), each with its K ranges as a group; smaller ones deal all
+// their (K range, output) pairs to lanes, with the number of ranges raised
+// while more than 1 lane in 16 would stay empty.  An item that reads an operand
+// through views walks its K range in the views' segments, so its entries share
+// one range.
+std::vector<FlatItem> plan_fp64_flat(const std::vector<tn_sector_gemm>& list, int num_sms, int64_t* ws_elems,
+                                     int64_t* ngroups, const std::vector<std::pair<int, int>>* vw) {
+  double total = 0;
+  for (const auto& g : list)
+    if (g.M > 0 && g.N > 0 && g.K > 0) total += std::ceil((double)g.M * g.N / 32.0) * (double)g.K;
+  const int64_t target = (int64_t)std::min(4096.0, std::max(64.0, total / (4.0 * num_sms * 16.0)));
+  std::vector<FlatItem> out;
+  int64_t ws = 0, ngrp = 0;
+  const int64_t most_plain = std::max<int64_t>(1, std::min<int64_t>(kFlatSlots, target / 256));  // slots per chunk
+  for (size_t gi = 0; gi < list.size(); gi++) {
+    const auto& g = list[gi];
+    if (g.M <= 0 || g.N <= 0 || g.K <= 0) continue;
+    FlatItem t;
+    std::memset(&t, 0, sizeof(t));
+    t.a_off = g.a_off;
+    t.b_off = g.b_off;
+    t.c_off = g.c_off;
+    t.N = (int32_t)g.N;
+    t.K = (int32_t)g.K;
+    t.grp = -1;
+    t.nsplit = 1;
+    t.a_vw = vw ? (*vw)[gi].first : -1;
+    t.b_vw = vw ? (*vw)[gi].second : -1;
+    const bool viewed = t.a_vw >= 0 || t.b_vw >= 0;
+    if (g.N <= 2 && g.K >= 32 && !viewed) {  // lanes along K
+      t.rows = 1;
+      t.mn = (int32_t)g.M;
+      const int64_t per = std::max<int64_t>(1, std::min<int64_t>(64, target / (g.N * ((g.K + 31) / 32 + 5))));
+      for (int64_t m0 = 0; m0 < g.M; m0 += per) {
+        t.v0 = (int32_t)m0;
+        t.nv = (int32_t)std::min(per, g.M - m0);
+        out.push_back(t);
+      }
+      continue;
+    }
+    const int64_t mn = g.M * g.N, slots = (mn + 31) / 32;
+    t.mn = (int32_t)mn;
+    if (mn >= 128 || viewed) {
+      const int64_t most = viewed ? std::min<int64_t>(most_plain, kFlatViewSlots) : most_plain;
+      const int64_t nch = (slots + most - 1) / most;
+      const int64_t kc0 = std::max<int64_t>(32, target * nch / slots);
+      const int64_t ns = std::max<int64_t>(1, std::min<int64_t>((g.K + kc0 / 2) / kc0, 256));
+      t.kc = (int32_t)((g.K + ns - 1) / ns);
+      t.nsplit = (int32_t)((g.K + t.kc - 1) / t.kc);
+      for (int64_t c = 0; c < nch; c++) {
+        const int64_t o0 = 32 * (slots * c / nch), o1 = std::min(mn, 32 * (slots * (c + 1) / nch));
+        if (t.nsplit > 1) {
+          t.grp = (int32_t)ngrp++;
+          t.cnt = t.nsplit;
+          t.o0 = (int32_t)o0;
+          t.go = (int32_t)(o1 - o0);
+          t.gs = t.go;
+          t.ws_off = ws;
+          ws += (int64_t)t.nsplit * t.go;
+        }
+        for (int q = 0; q < t.nsplit; q++) {
+          t.v0 = (int32_t)(q * mn + o0);
+          t.nv = (int32_t)(o1 - o0);
+          out.push_back(t);
+        }
+      }
+    } else {
+      const int64_t kc0 = std::max<int64_t>(32, target);
+      int64_t ns = std::max<int64_t>(1, (g.K + kc0 - 1) / kc0);
+      auto waste = [&](int64_t n) { return (double)((mn * n + 31) / 32 * 32) / (double)(mn * n); };
+      while (waste(ns) > 1.0625 && ns < 32 && g.K / (ns + 1) >= 32) ns++;
+      t.kc = (int32_t)((g.K + ns - 1) / ns);
+      t.nsplit = (int32_t)((g.K + t.kc - 1) / t.kc);
+      const int64_t nv = mn * t.nsplit;
+      // entries per item: as many slots as the target allows
+      const int64_t per = 32 * std::max<int64_t>(1, std::min<int64_t>(kFlatSlots, target / std::max(1, (int)t.kc)));
+      if (t.nsplit > 1) {
+        t.grp = (int32_t)ngrp++;
+        t.cnt = (int32_t)((nv + per - 1) / per);
+        t.go = t.gs = (int32_t)mn;
+        t.ws_off = ws;
+        ws += nv;
+      }
+      for (int64_t v0 = 0; v0 < nv; v0 += per) {
+        t.v0 = (int32_t)v0;
+        t.nv = (int32_t)std::min(per, nv - v0);
+        out.push_back(t);
+      }
+    }
+  }
+  *ws_elems = ws;
+  *ngroups = ngrp;
+  // the warps of a CTA take kWarps consecutive items; with more items than the
+  // grid holds at once, costly ones first, in bands alternately reversed, as
+  // for the tiles above
+  const int64_t grid_items = (int64_t)num_sms * kFlatCtasPerSm * kFlatWarps;
+  if ((int64_t)out.size() <= grid_items) return out;
+  auto cost = [](const FlatItem& t) {
+    return t.rows ? (int64_t)t.nv * t.N * ((t.K + 31) / 32 + 5) : (int64_t)((t.nv + 31) / 32) * std::min(t.kc, t.K);
+  };
+  std::stable_sort(out.begin(), out.end(), [&](const FlatItem& a, const FlatItem& b) { return cost(a) > cost(b); });
+  const size_t band = (size_t)grid_items;
+  for (size_t b0 = band; b0 < out.size(); b0 += 2 * band)
+    std::reverse(out.begin() + b0, out.begin() + std::min(out.size(), b0 + band));
+  return out;
+}
+
+// 32-bit entry numbers: a sector of 2^31 / 256 outputs or more takes the tiles
+static bool flat_fits(const std::vector<tn_sector_gemm>& list) {
+  for (const auto& g : list)
+    if (g.M > 0 && g.N > 0 && g.K > 0 &&
+        (g.M > INT32_MAX || g.N > INT32_MAX || g.K > INT32_MAX / 2 || (double)g.M * (double)g.N >= (double)(1 << 23)))
+      return false;
+  return true;
+}
+
 struct Fp64Plan {
+  DevBufP flat;  // FlatItem list (then no tiles)
+  int nflat = 0;
   std::vector<tn_sector_gemm> list;
   std::vector<std::pair<int, int>> vw;  // operand view ids per sector (empty: contiguous operands)
   const void* table = nullptr;          // the view table the ids index
@@ -165,7 +288,7 @@ static std::shared_ptr<Fp64Plan> get_fp64_plan(Ctx& ctx, const std::vector<tn_se
                                                const Fp64Policy& pol,
                                                const std::vector<std::pair<int, int>>* vw = nullptr,
                                                const void* table = nullptr) {
-  uint64_t key = hash_list(list, 64 + 16 * pol.tn_rule + pol.items_per_sm + 1024 * pol.spread);
+  uint64_t key = hash_list(list, 64 + 16 * pol.tn_rule + pol.items_per_sm + 1024 * pol.spread + (pol.flat ? 65536 : 0));
   if (vw) {
     for (const auto& v : *vw) key = (key ^ (uint64_t)(uint32_t)v.first ^ ((uint64_t)(uint32_t)v.second << 32)) * 1099511628211ull;
     key ^= (uint64_t)(uintptr_t)table;
@@ -190,17 +313,31 @@ static std::shared_ptr<Fp64Plan> get_fp64_plan(Ctx& ctx, const std::vector<tn_se
     P->vw = *vw;
     P->table = table;
   }
-  std::vector<GemmTile> tiles = plan_fp64_split(list, ctx.num_sms, true, &P->ws_elems, pol, vw);
+  const bool flat = pol.flat && flat_fits(list);
+  int64_t ngrp = 0;
+  std::vector<FlatItem> items;
+  std::vector<GemmTile> tiles;
+  if (flat) {
+    items = plan_fp64_flat(list, ctx.num_sms, &P->ws_elems, &ngrp, vw);
+    P->nflat = (int)items.size();
+  } else {
+    tiles = plan_fp64_split(list, ctx.num_sms, true, &P->ws_elems, pol, vw);
+    for (const auto& t : tiles) ngrp = std::max<int64_t>(ngrp, (int64_t)t.grp + 1);
+  }
   P->ntiles = (int)tiles.size();
   for (const auto& g : list) {
     P->flops += 2.0 * g.M * g.N * g.K;
     P->bytes += 8.0 * (g.M * g.K + g.K * g.N + g.M * g.N);
   }
-  int64_t ngrp = 0;
-  for (const auto& t : tiles) ngrp = std::max<int64_t>(ngrp, (int64_t)t.grp + 1);
   if (ngrp > 0) {
     P->counters = std::make_shared<DevBuf>((size_t)ngrp * sizeof(int), ctx);
     TN_CUDA(cudaMemsetAsync(P->counters->ptr, 0, (size_t)ngrp * sizeof(int), ctx.stream));
+  }
+  if (!items.empty()) {
+    P->flat = std::make_shared<DevBuf>(items.size() * sizeof(FlatItem), ctx);
+    TN_CUDA(cudaMemcpyAsync(P->flat->ptr, items.data(), items.size() * sizeof(FlatItem), cudaMemcpyHostToDevice,
+                            ctx.stream));
+    TN_CUDA(cudaStreamSynchronize(ctx.stream));  // the host copy dies here
   }
   if (!tiles.empty()) {
     P->tiles = std::make_shared<DevBuf>(tiles.size() * sizeof(GemmTile), ctx);
@@ -220,7 +357,14 @@ static void launch_fp64_plan(Ctx& ctx, const Fp64Plan& P, const double* A, const
   double* ws = nullptr;
   if (P.ws_elems > 0) ws = (double*)ctx.ensure_workspace(P.ws_elems * sizeof(double))->ptr;
   int grid = (int)std::min<int64_t>((int64_t)P.ntiles, (int64_t)ctx.num_sms * 16);
-  {
+  if (P.nflat) {
+    ProfScope ps(ctx, "gemm_fp64", P.bytes, P.flops);
+    grid = (int)std::min<int64_t>(((int64_t)P.nflat + kFlatWarps - 1) / kFlatWarps,
+                                  (int64_t)ctx.num_sms * kFlatCtasPerSm);
+    launch_gemm_fp64_flat((const FlatItem*)P.flat->ptr, P.nflat, A, B, C, ws,
+                          P.counters ? (int*)P.counters->ptr : nullptr, views, pool, grid, ctx.stream);
+    ctx.launched();
+  } else {
     // split tiles are summed by the last CTA of each group (no second launch)
     ProfScope ps(ctx, "gemm_fp64", P.bytes, P.flops);
     launch_gemm_fp64((const GemmTile*)P.tiles->ptr, P.ntiles, A, B, C, ws,
@@ -251,10 +395,12 @@ uint64_t sector_histogram_key(const std::vector<tn_sector_gemm>& list) {
 const std::vector<Fp64Policy>& fp64_candidates() {
   static const std::vector<Fp64Policy> c = [] {
     std::vector<Fp64Policy> v;
+    v.push_back(Fp64Policy());  // flat
     for (int rule : {0, 1})
       for (int items : {2, 8, 16})
         for (int spread : {0, 1, 2, 4}) {
           Fp64Policy p;
+          p.flat = false;
           p.tn_rule = rule;
           p.items_per_sm = items;
           p.spread = spread;
@@ -279,7 +425,7 @@ static Fp64Policy tune_fp64(Ctx& ctx, uint64_t key, const std::vector<tn_sector_
   TN_CUDA(cudaEventCreate(&e1));
   auto time_of = [&](const Fp64Policy& pol) -> float {
     auto P = get_fp64_plan(ctx, list, pol, vw, table);
-    if (!P->ntiles) return -1.0f;
+    if (!P->ntiles && !P->nflat) return -1.0f;
     launch_fp64_plan(ctx, *P, A, B, C, views, pool);  // warm the plan and the caches
     TN_CUDA(cudaEventRecord(e0, ctx.stream));
     for (int r = 0; r < 3; r++) launch_fp64_plan(ctx, *P, A, B, C, views, pool);
@@ -329,7 +475,7 @@ static void run_fp64(Ctx& ctx, const std::vector<tn_sector_gemm>& list, const do
     }
   }
   auto P = get_fp64_plan(ctx, list, pol);
-  if (!P->ntiles) return;
+  if (!P->ntiles && !P->nflat) return;
   launch_fp64_plan(ctx, *P, A, B, C);
 }
 
@@ -539,7 +685,7 @@ void run_sector_gemms_views(Ctx& ctx, int mode, const std::vector<tn_sector_gemm
         pol = tune_fp64(ctx, key, list, A, B, C, &vw, T.get(), views, pool);
     }
     auto P = get_fp64_plan(ctx, list, pol, &vw, T.get());
-    if (P->ntiles) launch_fp64_plan(ctx, *P, A, B, C, views, pool);
+    if (P->ntiles || P->nflat) launch_fp64_plan(ctx, *P, A, B, C, views, pool);
   };
   const bool tuned = ctx.route_tuned.count(route_key(mode, list)) > 0;
   const GemmRoute route = tune_route(ctx, mode, list, fused, fp64, (decltype(fp64)*)nullptr);

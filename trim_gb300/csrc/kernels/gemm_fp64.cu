@@ -1,7 +1,11 @@
 // Plain FP64 grouped sector GEMM: every C_q = A_q . B_q of one contraction
 // (contract's per-sector matrixMul, tensor-network/lib/UniTensorTools.cpp:191-203;
 // row-major dgemm, numeric/lapack/lib/uni10_lapack_cpu.cpp:41-44) in one
-// launch over a device work list of output tiles.
+// launch over a device work list of output tiles: the form for lists with a
+// sector of 2^23 outputs and more (padding is nothing there, and a tile loads
+// 1.25 operands per FMA where the flat form of gemm_fp64_flat.cu loads 2), for
+// the fixed-scratch entry point, whose work list is bounded, and the
+// autotuner's other candidates.
 //
 // An operand may be read through views of its unpermuted source (the permute
 // fused into the operand load, see ViewHdr): K is then walked in segments
