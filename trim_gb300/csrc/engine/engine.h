@@ -462,6 +462,13 @@ void launch_fill(double* p, int64_t n, double v, cudaStream_t s);
 void launch_tc_maxima(const TcSector* secs, int nsec, const int64_t* a_ts, int64_t a_tiles, const int64_t* b_ts,
                       int64_t b_tiles, const double* A, const double* B, unsigned long long* amax,
                       unsigned long long* bmax, int64_t nmax, int num_sms, cudaStream_t s);
+// both in one pass over the operands; items: (sector, s) for the 16-column
+// strip s of B, (sector, -1 - r) for the rows 8 r .. 8 r + 7 of A, or its row r
+// where K > kRowWarp
+constexpr int kRowWarp = 2000;
+void launch_tc_slice_once(int ns, const TcSector* secs, const int2* items, int nitems, const double* A,
+                          const double* B, unsigned long long* ea, unsigned long long* eb, uint8_t* images,
+                          int num_sms, cudaStream_t s);
 void launch_tc_slices(int ns, const TcSector* secs, int nsec, const int64_t* a_ts, int64_t a_tiles,
                       const int64_t* b_ts, int64_t b_tiles, const double* A, const double* B,
                       const unsigned long long* amax, const unsigned long long* bmax, uint8_t* images, int num_sms,
@@ -483,9 +490,9 @@ size_t tc_fused_smem(int ns);
 void launch_tc_fused(int ns, const TcSector* secs, const int4* items, int nitems, const double* A, const double* B,
                      double* C, const ViewHdr* views, const int64_t* pool, int* err, int grid, int rpi,
                      cudaStream_t s);
-// C tile = sum over the K ranges of its FP64 partial tiles, in range order
-void launch_tc_reduce(const TcSector* secs, const int4* ritems, int nred, const double* part, double* C, int grid,
-                      cudaStream_t s);
+// C tile = sum over the K ranges of its FP64 partial tiles, in range order, scaled
+void launch_tc_reduce(int ns, const TcSector* secs, const int4* ritems, int nred, const double* part, double* C,
+                      const unsigned long long* ea, const unsigned long long* eb, int grid, cudaStream_t s);
 void launch_scale(double* p, int64_t n, double a, cudaStream_t s);
 
 // A rows x cols piece of a product with a diagonal factor (RDotR's

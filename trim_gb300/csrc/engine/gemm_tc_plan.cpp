@@ -21,10 +21,11 @@ struct TcPlan {
   std::vector<tn_sector_gemm> list;
   int ns = kSplitDigits;
   DevBufP meta;
-  size_t off_secs = 0, off_rb = 0, off_cb = 0, off_at = 0, off_bt = 0, off_it = 0, off_rit = 0;
+  size_t off_secs = 0, off_si = 0, off_at = 0, off_bt = 0, off_it = 0, off_rit = 0;
   int nsec = 0, nitems = 0, nred = 0;
+  int nslice = 0;  // items of the one-pass slicing, 0: tile by tile
   int64_t part_elems = 0;  // FP64 partial tiles of the K-split sectors
-  int64_t rows = 0, cols = 0, nrb = 0, ncb = 0, a_tiles = 0, b_tiles = 0, img = 0;
+  int64_t rows = 0, cols = 0, max_k = 0, a_tiles = 0, b_tiles = 0, img = 0;
   double flops = 0, in_bytes = 0;
 };
 
@@ -43,7 +44,7 @@ static std::shared_ptr<TcPlan> build_tc_plan(Ctx& ctx, const std::vector<tn_sect
   P->list = list;
   P->ns = ns;
   std::vector<TcSector> secs;
-  std::vector<int64_t> rb(1, 0), cb(1, 0), ats(1, 0), bts(1, 0);
+  std::vector<int64_t> ats(1, 0), bts(1, 0);
   std::vector<int4> items;
   for (const auto& g : list) {
     if (g.M <= 0 || g.N <= 0 || g.K <= 0) continue;
@@ -68,8 +69,7 @@ static std::shared_ptr<TcPlan> build_tc_plan(Ctx& ctx, const std::vector<tn_sect
     P->img += (int64_t)s.nmt * s.nkt * ns * kTM * kTK * 2;
     s.b_img = P->img;
     P->img += (int64_t)s.nnt * s.nkt * ns * kTN * kTK * 2;
-    P->nrb += s.nmt;
-    P->ncb += s.nnt;
+    P->max_k = std::max<int64_t>(P->max_k, g.K);
     P->a_tiles += (int64_t)s.nmt * s.nkt;
     P->b_tiles += (int64_t)s.nnt * s.nkt;
     s.nsplit = 1;
@@ -77,8 +77,6 @@ static std::shared_ptr<TcPlan> build_tc_plan(Ctx& ctx, const std::vector<tn_sect
     s.p_off = -1;
     s.a_vw = s.b_vw = -1;
     secs.push_back(s);
-    rb.push_back(P->nrb);
-    cb.push_back(P->ncb);
     ats.push_back(P->a_tiles);
     bts.push_back(P->b_tiles);
     P->flops += 2.0 * g.M * g.N * g.K;
@@ -127,23 +125,37 @@ static std::shared_ptr<TcPlan> build_tc_plan(Ctx& ctx, const std::vector<tn_sect
   P->nitems = (int)items.size();
   P->nred = (int)ritems.size();
   if (!P->nsec) return P;
+  // One pass over the operands, an item over all of K, unless that leaves most of
+  // the chip idle on long rows: fewer items than CTAs in flight and K beyond what
+  // an item of A keeps.  There the maxima and the images are made tile by tile
+  // in two launches (as for a list whose items would not number in 32 bits).
+  int64_t nsl = 0;
+  for (const auto& s : secs) nsl += cdiv(s.N, 16) + (s.K > kRowWarp ? s.M : cdiv(s.M, 8));
+  std::vector<int2> sitems;
+  if (nsl < INT32_MAX / 2 && (nsl >= 3 * (int64_t)ctx.num_sms || P->max_k <= 8192)) {
+    sitems.reserve(nsl);
+    for (int g = 0; g < P->nsec; g++)
+      for (int64_t c = 0; c < cdiv(secs[g].N, 16); c++) sitems.push_back(make_int2(g, (int)c));
+    for (int g = 0; g < P->nsec; g++)
+      for (int64_t r = 0; r < (secs[g].K > kRowWarp ? secs[g].M : cdiv(secs[g].M, 8)); r++)
+        sitems.push_back(make_int2(g, (int)(-1 - r)));
+  }
+  P->nslice = (int)sitems.size();
   const int n1 = P->nsec + 1;
   P->off_secs = 0;
-  P->off_rb = P->off_secs + P->nsec * sizeof(TcSector);
-  P->off_cb = P->off_rb + n1 * sizeof(int64_t);
-  P->off_at = P->off_cb + n1 * sizeof(int64_t);
+  P->off_at = P->off_secs + P->nsec * sizeof(TcSector);
   P->off_bt = P->off_at + n1 * sizeof(int64_t);
   P->off_it = (P->off_bt + n1 * sizeof(int64_t) + 15) & ~(size_t)15;
   P->off_rit = P->off_it + items.size() * sizeof(int4);
-  size_t bytes = P->off_rit + ritems.size() * sizeof(int4);
+  P->off_si = P->off_rit + ritems.size() * sizeof(int4);
+  size_t bytes = P->off_si + sitems.size() * sizeof(int2);
   std::vector<uint8_t> meta(bytes);
   std::memcpy(meta.data() + P->off_secs, secs.data(), P->nsec * sizeof(TcSector));
-  std::memcpy(meta.data() + P->off_rb, rb.data(), n1 * sizeof(int64_t));
-  std::memcpy(meta.data() + P->off_cb, cb.data(), n1 * sizeof(int64_t));
   std::memcpy(meta.data() + P->off_at, ats.data(), n1 * sizeof(int64_t));
   std::memcpy(meta.data() + P->off_bt, bts.data(), n1 * sizeof(int64_t));
   std::memcpy(meta.data() + P->off_it, items.data(), items.size() * sizeof(int4));
   if (!ritems.empty()) std::memcpy(meta.data() + P->off_rit, ritems.data(), ritems.size() * sizeof(int4));
+  if (!sitems.empty()) std::memcpy(meta.data() + P->off_si, sitems.data(), sitems.size() * sizeof(int2));
   P->meta = std::make_shared<DevBuf>(bytes, ctx);
   TN_CUDA(cudaMemcpyAsync(P->meta->ptr, meta.data(), bytes, cudaMemcpyHostToDevice, ctx.stream));
   TN_CUDA(cudaStreamSynchronize(ctx.stream));  // the host copy dies here
@@ -190,13 +202,18 @@ void run_tc_gemms(Ctx& ctx, int ns, const std::vector<tn_sector_gemm>& list, con
   int* err = ctx.device_error_word();
   const int64_t* ats = (const int64_t*)(mb + P->off_at);
   const int64_t* bts = (const int64_t*)(mb + P->off_bt);
-  {
-    ProfScope ps(ctx, "tc_maxima", P->in_bytes, 0);
-    launch_tc_maxima(dsecs, P->nsec, ats, P->a_tiles, bts, P->b_tiles, A, B, ea, eb, P->rows + P->cols, ctx.num_sms,
-                     ctx.stream);
+  if (P->nslice) {
+    ProfScope ps(ctx, "tc_slice", P->in_bytes * (1.0 + 0.25 * ns), 0);
+    launch_tc_slice_once(ns, dsecs, (const int2*)(mb + P->off_si), P->nslice, A, B, ea, eb, images, ctx.num_sms,
+                         ctx.stream);
     ctx.launched();
-  }
-  {
+  } else {
+    {
+      ProfScope ps(ctx, "tc_maxima", P->in_bytes, 0);
+      launch_tc_maxima(dsecs, P->nsec, ats, P->a_tiles, bts, P->b_tiles, A, B, ea, eb, P->rows + P->cols, ctx.num_sms,
+                       ctx.stream);
+      ctx.launched();
+    }
     ProfScope ps(ctx, "tc_slice", P->in_bytes + (double)P->img, 0);
     launch_tc_slices(ns, dsecs, P->nsec, ats, P->a_tiles, bts, P->b_tiles, A, B, ea, eb, images, ctx.num_sms,
                      ctx.stream);
@@ -216,7 +233,7 @@ void run_tc_gemms(Ctx& ctx, int ns, const std::vector<tn_sector_gemm>& list, con
   if (P->nred > 0) {
     ProfScope ps(ctx, "tc_reduce", 0, 0);
     const int grid = (int)std::min<int64_t>((int64_t)P->nred, (int64_t)ctx.num_sms * 4);
-    launch_tc_reduce(dsecs, (const int4*)(mb + P->off_rit), P->nred, part, C, grid, ctx.stream);
+    launch_tc_reduce(ns, dsecs, (const int4*)(mb + P->off_rit), P->nred, part, C, ea, eb, grid, ctx.stream);
     ctx.launched();
   }
 }

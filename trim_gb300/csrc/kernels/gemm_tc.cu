@@ -229,7 +229,234 @@ __device__ __forceinline__ void slice_b_tile(const TcSector* __restrict__ secs, 
   }
 }
 
-// every A tile, then every B tile, in one launch
+// ---------------------------------------------------------------- one pass
+// Maxima and images of an operand in one kernel: an item is 8 rows of A (a warp
+// each; one row beyond kRowWarp k) or a strip of 16 columns of B, over all of
+// K.  What an item holds in shared memory (74 KB, three CTAs per SM: rows of
+// up to kRowKeep k per warp or 8192 per CTA, strips of up to kWideK) is read from
+// memory once; longer ones are read again, through L2.  Staging is by 8-byte
+// cp.async, consecutive lanes on consecutive addresses whatever a row's
+// alignment; a thread then slices 8 consecutive k.  HBM bound: 8 bytes read and
+// 2 bytes per digit written per element.  Only what the GEMM uses is written:
+// no row past M or column past N (accumulator rows and columns nobody reads),
+// no k past the last 16-k step.
+constexpr int kStageDoubles = 9216, kRowKeep = 1024, kWideK = 576;
+__host__ __device__ constexpr int padded(int k) { return k + (k >> 3); }  // 9 doubles per 8: no bank conflicts
+static_assert(8 * padded(kRowKeep) <= kStageDoubles && padded(8192) <= kStageDoubles && 16 * kWideK <= kStageDoubles,
+              "the staged extents fit");
+
+struct SliceShared {
+  uint32_t part[8][16];
+  unsigned long long full[16];
+};
+
+__device__ __forceinline__ uint32_t abs_hi(double x) { return (uint32_t)__double2hiint(x) & 0x7FFFFFFFu; }
+__device__ __forceinline__ unsigned long long abs_bits(double x) {
+  return (unsigned long long)__double_as_longlong(x) & 0x7FFFFFFFFFFFFFFFull;
+}
+
+// Row i of A by the lanes id, id + n, .. of a warp (n = 32) or a CTA (n = 256).
+// Only the exponent field of the maximum matters (exp_of), so the high words
+// are compared; a row of zeros and subnormals takes the full patterns.
+template <int NS, int n>
+__device__ __forceinline__ void slice_row(const TcSector& S, int64_t i, int id, const double* __restrict__ A,
+                                          unsigned long long* __restrict__ ea, uint8_t* __restrict__ ws, double* buf,
+                                          SliceShared& sh) {
+  constexpr int keep_k = n == 32 ? kRowKeep : 8192, half = keep_k / 2;
+  auto sync = [] {
+    if (n == 32)
+      __syncwarp();
+    else
+      __syncthreads();
+  };
+  const double* src = A + S.a_off + i * S.K;
+  const int kend = (S.K + 15) & ~15;  // the last 16-k step
+  uint8_t* img = ws + S.a_img + (i / kTM) * S.nkt * NS * kATile;
+  const int r = (int)(i % kTM);
+  const bool keep = kend <= keep_k;
+  // k0 .. k0 + len - 1 (zero past K) on their way into the buffer at `at`
+  auto stage = [&](int k0, int len, int at) {
+    for (int k = id; k < min(len, kend - k0); k += n)
+      cp_async8(buf + padded(at + k), k0 + k < S.K ? src + k0 + k : src, k0 + k < S.K);
+    cp_async_commit();
+  };
+  uint32_t hi = 0;
+  if (keep) {
+    sync();  // the buffer's last contents have been read
+    stage(0, keep_k, 0);
+    cp_async_wait<0>();
+    sync();
+    for (int k = id; k < kend; k += n) hi = max(hi, abs_hi(buf[padded(k)]));
+  } else {
+    sync();
+    stage(0, half, 0);  // the first half buffer loads while the maximum is taken
+#pragma unroll 16
+    for (int k = id; k < S.K; k += n) hi = max(hi, abs_hi(__ldg(src + k)));
+  }
+  hi = __reduce_max_sync(0xffffffffu, hi);
+  if (n > 32) {
+    if ((id & 31) == 0) sh.part[id >> 5][0] = hi;
+    if (id == 0) sh.full[0] = 0;
+    __syncthreads();
+#pragma unroll
+    for (int w = 0; w < n / 32; w++) hi = max(hi, sh.part[w][0]);
+  }
+  unsigned long long m = (unsigned long long)hi << 32;
+  if ((hi >> 20) == 0) {
+    m = 0;
+    for (int k = id; k < S.K; k += n) m = max(m, abs_bits(__ldg(src + k)));
+    if (n == 32) {
+#pragma unroll
+      for (int o = 16; o; o >>= 1) m = max(m, __shfl_xor_sync(0xffffffffu, m, o));
+    } else {
+      if (m) atomicMax(&sh.full[0], m);
+      __syncthreads();
+      m = sh.full[0];
+    }
+  }
+  if (id == 0) ea[S.ea_off + i] = m;
+  const int e = exp_of(m);
+  auto slice = [&](int k0, int len, int at) {
+    for (int k = id * 8; k < min(len, kend - k0); k += 8 * n) {
+      double x[8];
+#pragma unroll
+      for (int q = 0; q < 8; q++) x[q] = buf[padded(at + k) + q];
+      store_chunk<NS>(img + (int64_t)((k0 + k) / kTK) * NS * kATile, kATile, r, (k / 8) % 8, x, e);
+    }
+  };
+  if (keep) {
+    slice(0, keep_k, 0);
+  } else {  // half buffers in turn: one loads (from L2) while the other is sliced
+    for (int k0 = 0, at = 0; k0 < kend; k0 += half, at ^= half) {
+      stage(k0 + half, half, at ^ half);
+      cp_async_wait<1>();
+      sync();
+      slice(k0, half, at);
+      sync();
+    }
+    cp_async_wait<0>();
+  }
+}
+
+// where a B image keeps column n of its 64 (image_column's inverse)
+template <int NS>
+__device__ __forceinline__ int image_row(int n) {
+  if (NS != kSplitDigits) return n;
+  return (n & ~15) | ((n & 2) << 2) | ((n & 12) >> 1) | (n & 1);
+}
+
+// 16 columns of B by a CTA: thread (c, g) has column c and the groups g, g +
+// 16, .. of 8 k; it stages the values it slices itself
+template <int NS>
+__device__ __forceinline__ void slice_strip(const TcSector& S, int64_t strip, const double* __restrict__ B,
+                                            unsigned long long* __restrict__ eb, uint8_t* __restrict__ ws, double* buf,
+                                            SliceShared& sh) {
+  constexpr int W = 16, kPass = 8 * 256 / W;
+  const int c = threadIdx.x % W, g = threadIdx.x / W, warp = threadIdx.x >> 5;
+  const int64_t n = strip * W + c;
+  const int cols = n < S.N ? S.K : 0;  // k values this thread's column has
+  const double* src = B + S.b_off + n;
+  const int kend = (S.K + 15) & ~15;
+  const bool keep = kend <= kWideK;
+  auto at = [&](int k) { return k * W + c; };
+  auto load = [&](int k, double(&v)[8]) {
+#pragma unroll
+    for (int q = 0; q < 8; q++) v[q] = k + q < cols ? __ldg(src + (int64_t)(k + q) * S.N) : 0.0;
+  };
+  uint32_t hi = 0;
+  if (keep) {
+#pragma unroll
+    for (int q = 0; q < 8; q++)
+      for (int k = g * 8 + q; k < kend; k += kPass)
+        cp_async8(buf + at(k), k < cols ? src + (int64_t)k * S.N : B, k < cols);
+    cp_async_commit();
+    cp_async_wait<0>();
+    for (int k = g * 8; k < kend; k += kPass)
+#pragma unroll
+      for (int q = 0; q < 8; q++) hi = max(hi, abs_hi(buf[at(k + q)]));
+  } else {
+    for (int k = g * 8; k < cols; k += 2 * kPass) {  // 16 loads in flight
+      double x[8], y[8];
+      load(k, x);
+      load(k + kPass, y);
+#pragma unroll
+      for (int q = 0; q < 8; q++) hi = max(hi, max(abs_hi(x[q]), abs_hi(y[q])));
+    }
+  }
+#pragma unroll
+  for (int o = W; o < 32; o <<= 1) hi = max(hi, __shfl_xor_sync(0xffffffffu, hi, o));
+  __syncthreads();  // the previous item's maxima have been read
+  if ((threadIdx.x & 31) < W) sh.part[warp][c] = hi;
+  if (threadIdx.x < W) sh.full[c] = 0;
+  __syncthreads();
+#pragma unroll
+  for (int w = 0; w < 8; w++) hi = max(hi, sh.part[w][c]);
+  const bool low = (hi >> 20) == 0;  // zero or subnormal column: the full pattern decides
+  if (low) {
+    unsigned long long m = 0;
+    for (int k = g; k < cols; k += 256 / W) m = max(m, abs_bits(__ldg(src + (int64_t)k * S.N)));
+    if (m) atomicMax(&sh.full[c], m);
+  }
+  __syncthreads();
+  const unsigned long long m = low ? sh.full[c] : (unsigned long long)hi << 32;
+  if (g == 0 && n < S.N) eb[S.eb_off + n] = m;
+  if (n >= S.N) return;
+  const int e = exp_of(m);
+  uint8_t* img = ws + S.b_img + (n / kTN) * S.nkt * NS * kBTile;
+  const int r = image_row<NS>((int)(n % kTN));
+  double x[8];
+  if (keep) {
+    for (int k = g * 8; k < kend; k += kPass) {
+#pragma unroll
+      for (int q = 0; q < 8; q++) x[q] = buf[at(k + q)];
+      store_chunk<NS>(img + (int64_t)(k / kTK) * NS * kBTile, kBTile, r, (k / 8) % 8, x, e);
+    }
+  } else {
+    load(g * 8, x);
+    for (int k = g * 8; k < kend; k += kPass) {  // the next group loads while this one is sliced
+      double y[8];
+      load(k + kPass, y);
+      store_chunk<NS>(img + (int64_t)(k / kTK) * NS * kBTile, kBTile, r, (k / 8) % 8, x, e);
+#pragma unroll
+      for (int q = 0; q < 8; q++) x[q] = y[q];
+    }
+  }
+}
+
+// items: (sector, strip of B), or (sector, -1 - row group of A)
+template <int NS>
+__global__ void __launch_bounds__(256, 3) tc_slice_once(const TcSector* __restrict__ secs,
+                                                        const int2* __restrict__ items, int nitems,
+                                                        const double* __restrict__ A, const double* __restrict__ B,
+                                                        unsigned long long* __restrict__ ea,
+                                                        unsigned long long* __restrict__ eb, uint8_t* __restrict__ ws) {
+  __shared__ SliceShared sh;
+  extern __shared__ double stage[];  // kStageDoubles
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  int2 next = items[blockIdx.x];
+  bool cta = false;  // the last item used the buffer as a CTA
+  for (int t = blockIdx.x; t < nitems; t += gridDim.x) {
+    const int2 it = next;
+    if (t + gridDim.x < nitems) next = items[t + gridDim.x];
+    const TcSector& S = secs[it.x];
+    if (it.y >= 0) {
+      __syncthreads();
+      slice_strip<NS>(S, it.y, B, eb, ws, stage, sh);
+      cta = true;
+    } else if (S.K > kRowWarp) {
+      __syncthreads();
+      slice_row<NS, 256>(S, -1 - it.y, threadIdx.x, A, ea, ws, stage, sh);
+      cta = true;
+    } else {
+      if (cta) __syncthreads();
+      cta = false;
+      const int64_t i = (int64_t)(-1 - it.y) * 8 + warp;
+      if (i < S.M) slice_row<NS, 32>(S, i, lane, A, ea, ws, stage + warp * padded(kRowKeep), sh);
+    }
+  }
+}
+
+// every A tile, then every B tile, in one launch (after tc_maxima)
 template <int NS>
 __global__ void __launch_bounds__(256) tc_slices(const TcSector* __restrict__ secs, const int64_t* __restrict__ a_ts,
                                                  const int64_t* __restrict__ b_ts, int nsec, int64_t a_tiles,
@@ -311,17 +538,21 @@ __global__ void __launch_bounds__(kThreadsTc, 1) tc_gemm(const TcSector* __restr
         const uint8_t* a_src = ws + S.a_img + (int64_t)w.y * S.nkt * NS * kATile;
         const uint8_t* b_src = ws + S.b_img + (int64_t)w.z * S.nkt * NS * kBTile;
         const int kb = w.w * S.kts, ke = min(S.nkt, kb + S.kts);  // this item's K range
+        // rows of the images that hold data, to whole groups of 8 rows (1 KB)
+        const uint32_t a_bytes = (uint32_t)((min(kTM, S.M - w.y * kTM) + 7) >> 3) * 1024;
+        const uint32_t b_bytes = (uint32_t)((min(kTN, S.N - w.z * kTN) + 7) >> 3) * 1024;
         for (int kt = kb; kt < ke && ok; kt++) {
           const int sb = nb % kBRing;
           if (!mbar_wait(&sh.emptyB[sb], ((nb / kBRing) & 1) ^ 1, &sh.abort)) { ok = false; break; }
-          mbar_arrive_expect_tx(&sh.fullB[sb], NS * kBTile);
-          bulk_g2s(bbuf + sb * NS * kBTile, b_src + (int64_t)kt * NS * kBTile, NS * kBTile, &sh.fullB[sb]);
+          mbar_arrive_expect_tx(&sh.fullB[sb], NS * b_bytes);
+          for (int s = 0; s < NS; s++)
+            bulk_g2s(bbuf + (sb * NS + s) * kBTile, b_src + ((int64_t)kt * NS + s) * kBTile, b_bytes, &sh.fullB[sb]);
           nb++;
           for (int s = 0; s < NS; s++) {
             const int sa = na % kARing;
             if (!mbar_wait(&sh.emptyA[sa], ((na / kARing) & 1) ^ 1, &sh.abort)) { ok = false; break; }
-            mbar_arrive_expect_tx(&sh.fullA[sa], kATile);
-            bulk_g2s(abuf + sa * kATile, a_src + ((int64_t)kt * NS + s) * kATile, kATile, &sh.fullA[sa]);
+            mbar_arrive_expect_tx(&sh.fullA[sa], a_bytes);
+            bulk_g2s(abuf + sa * kATile, a_src + ((int64_t)kt * NS + s) * kATile, a_bytes, &sh.fullA[sa]);
             na++;
           }
         }
@@ -423,7 +654,9 @@ __global__ void __launch_bounds__(kThreadsTc, 1) tc_gemm(const TcSector* __restr
           const int64_t jj = (int64_t)w.z * kTN + half * kEpiCols + j;
           // one FP64-pipe operation per output (the conversion), the power-of-two
           // scale on the exponent field
-          if (jj < S.N) crow[jj] = scale_pow2((double)v[j], e_i + exp_of(eb[S.eb_off + jj]) - 14);
+          // (a K-split sector's partial tiles are scaled after their sum)
+          if (jj < S.N)
+            crow[jj] = S.nsplit > 1 ? (double)v[j] : scale_pow2((double)v[j], e_i + exp_of(eb[S.eb_off + jj]) - 14);
         }
       }
     }
@@ -435,9 +668,13 @@ __global__ void __launch_bounds__(kThreadsTc, 1) tc_gemm(const TcSector* __restr
   if (warp == 1) tmem_dealloc(tmem, 512);
 }
 
-// one CTA per split output tile: C = sum of its partial tiles in K-range order
+// one CTA per split output tile: C = the sum of its partial tiles in K-range
+// order, scaled by 2^(ea + eb - unit) (the split kernel's partial tiles carry
+// no unit)
 __global__ void __launch_bounds__(256) tc_reduce(const TcSector* __restrict__ secs, const int4* __restrict__ ritems,
-                                                 int nred, const double* __restrict__ part, double* __restrict__ C) {
+                                                 int nred, const double* __restrict__ part, double* __restrict__ C,
+                                                 const unsigned long long* __restrict__ ea,
+                                                 const unsigned long long* __restrict__ eb, int unit) {
   for (int it = blockIdx.x; it < nred; it += gridDim.x) {
     const int4 w = ritems[it];
     const TcSector& S = secs[w.x];
@@ -447,7 +684,7 @@ __global__ void __launch_bounds__(256) tc_reduce(const TcSector* __restrict__ se
       if (i >= S.M || j >= S.N) continue;
       double s = 0.0;
       for (int q = 0; q < S.nsplit; q++) s += p[(int64_t)q * (kTM * kTN) + e];
-      C[S.c_off + i * S.N + j] = s;
+      C[S.c_off + i * S.N + j] = scale_pow2(s, exp_of(ea[S.ea_off + i]) + exp_of(eb[S.eb_off + j]) - unit);
     }
   }
 }
@@ -461,6 +698,22 @@ void launch_tc_maxima(const TcSector* secs, int nsec, const int64_t* a_ts, int64
   TN_CUDA(cudaMemsetAsync(amax, 0, (size_t)nmax * sizeof(unsigned long long), s));  // bmax follows amax
   int g1 = (int)std::min<int64_t>(a_tiles + b_tiles, (int64_t)num_sms * 8);
   tc_maxima<<<g1, 256, 0, s>>>(secs, a_ts, b_ts, nsec, a_tiles, b_tiles, A, B, amax, bmax);
+  TN_CUDA(cudaGetLastError());
+}
+
+void launch_tc_slice_once(int ns, const TcSector* secs, const int2* items, int nitems, const double* A,
+                          const double* B, unsigned long long* ea, unsigned long long* eb, uint8_t* images,
+                          int num_sms, cudaStream_t s) {
+  const int grid = std::min(nitems, num_sms * 3);
+  auto k = ns == kSplitDigits ? tc_slice_once<kSplitDigits> : (ns == 2 ? tc_slice_once<2> : tc_slice_once<1>);
+  constexpr int smem = kStageDoubles * (int)sizeof(double);
+  static bool attr[3] = {false, false, false};  // per instantiation
+  bool& done = attr[ns == kSplitDigits ? 0 : ns];
+  if (!done) {
+    TN_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+    done = true;
+  }
+  k<<<grid, 256, smem, s>>>(secs, items, nitems, A, B, ea, eb, images);
   TN_CUDA(cudaGetLastError());
 }
 
@@ -502,10 +755,10 @@ void launch_tc_gemm(int ns, const TcSector* secs, const int4* items, int nitems,
   TN_CUDA(cudaGetLastError());
 }
 
-void launch_tc_reduce(const TcSector* secs, const int4* ritems, int nred, const double* part, double* C, int grid,
-                      cudaStream_t s) {
+void launch_tc_reduce(int ns, const TcSector* secs, const int4* ritems, int nred, const double* part, double* C,
+                      const unsigned long long* ea, const unsigned long long* eb, int grid, cudaStream_t s) {
   if (nred <= 0) return;
-  tc_reduce<<<grid, 256, 0, s>>>(secs, ritems, nred, part, C);
+  tc_reduce<<<grid, 256, 0, s>>>(secs, ritems, nred, part, C, ea, eb, ns == kSplitDigits ? 0 : 14);
   TN_CUDA(cudaGetLastError());
 }
 

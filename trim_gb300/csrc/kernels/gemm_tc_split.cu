@@ -300,6 +300,10 @@ __global__ void __launch_bounds__(kThreadsSplit, 1) tc_gemm_split(const TcSector
         const uint8_t* a_src = ws + S.a_img + (int64_t)w.y * S.nkt * kDigits * kATile;
         const uint8_t* b_src = ws + S.b_img + (int64_t)w.z * S.nkt * kDigits * kBTile;
         const int kb = w.w * S.kts, ke = min(S.nkt, kb + S.kts);  // this item's K range
+        // rows of the images that hold data: A's to whole groups of 8 rows (1 KB),
+        // B's to the 16 columns that are stored in permuted order
+        const uint32_t a_bytes = (uint32_t)((min(kTM, S.M - w.y * kTM) + 7) >> 3) * 1024;
+        const uint32_t b_bytes = (uint32_t)((min(kTN, S.N - w.z * kTN) + 15) >> 4) * 2048;
         for (int kt = kb; kt < ke && ok; kt++) {
           const int sb = nb % kBRing;
           if (!mbar_wait(&sh.emptyB[sb], ((nb / kBRing) & 1) ^ 1, &sh.abort)) {
@@ -307,9 +311,13 @@ __global__ void __launch_bounds__(kThreadsSplit, 1) tc_gemm_split(const TcSector
             break;
           }
           sh.steps[sb] = min(kTK, S.K - kt * kTK + 15) >> 4;
-          mbar_arrive_expect_tx(&sh.fullB[sb], kDigits * kBTile);
-          bulk_g2s(bbuf + sb * kDigits * kBTile, b_src + (int64_t)kt * kDigits * kBTile, kDigits * kBTile,
-                   &sh.fullB[sb]);
+          uint8_t* bd = bbuf + sb * kDigits * kBTile;
+          const uint8_t* bs = b_src + (int64_t)kt * kDigits * kBTile;
+          mbar_arrive_expect_tx(&sh.fullB[sb], kDigits * b_bytes);
+          if (b_bytes == kBTile)
+            bulk_g2s(bd, bs, kDigits * kBTile, &sh.fullB[sb]);
+          else
+            for (int s = 0; s < kDigits; s++) bulk_g2s(bd + s * kBTile, bs + s * kBTile, b_bytes, &sh.fullB[sb]);
           nb++;
           for (int s = 0; s < kDigits; s++) {
             const int sa = na % kARing;
@@ -317,8 +325,8 @@ __global__ void __launch_bounds__(kThreadsSplit, 1) tc_gemm_split(const TcSector
               ok = false;
               break;
             }
-            mbar_arrive_expect_tx(&sh.fullA[sa], kATile);
-            bulk_g2s(abuf + sa * kATile, a_src + ((int64_t)kt * kDigits + s) * kATile, kATile, &sh.fullA[sa]);
+            mbar_arrive_expect_tx(&sh.fullA[sa], a_bytes);
+            bulk_g2s(abuf + sa * kATile, a_src + ((int64_t)kt * kDigits + s) * kATile, a_bytes, &sh.fullA[sa]);
             na++;
           }
         }
@@ -433,7 +441,8 @@ __global__ void __launch_bounds__(kThreadsSplit, 1) tc_gemm_split(const TcSector
                                      : C + S.c_off + i0 * S.N + j0 + p4;
           const int64_t ld = S.nsplit > 1 ? kTN : S.N;
           const int rows = (int)min((int64_t)32, S.M - i0);
-          const bool wide = plain && nc == kEpiCols && k0 == kb && (((uintptr_t)out | (uintptr_t)(8 * ld)) & 31) == 0;
+          const bool several = S.nsplit > 1 || ke - kb > kSegTiles;  // partial tiles or segments
+          const bool wide = plain && nc == kEpiCols && (S.nsplit > 1 || !several) && (((uintptr_t)out | (uintptr_t)(8 * ld)) & 31) == 0;
 #pragma unroll
           for (int t = 0; t < 4; t++) {  // row r + 8 t: values 8 (t / 2) + 2 (t % 2) + {0, 1, 4, 5}
             const int e_i = __shfl_sync(0xffffffffu, e_row, r + 8 * t);
@@ -443,14 +452,20 @@ __global__ void __launch_bounds__(kThreadsSplit, 1) tc_gemm_split(const TcSector
 #pragma unroll
             for (int c = 0; c < 4; c++) {
               const long long x = acc[8 * (t >> 1) + 2 * (t & 1) + 4 * (c >> 1) + (c & 1)];
-              v[c] = plain ? fixed_to_double_inrange(x, e_i + ej[c]) : fixed_to_double(x, e_i + ej[c]);
+              // several sums to add: without the scales, which the last addition is
+              // followed by (so a result in the subnormal range is rounded once)
+              const int q = several ? -kUnit : e_i + ej[c];
+              v[c] = plain ? fixed_to_double_inrange(x, q) : fixed_to_double(x, q);
             }
             if (wide) {
               if (live) store4(crow, v);
             } else {
 #pragma unroll
               for (int c = 0; c < 4; c++)
-                if (live && p4 + c < nc) crow[c] = k0 > kb ? crow[c] + v[c] : v[c];  // the segments of a long K, in order
+                if (live && p4 + c < nc) {
+                  if (k0 > kb) v[c] += crow[c];  // the segments of a long K, in order
+                  crow[c] = several && S.nsplit == 1 && k1 == ke ? scale_pow2(v[c], e_i + ej[c] + kUnit) : v[c];
+                }
             }
           }
         }

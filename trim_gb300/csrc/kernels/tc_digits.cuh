@@ -24,6 +24,23 @@ __device__ __forceinline__ int exp_of(uint64_t maxbits) {
   return ef - 1022;
 }
 
+// The FP32 bit pattern of x * 2^(7 - e), rounded to nearest even, the scaling
+// done on the exponent field.  Integer operations: a cvt.f32.f64 runs on the
+// FP64 pipe (two per clock and SM), which made the one-digit slices take longer
+// than the six of the split form.
+__device__ __forceinline__ uint32_t scaled_f32_bits(double x, int e) {
+  const uint32_t hi = (uint32_t)__double2hiint(x), lo = (uint32_t)__double2loint(x);
+  const int ef = (int)((hi >> 20) & 0x7FFu);
+  const int fe = ef + 7 - e - 896;  // the FP32 exponent field
+  if (ef != 0 && fe >= 1 && fe <= 254) {
+    const uint32_t mant = ((hi & 0xFFFFFu) << 3) | (lo >> 29);
+    const uint32_t up = ((lo & 0x1FFFFFFFu) + 0x0FFFFFFFu + (mant & 1u)) >> 29;
+    return (hi & 0x80000000u) | (((uint32_t)fe << 23) + mant + up);
+  }
+  if (((hi << 1) | lo) == 0) return hi;               // zero of either sign
+  return __float_as_uint((float)ldexp(x, 7 - e));     // subnormal or far below the row's scale
+}
+
 // ---------------------------------------------------------------- slicing
 // 8 consecutive-k values of one row -> NS slices of 8 bf16 (packed in uint4).
 //
@@ -46,67 +63,64 @@ __device__ __forceinline__ int exp_of(uint64_t maxbits) {
 template <int NS>
 __device__ __forceinline__ void make_slices(const double (&x)[8], int e, uint4 (&out)[NS]) {
   static_assert(NS == 1 || NS == 6 || NS == 7, "6 or 7 digits (split) or one BF16 slice (fast)");
-  uint32_t hbits[NS][8];
+  uint32_t packed[NS][4];
 #pragma unroll
-  for (int i = 0; i < 8; i++) {
-    const uint64_t bits = (uint64_t)__double_as_longlong(x[i]);
-    const int ef = (int)((bits >> 52) & 0x7FF);
-    if (NS == 1) {
-      float f;
-      const int nex = ef + 7 - e;  // biased exponent of x * 2^(7-e)
-      if (ef != 0 && nex >= 1 && nex <= 2046)
-        f = __double2float_rn(__longlong_as_double(
-            (long long)((bits & ~(0x7FFull << 52)) | ((uint64_t)nex << 52))));
-      else
-        f = (float)ldexp(x[i], 7 - e);  // zero, subnormal or far below the row's scale
-      hbits[0][i] = (uint32_t)__bfloat16_as_ushort(__float2bfloat16_rn(f)) << 16;
-    } else {
-      uint64_t mant = bits & ((1ull << 52) - 1);
-      int E = -1022;
-      if (ef) {
-        mant |= 1ull << 52;
-        E = ef - 1023;
-      }
-      const int sh = (NS == 7 ? 3 : 0) + e - E;  // X = mant * 2^(E - 52) * 2^(49 - e), or 2^(52 - e) for 6 digits
-      const uint64_t X = (sh >= 64) ? 0ull : (sh > 0 ? ((mant + (1ull << (sh - 1))) >> sh) : (mant << (-sh)));
-      const long long V = (bits >> 63) ? -(long long)X : (long long)X;
-      if constexpr (NS == 6) {
-        const uint64_t Y = (uint64_t)(V + 17626613022976ll);  // + 256 * (512^5 - 1) / 511
-        const uint32_t lo = (uint32_t)Y, hi = (uint32_t)(Y >> 32);
-        // the five lower digits plus 256, in the low bits
-        const uint32_t d[6] = {(uint32_t)((int)hi >> 13),
-                               (hi >> 4) & 511u,
-                               __funnelshift_r(lo, hi, 27) & 511u,
-                               (lo >> 18) & 511u,
-                               (lo >> 9) & 511u,
-                               lo & 511u};
-        const float magic = __uint_as_float(0x4B400000u);  // 1.5 * 2^23
+  for (int j = 0; j < 4; j++) {  // pair by pair, so few digits are held at once
+    uint32_t hbits[NS][2];
 #pragma unroll
-        for (int s = 0; s < 6; s++)
-          hbits[s][i] = __float_as_uint(__uint_as_float(0x4B400000u + d[s]) - (s ? magic + 256.f : magic));
-      } else if constexpr (NS == 7) {
-        const uint64_t Y = (uint64_t)(V + 2216338399296ll);  // + 64 * (128^6 - 1) / 127
-        const uint32_t lo = (uint32_t)Y, hi = (uint32_t)(Y >> 32);
-        int d[7];
-        d[6] = (int)(lo & 127u) - 64;
-        d[5] = (int)((lo >> 7) & 127u) - 64;
-        d[4] = (int)((lo >> 14) & 127u) - 64;
-        d[3] = (int)((lo >> 21) & 127u) - 64;
-        d[2] = (int)(__funnelshift_r(lo, hi, 28) & 127u) - 64;
-        d[1] = (int)((hi >> 3) & 127u) - 64;
-        d[0] = (int)hi >> 10;
+    for (int i = 0; i < 2; i++) {
+      const uint64_t bits = (uint64_t)__double_as_longlong(x[2 * j + i]);
+      const int ef = (int)((bits >> 52) & 0x7FF);
+      if (NS == 1) {
+        hbits[0][i] = (uint32_t)__bfloat16_as_ushort(__float2bfloat16_rn(__uint_as_float(scaled_f32_bits(x[2 * j + i], e)))) << 16;
+      } else {
+        uint64_t mant = bits & ((1ull << 52) - 1);
+        int E = -1022;
+        if (ef) {
+          mant |= 1ull << 52;
+          E = ef - 1023;
+        }
+        const int sh = (NS == 7 ? 3 : 0) + e - E;  // X = mant * 2^(E - 52) * 2^(49 - e), or 2^(52 - e) for 6 digits
+        const uint64_t X = (sh >= 64) ? 0ull : (sh > 0 ? ((mant + (1ull << (sh - 1))) >> sh) : (mant << (-sh)));
+        const long long V = (bits >> 63) ? -(long long)X : (long long)X;
+        if constexpr (NS == 6) {
+          const uint64_t Y = (uint64_t)(V + 17626613022976ll);  // + 256 * (512^5 - 1) / 511
+          const uint32_t lo = (uint32_t)Y, hi = (uint32_t)(Y >> 32);
+          // the five lower digits plus 256, in the low bits
+          const uint32_t d[6] = {(uint32_t)((int)hi >> 13),
+                                 (hi >> 4) & 511u,
+                                 __funnelshift_r(lo, hi, 27) & 511u,
+                                 (lo >> 18) & 511u,
+                                 (lo >> 9) & 511u,
+                                 lo & 511u};
+          const float magic = __uint_as_float(0x4B400000u);  // 1.5 * 2^23
 #pragma unroll
-        for (int s = 0; s < 7; s++) {
-          const float magic = __uint_as_float(0x4B400000u - ((uint32_t)(7 * s) << 23));  // 1.5 * 2^(23-7s)
-          hbits[s][i] = __float_as_uint(__uint_as_float(__float_as_uint(magic) + (uint32_t)d[s]) - magic);
+          for (int s = 0; s < 6; s++)
+            hbits[s][i] = __float_as_uint(__uint_as_float(0x4B400000u + d[s]) - (s ? magic + 256.f : magic));
+        } else if constexpr (NS == 7) {
+          const uint64_t Y = (uint64_t)(V + 2216338399296ll);  // + 64 * (128^6 - 1) / 127
+          const uint32_t lo = (uint32_t)Y, hi = (uint32_t)(Y >> 32);
+          int d[7];
+          d[6] = (int)(lo & 127u) - 64;
+          d[5] = (int)((lo >> 7) & 127u) - 64;
+          d[4] = (int)((lo >> 14) & 127u) - 64;
+          d[3] = (int)((lo >> 21) & 127u) - 64;
+          d[2] = (int)(__funnelshift_r(lo, hi, 28) & 127u) - 64;
+          d[1] = (int)((hi >> 3) & 127u) - 64;
+          d[0] = (int)hi >> 10;
+#pragma unroll
+          for (int s = 0; s < 7; s++) {
+            const float magic = __uint_as_float(0x4B400000u - ((uint32_t)(7 * s) << 23));  // 1.5 * 2^(23-7s)
+            hbits[s][i] = __float_as_uint(__uint_as_float(__float_as_uint(magic) + (uint32_t)d[s]) - magic);
+          }
         }
       }
     }
+#pragma unroll
+    for (int s = 0; s < NS; s++) packed[s][j] = __byte_perm(hbits[s][0], hbits[s][1], 0x7632);
   }
 #pragma unroll
-  for (int s = 0; s < NS; s++)
-    out[s] = make_uint4(__byte_perm(hbits[s][0], hbits[s][1], 0x7632), __byte_perm(hbits[s][2], hbits[s][3], 0x7632),
-                        __byte_perm(hbits[s][4], hbits[s][5], 0x7632), __byte_perm(hbits[s][6], hbits[s][7], 0x7632));
+  for (int s = 0; s < NS; s++) out[s] = make_uint4(packed[s][0], packed[s][1], packed[s][2], packed[s][3]);
 }
 
 // TF32 fast mode: 8 consecutive-k values of one row as TF32 patterns of
@@ -117,15 +131,7 @@ __device__ __forceinline__ void make_tf32(const double (&x)[8], int e, uint4 (&o
   uint32_t w[8];
 #pragma unroll
   for (int i = 0; i < 8; i++) {
-    const uint64_t bits = (uint64_t)__double_as_longlong(x[i]);
-    const int ef = (int)((bits >> 52) & 0x7FF);
-    const int nex = ef + 7 - e;
-    float f;
-    if (ef != 0 && nex >= 1 && nex <= 2046)
-      f = __double2float_rn(__longlong_as_double((long long)((bits & ~(0x7FFull << 52)) | ((uint64_t)nex << 52))));
-    else
-      f = (float)ldexp(x[i], 7 - e);  // zero, subnormal or far below the row's scale
-    const uint32_t u = __float_as_uint(f);
+    const uint32_t u = scaled_f32_bits(x[i], e);
     w[i] = ((u & 0x7F800000u) == 0x7F800000u) ? u : ((u + 0x1000u) & 0xFFFFE000u);
   }
   out[0] = make_uint4(w[0], w[1], w[2], w[3]);
