@@ -54,3 +54,21 @@ def test_exact_products(env, mode, grouped):
         c = C.cpu().numpy()
         for (m, n, k, _, _, off), w in zip(gemms, want):
             assert np.array_equal(c[off:off + m * n].reshape(m, n), w), (mode, m, n, k)
+
+
+@pytest.mark.parametrize("mode", ["bf16_tiled", "tf32_tc", "split_tiled"])
+@pytest.mark.parametrize("m,n,k", [(9000, 323, 70), (19400, 577, 33), (2050, 1300, 129), (640, 4100, 64), (8, 9728, 8300)])
+def test_wide_items_exact(env, mode, m, n, k):
+    """Enough output tiles for items of two and four column tiles, the last of
+    them ragged, and two K ranges of more than 4096 k; small integers, so every
+    mode's result is exact."""
+    torch, tu = env
+    rng = np.random.default_rng(m)
+    a = rng.integers(-8, 9, (m, k)).astype(np.float64)
+    b = rng.integers(-8, 9, (k, n)).astype(np.float64)
+    A, B = torch.from_numpy(a.ravel()).cuda(), torch.from_numpy(b.ravel()).cuda()
+    C = torch.full((m * n,), float("nan"), dtype=torch.float64, device="cuda")
+    torch.cuda.synchronize()
+    tu.contract_sectors(mode, [(m, n, k, 0, 0, 0)], A.data_ptr(), B.data_ptr(), C.data_ptr())
+    tu.sync()
+    assert np.array_equal(C.cpu().numpy().reshape(m, n), a @ b)

@@ -473,15 +473,18 @@ void launch_tc_slices(int ns, const TcSector* secs, int nsec, const int64_t* a_t
                       const int64_t* b_ts, int64_t b_tiles, const double* A, const double* B,
                       const unsigned long long* amax, const unsigned long long* bmax, uint8_t* images, int num_sms,
                       cudaStream_t s);
-// the fast modes' GEMM (ns = 1: BF16, 2: TF32) and the split mode's, on images
-// of kSplitDigits digits per operand tile (part: FP64 partial tiles of K-split sectors)
+// the split mode's GEMM, on images of kSplitDigits digits per operand tile
+// (part: FP64 partial tiles of K-split sectors)
 constexpr int kSplitDigits = 6;
 void launch_tc_gemm_split(const TcSector* secs, const int4* items, int nitems, const uint8_t* ws,
                           const unsigned long long* ea, const unsigned long long* eb, double* C, double* part,
                           int* err, int grid, cudaStream_t s);
-void launch_tc_gemm(int ns, const TcSector* secs, const int4* items, int nitems, const uint8_t* ws,
-                    const unsigned long long* ea, const unsigned long long* eb, double* C, double* part, int* err,
-                    int grid, cudaStream_t s);
+// the fast modes' (ns = 1: BF16, 2: TF32), items of up to `wide` <= kFastWide
+// adjacent 64-column tiles
+constexpr int kFastWide = 4;
+void launch_tc_gemm_fast(int ns, const TcSector* secs, const int4* items, int nitems, int wide, const uint8_t* ws,
+                         const unsigned long long* ea, const unsigned long long* eb, double* C, double* part, int* err,
+                         int grid, cudaStream_t s);
 // Fused form for contractions of small sectors: one launch per contraction,
 // one CTA per 128 x 64 output tile (items: sector, row tile, column tile),
 // which slices its operands 64 k at a time into shared memory and runs the

@@ -23,6 +23,7 @@ struct TcPlan {
   DevBufP meta;
   size_t off_secs = 0, off_si = 0, off_at = 0, off_bt = 0, off_it = 0, off_rit = 0;
   int nsec = 0, nitems = 0, nred = 0;
+  int wide = 1;    // 64-column tiles per item (fast modes)
   int nslice = 0;  // items of the one-pass slicing, 0: tile by tile
   int64_t part_elems = 0;  // FP64 partial tiles of the K-split sectors
   int64_t rows = 0, cols = 0, max_k = 0, a_tiles = 0, b_tiles = 0, img = 0;
@@ -89,6 +90,15 @@ static std::shared_ptr<TcPlan> build_tc_plan(Ctx& ctx, const std::vector<tn_sect
   for (const auto& s : secs) tiles += (int64_t)s.nmt * s.nnt;
   const int64_t want = 2 * (int64_t)ctx.num_sms;
   const int64_t factor = tiles > 0 ? std::max<int64_t>(1, (want + tiles - 1) / tiles) : 1;
+  // A fast-mode item spans up to four column tiles (N = 256 MMAs, half the
+  // operand bytes per flop of 64 columns), fewer where that would leave SMs with
+  // less than two items each.  The K ranges do not depend on it.
+  if (ns != kSplitDigits)
+    for (P->wide = kFastWide; P->wide > 1; P->wide /= 2) {
+      int64_t n = 0;
+      for (const auto& s : secs) n += (int64_t)s.nmt * cdiv(s.nnt, P->wide);
+      if (n * std::min<int64_t>(factor, 64) >= want) break;
+    }
   std::vector<int4> ritems;
   for (int idx = 0; idx < (int)secs.size(); idx++) {
     TcSector& s = secs[idx];
@@ -110,7 +120,8 @@ static std::shared_ptr<TcPlan> build_tc_plan(Ctx& ctx, const std::vector<tn_sect
     // shorter tile count, so each image of the longer operand is brought in
     // once and reused by the neighbouring items from L2
     auto add = [&](int mt, int nt) {
-      for (int q = 0; q < s.nsplit; q++) items.push_back(make_int4(idx, mt, nt, q));
+      if (nt % P->wide == 0)
+        for (int q = 0; q < s.nsplit; q++) items.push_back(make_int4(idx, mt, nt, q));
       if (s.nsplit > 1) ritems.push_back(make_int4(idx, mt, nt, 0));
     };
     if (s.nnt <= s.nmt) {
@@ -226,8 +237,8 @@ void run_tc_gemms(Ctx& ctx, int ns, const std::vector<tn_sector_gemm>& list, con
       launch_tc_gemm_split(dsecs, (const int4*)(mb + P->off_it), P->nitems, images, ea, eb, C, part, err, grid,
                            ctx.stream);
     else
-      launch_tc_gemm(ns, dsecs, (const int4*)(mb + P->off_it), P->nitems, images, ea, eb, C, part, err, grid,
-                     ctx.stream);
+      launch_tc_gemm_fast(ns, dsecs, (const int4*)(mb + P->off_it), P->nitems, P->wide, images, ea, eb, C, part, err,
+                          grid, ctx.stream);
     ctx.launched();
   }
   if (P->nred > 0) {

@@ -123,21 +123,6 @@ __device__ __forceinline__ bool warp_wait(uint64_t* bar, uint32_t parity, SplitS
   return __all_sync(0xffffffffu, mbar_wait(bar, parity, &sh->abort));
 }
 
-// Whether a phase completed, without waiting.  The tensor pipe takes few MMAs
-// ahead, so a wait between two groups of MMAs (about 125 clocks even when its
-// phase has completed) would leave it idle: the barriers of the next stage are
-// tested before a stage's MMAs are issued, the answer is there after them, and
-// only a barrier that was not ready yet is waited on.
-__device__ __forceinline__ bool mbar_test(uint64_t* bar, uint32_t parity) {
-  uint32_t ok;
-  asm volatile(
-      "{\n .reg .pred p;\n mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n selp.u32 %0, 1, 0, p;\n}\n"
-      : "=r"(ok)
-      : "r"(smem_u32(bar)), "r"(parity)
-      : "memory");
-  return ok != 0;
-}
-
 // the MMAs of A digit S into levels L..5
 template <int M, int S, int L, bool FULL>
 __device__ __forceinline__ bool split_groups(MmaState& st, uint64_t adesc) {
@@ -238,13 +223,6 @@ __device__ __forceinline__ void tmem_ld32x16x2(uint32_t a, uint32_t b, float (&v
 
 __device__ __forceinline__ void prefetch_l1(const void* p) {
   asm volatile("prefetch.global.L1 [%0];" ::"l"(__cvta_generic_to_global(p)));
-}
-
-// 32 bytes in one store (sm_100 and up); four lanes write a row's 128 bytes
-__device__ __forceinline__ void store4(double* p, const double* v) {
-  asm volatile("st.global.v4.f64 [%0], {%1, %2, %3, %4};" ::"l"(__cvta_generic_to_global(p)), "d"(v[0]), "d"(v[1]),
-               "d"(v[2]), "d"(v[3])
-               : "memory");
 }
 
 __global__ void __launch_bounds__(kThreadsSplit, 1) tc_gemm_split(const TcSector* __restrict__ secs,
@@ -442,7 +420,7 @@ __global__ void __launch_bounds__(kThreadsSplit, 1) tc_gemm_split(const TcSector
           const int64_t ld = S.nsplit > 1 ? kTN : S.N;
           const int rows = (int)min((int64_t)32, S.M - i0);
           const bool several = S.nsplit > 1 || ke - kb > kSegTiles;  // partial tiles or segments
-          const bool wide = plain && nc == kEpiCols && (S.nsplit > 1 || !several) && (((uintptr_t)out | (uintptr_t)(8 * ld)) & 31) == 0;
+          const bool wide = plain && nc == kEpiCols && ke - kb <= kSegTiles && (((uintptr_t)out | (uintptr_t)(8 * ld)) & 31) == 0;
 #pragma unroll
           for (int t = 0; t < 4; t++) {  // row r + 8 t: values 8 (t / 2) + 2 (t % 2) + {0, 1, 4, 5}
             const int e_i = __shfl_sync(0xffffffffu, e_row, r + 8 * t);

@@ -59,6 +59,21 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, volati
   }
 }
 
+// Whether a phase completed, without waiting.  The tensor pipe takes few MMAs
+// ahead, so a wait between two groups of MMAs (about 125 clocks even when its
+// phase has completed) would leave it idle: the barriers of the next stage are
+// tested before a stage's MMAs are issued, the answer is there after them, and
+// only a barrier that was not ready yet is waited on.
+__device__ __forceinline__ bool mbar_test(uint64_t* bar, uint32_t parity) {
+  uint32_t ok;
+  asm volatile(
+      "{\n .reg .pred p;\n mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n selp.u32 %0, 1, 0, p;\n}\n"
+      : "=r"(ok)
+      : "r"(smem_u32(bar)), "r"(parity)
+      : "memory");
+  return ok != 0;
+}
+
 // ---------------------------------------------------------------- async copy
 // 8-byte global -> shared copy without register staging; valid == false
 // writes zeros and reads nothing (src must still be a valid address)
@@ -73,6 +88,13 @@ __device__ __forceinline__ void cp_async_wait() {
   asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
 }
 __device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;" ::: "memory"); }
+
+// 32 bytes in one store (sm_100 and up); four lanes write a row's 128 bytes
+__device__ __forceinline__ void store4(double* p, const double* v) {
+  asm volatile("st.global.v4.f64 [%0], {%1, %2, %3, %4};" ::"l"(__cvta_generic_to_global(p)), "d"(v[0]), "d"(v[1]),
+               "d"(v[2]), "d"(v[3])
+               : "memory");
+}
 
 // ---------------------------------------------------------------- bulk copy
 // global -> shared, completion counted in bytes on the mbarrier
