@@ -148,6 +148,7 @@ class UniTensor {
  private:
   struct NoFill {};
   UniTensor(const std::vector<Bond>& _bonds, const std::string& _name, NoFill);
+  UniTensor(std::vector<Bond>&& _bonds, const std::string& _name, std::shared_ptr<const tn::SectorMap> _smap, bool zero);
   static UniTensor permuted(const UniTensor& src, const std::vector<int>& newLabels, int rowBondNum);
   static UniTensor contract_impl(UniTensor& Ta, UniTensor& Tb, bool fast, bool mutate);
   struct DiagCall;

@@ -42,17 +42,12 @@ BondSig BondSig::changed(int t) const {
 }
 
 std::string sig_key(const std::vector<BondSig>& bonds) {
-  std::string k;
-  k.reserve(bonds.size() * 32);
+  SigKey k(bonds.size());
   for (const auto& b : bonds) {
-    k += (b.type > 0 ? 'I' : 'O');
-    for (size_t i = 0; i < b.q.size(); i++) {
-      k += std::to_string(b.q[i].u1) + ',' + char('0' + b.q[i].prt) + char('0' + b.q[i].prtf) + 'x' +
-           std::to_string(b.deg[i]) + ';';
-    }
-    k += '|';
+    k.bond(b.type, b.q.size());
+    for (size_t i = 0; i < b.q.size(); i++) k.run(b.q[i].u1, b.q[i].prt, b.q[i].prtf, b.deg[i]);
   }
-  return k;
+  return std::move(k.s);
 }
 
 std::vector<BondSig> unpack_bonds(int nbonds, const int* btype, const int* nq, const int* qnum, const int* deg) {
@@ -181,13 +176,15 @@ SectorMapP build_sectormap(const std::vector<BondSig>& bonds) {
 static std::mutex g_smap_mu;
 static std::unordered_map<std::string, SectorMapP> g_smap_cache;
 
+SectorMapP find_sectormap(const std::string& key) {
+  std::lock_guard<std::mutex> lk(g_smap_mu);
+  auto it = g_smap_cache.find(key);
+  return it == g_smap_cache.end() ? nullptr : it->second;
+}
+
 SectorMapP get_sectormap(const std::vector<BondSig>& bonds) {
   std::string k = sig_key(bonds);
-  {
-    std::lock_guard<std::mutex> lk(g_smap_mu);
-    auto it = g_smap_cache.find(k);
-    if (it != g_smap_cache.end()) return it->second;
-  }
+  if (SectorMapP m = find_sectormap(k)) return m;
   SectorMapP m = build_sectormap(bonds);
   std::lock_guard<std::mutex> lk(g_smap_mu);
   if (g_smap_cache.size() > 65536) g_smap_cache.clear();

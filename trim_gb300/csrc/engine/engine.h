@@ -56,6 +56,26 @@ struct BondSig {
   BondSig changed(int t) const;  // Bond::change (data-structure/lib/Bond.cpp:150-157)
   bool operator==(const BondSig& o) const { return type == o.type && q == o.q && deg == o.deg; }
 };
+// The cache key of a bond signature: its numbers as raw 32-bit words, each bond
+// and the whole preceded by its count, so that keys are self-delimiting.  (As
+// decimal text, a dozen small strings per bond, the keys were a third of the
+// host time of an eager contraction of small tensors.)
+struct SigKey {
+  std::string s;
+  explicit SigKey(size_t nbonds) {
+    s.reserve(4 + nbonds * 96);
+    word((int32_t)nbonds);
+  }
+  void word(int32_t v) { s.append((const char*)&v, sizeof(v)); }
+  void bond(int type, size_t runs) {
+    word(type);
+    word((int32_t)runs);
+  }
+  void run(int u1, int prt, int prtf, int deg) {
+    const int32_t w[3] = {u1, prt + 2 * prtf, deg};
+    s.append((const char*)w, sizeof(w));
+  }
+};
 std::string sig_key(const std::vector<BondSig>& bonds);
 std::vector<BondSig> unpack_bonds(int nbonds, const int* btype, const int* nq, const int* qnum, const int* deg);
 
@@ -88,6 +108,7 @@ struct SectorMap {
 using SectorMapP = std::shared_ptr<const SectorMap>;
 SectorMapP build_sectormap(const std::vector<BondSig>& bonds);  // uncached
 SectorMapP get_sectormap(const std::vector<BondSig>& bonds);    // cached by signature
+SectorMapP find_sectormap(const std::string& key);              // the cached map, or null
 
 // ---------------------------------------------------------------- device memory
 struct Ctx;

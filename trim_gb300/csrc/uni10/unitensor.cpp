@@ -41,6 +41,19 @@ std::vector<tn::BondSig> to_sigs(const std::vector<Bond>& bonds) {
   return s;
 }
 
+// the cached sector map of a tensor's bonds, the key taken from the bonds themselves
+static tn::SectorMapP smap_of(const std::vector<Bond>& bonds) {
+  tn::SigKey k(bonds.size());
+  for (const Bond& b : bonds) {
+    const std::vector<Qnum>& q = b.qnums();
+    const std::vector<int>& d = b.qdegs();
+    k.bond(b.type(), q.size());
+    for (size_t i = 0; i < q.size(); i++) k.run(q[i].U1(), (int)q[i].prt(), (int)q[i].prtF(), d[i]);
+  }
+  if (tn::SectorMapP m = tn::find_sectormap(k.s)) return m;
+  return tn::get_sectormap(to_sigs(bonds));
+}
+
 static Qnum to_qnum(const tn::Q& q) { return Qnum((parityFType)q.prtf, q.u1, (parityType)q.prt); }
 
 static std::shared_ptr<DevBuf> alloc_elem(size_t n) {
@@ -92,10 +105,17 @@ UniTensor::UniTensor(const std::vector<Bond>& _bonds, const std::string& _name, 
   initUniT(false);
 }
 
+// the same with the bonds' sector map already at hand
+UniTensor::UniTensor(std::vector<Bond>&& _bonds, const std::string& _name, std::shared_ptr<const tn::SectorMap> _smap,
+                     bool zero)
+    : name(_name), bonds(std::move(_bonds)), status(0), smap(std::move(_smap)) {
+  initUniT(zero);
+}
+
 // UniTensorReal.cpp:1323-1363 -- grouping, allocation, zero fill
 void UniTensor::initUniT(bool zero) {
   if (!bonds.empty()) {
-    smap = tn::get_sectormap(to_sigs(bonds));
+    if (!smap) smap = smap_of(bonds);
     if (smap->blocks.empty()) {
       std::ostringstream err;
       err << "There is no symmetry block with the given bonds:\n";
@@ -415,6 +435,7 @@ UniTensor UniTensor::permuted(const UniTensor& src, const std::vector<int>& newL
     return same;
   }
   std::vector<Bond> outBonds;
+  outBonds.reserve(n);
   for (int b = 0; b < n; b++) outBonds.push_back(src.bonds[rsp[b]]);
   for (int b = 0; b < n; b++) outBonds[b].change(b < rowBondNum ? BD_IN : BD_OUT);
   UniTensor out(outBonds, src.name, NoFill{});
@@ -594,9 +615,10 @@ static PermShape permuted_shape(const UniTensor& src, const std::vector<int>& ne
   for (int i = 0; i < n; i++) inorder &= p.rsp[i] == i;
   p.moves = !(inorder && (int)src.inBondNum() == rowBondNum);
   const std::vector<Bond> b = src.bond();
+  p.bonds.reserve(n);
   for (int j = 0; j < n; j++) p.bonds.push_back(b[p.rsp[j]]);
   for (int j = 0; j < n; j++) p.bonds[j].change(j < rowBondNum ? BD_IN : BD_OUT);
-  p.smap = tn::get_sectormap(to_sigs(p.bonds));  // cached per signature
+  p.smap = smap_of(p.bonds);  // cached per signature
   return p;
 }
 
@@ -761,6 +783,7 @@ UniTensor UniTensor::contract_impl(UniTensor& Ta, UniTensor& Tb, bool fast, bool
     PermShape sa = permuted_shape(Ta, newLabelA, an - conBond);
     PermShape sb = permuted_shape(Tb, newLabelB, conBond);
     std::vector<Bond> cBonds;
+    cBonds.reserve(an + bn - 2 * conBond);
     for (int i = 0; i < an - conBond; i++) cBonds.push_back(sa.bonds[i]);
     for (int i = conBond; i < bn; i++) cBonds.push_back(sb.bonds[i]);
     // every block of Ta with a block of the same charge in Tb is one sector GEMM
@@ -768,8 +791,11 @@ UniTensor UniTensor::contract_impl(UniTensor& Ta, UniTensor& Tb, bool fast, bool
     std::vector<int> a_blk, b_blk;
     const tn::SectorMap* ma = sa.smap.get();
     const tn::SectorMap* mb = sb.smap.get();
-    std::shared_ptr<const tn::SectorMap> mcs = cBonds.empty() ? nullptr : tn::get_sectormap(to_sigs(cBonds));
+    std::shared_ptr<const tn::SectorMap> mcs = cBonds.empty() ? nullptr : smap_of(cBonds);
     const tn::SectorMap* mc = mcs.get();
+    list.reserve(ma->blocks.size());
+    a_blk.reserve(ma->blocks.size());
+    b_blk.reserve(ma->blocks.size());
     for (size_t ia = 0; ia < ma->blocks.size(); ia++) {
       const auto& ba = ma->blocks[ia];
       int ib = mb->find_block(ba.q);
@@ -793,8 +819,9 @@ UniTensor UniTensor::contract_impl(UniTensor& Ta, UniTensor& Tb, bool fast, bool
     }
     // the reference zeroes the result first (UniTensorTools.cpp:185); only
     // blocks no sector GEMM writes need it
-    UniTensor Tc = (!mc || list.size() == mc->blocks.size()) ? UniTensor(cBonds, "", NoFill{}) : UniTensor(cBonds);
-    if (!cBonds.empty()) Tc.setLabel(newLabelC);
+    const bool scalar = cBonds.empty();
+    UniTensor Tc(std::move(cBonds), "", mcs, mc && list.size() != mc->blocks.size());
+    if (!scalar) Tc.setLabel(newLabelC);
     // a diagonal operand contracted over one bond: a row or column scale
     const bool d_a = Ta.diag_ && an == 2 && conBond == 1;
     const bool d_b = !d_a && Tb.diag_ && bn == 2 && conBond == 1;
@@ -949,7 +976,7 @@ void UniTensor::prepare_contract(const UniTensor& Ta, const UniTensor& Tb, Contr
   for (int i = conBond; i < bn; i++) cBonds.push_back(w.pb.bonds[i]);
   const tn::SectorMap* ma = w.pa.smap.get();
   const tn::SectorMap* mb = w.pb.smap.get();
-  std::shared_ptr<const tn::SectorMap> mcs = cBonds.empty() ? nullptr : tn::get_sectormap(to_sigs(cBonds));
+  std::shared_ptr<const tn::SectorMap> mcs = cBonds.empty() ? nullptr : smap_of(cBonds);
   const tn::SectorMap* mc = mcs.get();
   for (const auto& ba : ma->blocks) {
     int ib = mb->find_block(ba.q);
