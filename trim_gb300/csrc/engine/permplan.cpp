@@ -22,7 +22,8 @@ struct Dim {
 //         source-contiguous dim), stores along x.
 // mode 3: mode-0 rows that are short on both sides (a few elements): tz
 //         row-sets of a third dim stacked into a dense [z][y][x] tile, loaded
-//         in source-stride order and stored in destination-stride order.
+//         in source-stride order and stored in destination-stride order; where
+//         that fills less than half a tile, tw values of a fourth dim repeat it.
 // mode 2: when a transpose tile of x and y is small (short bonds, e.g. 24 x
 //         24), a third dim z is stacked into it (tz planes of x by y) so
 //         that each tile still moves thousands of elements; z is the dim
@@ -38,8 +39,8 @@ void choose_tile(PermSub& ps, int es) {
   const int64_t kTile = 4096 / es, kStage = (64 * 65) / es, kRow = 64;
   const int n = ps.ndim;
   ps.ydim = -1;
-  ps.zdim = -1;
-  ps.tz = ps.ntz = 1;
+  ps.zdim = ps.wdim = -1;
+  ps.tz = ps.ntz = ps.tw = ps.ntw = 1;
   ps.mode = 0;
   if (n == 0) {
     ps.tx = ps.ty = 1;
@@ -100,6 +101,24 @@ void choose_tile(PermSub& ps, int es) {
       ps.mode = 3;
       ps.zdim = z;
       ps.tz = (int32_t)tz;
+      // A tile costs two barriers and its index set-up whatever it holds: the
+      // iPEPS operand's 4 x 4 x 64 tiles of 1024 elements (chi = 128, D = 8) ran
+      // 215 us, with 4 values of the second chi bond in a tile 118 us.
+      const int64_t tile = (int64_t)ps.tx * ps.ty * tz;
+      int w = -1;
+      if (tile <= kTile / 2)
+        for (int i = 0; i < n - 1; i++) {
+          if (i == ps.ydim || i == z) continue;
+          const int64_t c = std::min(ps.sstride[i], ps.dstride[i]);
+          if (w < 0 || c < best) {
+            w = i;
+            best = c;
+          }
+        }
+      if (w >= 0) {
+        ps.wdim = w;
+        ps.tw = (int32_t)std::min<int64_t>(ps.dims[w], kTile / tile);
+      }
     }
   }
   if (ps.mode == 1 && (int64_t)ps.tx * ps.ty <= kTile / 2 && n >= 3) {
@@ -124,9 +143,10 @@ void choose_tile(PermSub& ps, int es) {
   ps.ntx = (int32_t)((ps.dims[x] + ps.tx - 1) / ps.tx);
   ps.nty = ps.ydim >= 0 ? (int32_t)((ps.dims[ps.ydim] + ps.ty - 1) / ps.ty) : 1;
   ps.ntz = ps.zdim >= 0 ? (int32_t)((ps.dims[ps.zdim] + ps.tz - 1) / ps.tz) : 1;
+  ps.ntw = ps.wdim >= 0 ? (int32_t)((ps.dims[ps.wdim] + ps.tw - 1) / ps.tw) : 1;
   int64_t outer = 1;
   for (int i = 0; i < n; i++)
-    if (i != x && i != ps.ydim && i != ps.zdim) outer *= ps.dims[i];
+    if (i != x && i != ps.ydim && i != ps.zdim && i != ps.wdim) outer *= ps.dims[i];
   ps.nouter = outer;
 }
 
@@ -454,12 +474,13 @@ PermPlanP host_plan(std::vector<PermSub> subs, int64_t elem_num, int esz) {
   for (auto& ps : subs) {
     ps.tile_begin = tiles;
     tile_start.push_back(tiles);
-    tiles += ps.nouter * ps.ntx * ps.nty * ps.ntz;
+    tiles += ps.nouter * ps.ntx * ps.nty * ps.ntz * ps.ntw;
   }
   tile_start.push_back(tiles);
   plan->nsub = (int)subs.size();
   plan->ntiles = tiles;
   plan->elem_num = elem_num;
+  for (const auto& ps : subs) plan->short_rows |= ps.wdim >= 0;
   plan->host_subs = std::move(subs);
   return plan;
 }
@@ -532,7 +553,7 @@ void run_permute(Ctx& ctx, const PermPlan& plan, const void* src, void* dst) {
   int64_t grid = std::min<int64_t>(plan.ntiles, (int64_t)ctx.num_sms * 2);
   ProfScope ps(ctx, "permute", 2.0 * plan.esz * plan.elem_num, 0);
   launch_permute_kernel((const PermSub*)plan.subs->ptr, (const int64_t*)plan.tile_start->ptr, plan.nsub, plan.ntiles,
-                        plan.esz, plan.conj, src, dst, (int)grid, ctx.stream);
+                        plan.esz, plan.conj, plan.short_rows, src, dst, (int)grid, ctx.stream);
   ctx.launched();
 }
 

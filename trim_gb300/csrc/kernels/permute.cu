@@ -7,9 +7,9 @@
 // source-contiguous dim and the tile is transposed through shared memory so
 // loads are coalesced too; mode 2 stacks tz planes of a third dim z into a
 // small transpose tile; mode 3 stacks short rows (x contiguous on both sides
-// but only a few elements long) into a dense [z][y][x] tile that is loaded in
-// source-stride order and stored in destination-stride order.  Remaining dims
-// are decoded once per tile.
+// but only a few elements long) into a dense [w][z][y][x] tile that is loaded in
+// source-stride order and stored in destination-stride order, w a fourth dim
+// stepped with a constant stride.  Remaining dims are decoded once per tile.
 //
 // Elements are 8 bytes (real FP64) or 16 bytes (complex FP64 as (re, im)
 // pairs, the cflag twins UniTensorComplex.cpp:447-825): the kernel is the same
@@ -30,11 +30,19 @@ constexpr int kPerThread = 16;  // tile <= 4096 elements: 16 loads in flight per
 constexpr int kSmem = 64 * 65;  // >= ty * (tx + 1) of every transpose tile (checked on the host)
 
 struct TileInfo {
+  static constexpr bool kShortRows = false;
   int64_t bs, bd;     // base offsets of the tile origin
   int64_t sx, sy, sz, dx, dy, dz;
   int32_t nx, ny, nz; // valid extents of this tile
   int32_t tx, ty, tz; // full tile extents
   int32_t mode, neg;
+};
+// with the fourth tile dim of mode 3; plans that have none run a kernel without
+// it (the longer decode records cost the large transposes 1%)
+struct TileInfoW : TileInfo {
+  static constexpr bool kShortRows = true;
+  int64_t sw, dw;
+  int32_t nw, tw;
 };
 
 __host__ __device__ __forceinline__ int find_sub(const int64_t* ts, int nsub, int64_t t) {
@@ -52,17 +60,22 @@ __host__ __device__ __forceinline__ int find_sub(const int64_t* ts, int nsub, in
 // Decode tile number `local` of sub-block P: the tile origin's offsets, its
 // strides along x and y and its valid extents.  Shared by the kernel and the
 // host-side plan check.
-__host__ __device__ inline TileInfo decode_tile(const PermSub& P, int64_t local) {
+template <typename Info>
+__host__ __device__ inline Info decode_tile(const PermSub& P, int64_t local) {
   const int n = P.ndim;
   int64_t bs = P.src_base, bd = P.dst_base;
-  TileInfo w;
+  Info w;
   if (n == 0) {
     w.nx = w.ny = w.nz = w.tx = w.ty = w.tz = 1;
     w.sx = w.sy = w.sz = w.dx = w.dy = w.dz = 0;
+    if constexpr (Info::kShortRows) {
+      w.nw = w.tw = 1;
+      w.sw = w.dw = 0;
+    }
     w.mode = 0;
   } else {
-    const int x = n - 1, y = P.ydim, z = P.zdim;
-    int64_t xt, yt, zt;
+    const int x = n - 1, y = P.ydim, z = P.zdim, v = Info::kShortRows ? P.wdim : -1;
+    int64_t xt, yt, zt, wt = 0;
     if (local < 0x7fffffffLL) {  // 32-bit division is several times cheaper
       uint32_t l = (uint32_t)local;
       xt = l % (uint32_t)P.ntx;
@@ -71,8 +84,12 @@ __host__ __device__ inline TileInfo decode_tile(const PermSub& P, int64_t local)
       l /= (uint32_t)P.nty;
       zt = l % (uint32_t)P.ntz;
       l /= (uint32_t)P.ntz;
+      if (v >= 0) {
+        wt = l % (uint32_t)P.ntw;
+        l /= (uint32_t)P.ntw;
+      }
       for (int i = n - 1; i >= 0 && l; --i) {  // outer dims, innermost first
-        if (i == x || i == y || i == z) continue;
+        if (i == x || i == y || i == z || i == v) continue;
         uint32_t c = l % (uint32_t)P.dims[i];
         l /= (uint32_t)P.dims[i];
         bs += (int64_t)c * P.sstride[i];
@@ -85,8 +102,12 @@ __host__ __device__ inline TileInfo decode_tile(const PermSub& P, int64_t local)
       local /= P.nty;
       zt = local % P.ntz;
       local /= P.ntz;
+      if (v >= 0) {
+        wt = local % P.ntw;
+        local /= P.ntw;
+      }
       for (int i = n - 1; i >= 0; --i) {
-        if (i == x || i == y || i == z) continue;
+        if (i == x || i == y || i == z || i == v) continue;
         int64_t c = local % P.dims[i];
         local /= P.dims[i];
         bs += c * P.sstride[i];
@@ -104,6 +125,20 @@ __host__ __device__ inline TileInfo decode_tile(const PermSub& P, int64_t local)
     } else {
       w.sz = w.dz = 0;
       w.tz = w.nz = 1;
+    }
+    if constexpr (Info::kShortRows) {
+      if (v >= 0) {
+        const int64_t w0 = wt * P.tw;
+        bs += w0 * P.sstride[v];
+        bd += w0 * P.dstride[v];
+        w.sw = P.sstride[v];
+        w.dw = P.dstride[v];
+        w.tw = P.tw;
+        w.nw = (int32_t)((P.dims[v] - w0) < P.tw ? (P.dims[v] - w0) : P.tw);
+      } else {
+        w.sw = w.dw = 0;
+        w.tw = w.nw = 1;
+      }
     }
     int64_t x0 = xt * P.tx;
     bs += x0 * P.sstride[x];
@@ -193,13 +228,14 @@ __device__ __forceinline__ void walk3(const Ax& a, const Ax& b, const Ax& c, F f
 }
 
 // Decode of tile t, or an empty tile (mode -1) past the end of the list.
-__device__ __forceinline__ TileInfo decode_at(const PermSub* __restrict__ subs, const int64_t* __restrict__ tile_start,
-                                              int nsub, int64_t ntiles, int64_t t) {
+template <typename Info>
+__device__ __forceinline__ Info decode_at(const PermSub* __restrict__ subs, const int64_t* __restrict__ tile_start,
+                                          int nsub, int64_t ntiles, int64_t t) {
   if (t < ntiles) {
     const PermSub& P = subs[find_sub(tile_start, nsub, t)];
-    return decode_tile(P, t - P.tile_begin);
+    return decode_tile<Info>(P, t - P.tile_begin);
   }
-  TileInfo w{};
+  Info w{};
   w.mode = -1;
   return w;
 }
@@ -208,8 +244,8 @@ __device__ __forceinline__ TileInfo decode_at(const PermSub* __restrict__ subs, 
 // Mode 0 keeps the tile as [y][x] (pitch tx), mode 1 as [y][x] with pitch
 // tx + 1; loads run with lanes along x (mode 0) or along y, the
 // source-contiguous dim (mode 1).
-template <typename T>
-__device__ __forceinline__ void issue_tile(const TileInfo& w, const T* __restrict__ src, T* buf) {
+template <typename T, typename Info>
+__device__ __forceinline__ void issue_tile(const Info& w, const T* __restrict__ src, T* buf) {
   if (w.mode >= 0) {
     if (w.mode == 2) {
       // [z][y][x] with pitch tx + 1.  A thread takes (y, x) pairs with lanes
@@ -224,11 +260,19 @@ __device__ __forceinline__ void issue_tile(const TileInfo& w, const T* __restric
         for (int zz = 0; zz < w.nz; zz++, g += w.sz, sp += plane) cp_async_el(sp, g);
       }
     } else if (w.mode == 3) {
-      // [z][y][x] dense; elements in source-stride order
+      // [w][z][y][x] dense; elements of a (z, y, x) block in source-stride order,
+      // the w blocks with a constant step: one index computation for all of them
       Ax a{w.tx, w.nx, 1, w.sx}, b{w.ty, w.ny, w.tx, w.sy}, c{w.tz, w.nz, w.tx * w.ty, w.sz};
       sort3(a, b, c);
       const T* s0 = src + w.bs;
-      walk3(a, b, c, [&](int m, int64_t g) { cp_async_el(buf + m, s0 + g); });
+      walk3(a, b, c, [&](int m, int64_t g) {
+        const T* p = s0 + g;
+        T* sp = buf + m;
+        if constexpr (Info::kShortRows)
+          for (int ww = 0; ww < w.nw; ww++, p += w.sw, sp += w.tx * w.ty * w.tz) cp_async_el(sp, p);
+        else
+          cp_async_el(sp, p);
+      });
     } else if (w.mode == 0 && w.tx >= kThreads) {  // long rows: lanes stride along each row
       for (int yy = 0; yy < w.ny; yy++) {
         const T* g = src + w.bs + (int64_t)yy * w.sy + (int64_t)threadIdx.x * w.sx;
@@ -284,8 +328,8 @@ __device__ __forceinline__ void issue_tile(const TileInfo& w, const T* __restric
 }
 
 // Store a landed tile from shared memory with lanes along x (destination-contiguous).
-template <typename T>
-__device__ __forceinline__ void store_tile(const TileInfo& w, const T* buf, T* __restrict__ dst, uint64_t conj) {
+template <typename T, typename Info>
+__device__ __forceinline__ void store_tile(const Info& w, const T* buf, T* __restrict__ dst, uint64_t conj) {
   const uint64_t flip = w.neg ? 0x8000000000000000ull : 0ull;
   const Flip f{flip, flip ^ conj};
   if (w.mode == 2) {  // (x, y) pairs with lanes along x; the z planes with a constant step
@@ -303,7 +347,14 @@ __device__ __forceinline__ void store_tile(const TileInfo& w, const T* buf, T* _
     Ax a{w.tx, w.nx, 1, w.dx}, b{w.ty, w.ny, w.tx, w.dy}, c{w.tz, w.nz, w.tx * w.ty, w.dz};
     sort3(a, b, c);
     T* d0 = dst + w.bd;
-    walk3(a, b, c, [&](int m, int64_t g) { d0[g] = apply_flip(buf[m], f); });
+    walk3(a, b, c, [&](int m, int64_t g) {
+      T* p = d0 + g;
+      const T* sp = buf + m;
+      if constexpr (Info::kShortRows)
+        for (int ww = 0; ww < w.nw; ww++, p += w.dw, sp += w.tx * w.ty * w.tz) *p = apply_flip(*sp, f);
+      else
+        *p = apply_flip(*sp, f);
+    });
     return;
   }
   if constexpr (sizeof(T) == 8) {
@@ -403,15 +454,16 @@ __device__ __forceinline__ void store_tile(const TileInfo& w, const T* buf, T* _
 // the batch is first read 30 iterations later, after the barriers between.
 constexpr int kRing = 64;
 
-__device__ __forceinline__ void decode_batch(TileInfo* ring, const PermSub* __restrict__ subs,
+template <typename Info>
+__device__ __forceinline__ void decode_batch(Info* ring, const PermSub* __restrict__ subs,
                                              const int64_t* __restrict__ tile_start, int nsub, int64_t ntiles,
                                              int64_t k0) {
   const int lane = threadIdx.x & 31;
   const int64_t k = k0 + lane;
-  ring[k % kRing] = decode_at(subs, tile_start, nsub, ntiles, blockIdx.x + k * (int64_t)gridDim.x);
+  ring[k % kRing] = decode_at<Info>(subs, tile_start, nsub, ntiles, blockIdx.x + k * (int64_t)gridDim.x);
 }
 
-template <typename T>
+template <typename T, typename Info>
 __global__ void __launch_bounds__(kThreads, 2) permute_kernel(const PermSub* __restrict__ subs,
                                                               const int64_t* __restrict__ tile_start, int nsub,
                                                               int64_t ntiles, const T* __restrict__ src,
@@ -419,7 +471,7 @@ __global__ void __launch_bounds__(kThreads, 2) permute_kernel(const PermSub* __r
   constexpr int kSmemT = kSmem * (int)sizeof(double) / (int)sizeof(T);  // one stage, in elements
   extern __shared__ double smem_d[];  // kStages * kSmem doubles
   T* smem = (T*)smem_d;
-  __shared__ TileInfo ring[kRing];
+  __shared__ Info ring[kRing];
   pdl_trigger();
   const int64_t G = gridDim.x;
   if (threadIdx.x < 32) decode_batch(ring, subs, tile_start, nsub, ntiles, 0);  // plan data
@@ -427,7 +479,7 @@ __global__ void __launch_bounds__(kThreads, 2) permute_kernel(const PermSub* __r
   __syncthreads();
 #pragma unroll
   for (int s = 0; s < kStages - 1; s++) {
-    const TileInfo w = ring[s];
+    const Info w = ring[s];
     issue_tile(w, src, smem + s * kSmemT);
   }
   int stage = 0;
@@ -435,14 +487,14 @@ __global__ void __launch_bounds__(kThreads, 2) permute_kernel(const PermSub* __r
   for (int64_t t = blockIdx.x; t < ntiles; t += G, i++) {
     const int ns = (stage + kStages - 1) % kStages;  // stored in the previous iteration
     {
-      const TileInfo w = ring[(i + kStages - 1) % kRing];
+      const Info w = ring[(i + kStages - 1) % kRing];
       issue_tile(w, src, smem + ns * kSmemT);
     }
     if (threadIdx.x < 32 && (i & 31) == 0) decode_batch(ring, subs, tile_start, nsub, ntiles, i + 32);
     cp_async_wait<kStages - 1>();  // this thread's loads of tile t have landed
     __syncthreads();               // ... and every other thread's
     {
-      const TileInfo w = ring[i % kRing];
+      const Info w = ring[i % kRing];
       store_tile(w, smem + stage * kSmemT, dst, conj);
     }
     __syncthreads();  // the stage is reloaded in the next iteration
@@ -506,21 +558,23 @@ int64_t check_permute_plan_host(const PermPlan& plan, const double* src, double*
   int64_t written = 0;
   for (int64_t t = 0; t < plan.ntiles; t++) {
     const PermSub& P = plan.host_subs[find_sub(plan.host_tile_start.data(), plan.nsub, t)];
-    TileInfo w = decode_tile(P, t - P.tile_begin);
-    if (w.nx > w.tx || w.ny > w.ty || w.nz > w.tz || w.nx <= 0 || w.ny <= 0 || w.nz <= 0)
+    const TileInfoW w = decode_tile<TileInfoW>(P, t - P.tile_begin);
+    if (w.nx > w.tx || w.ny > w.ty || w.nz > w.tz || w.nw > w.tw || w.nx <= 0 || w.ny <= 0 || w.nz <= 0 || w.nw <= 0)
       fail(TN_ERR_ARG, "plan check: bad tile extents");
+    if (w.mode != 3 && w.tw != 1) fail(TN_ERR_ARG, "plan check: a fourth tile dim outside mode 3");
     if (w.mode < 2 && w.tz != 1) fail(TN_ERR_ARG, "plan check: stacked planes outside modes 2 and 3");
-    const int64_t stage = (w.mode == 1 || w.mode == 2) ? (int64_t)w.tz * w.ty * (w.tx + 1) : (int64_t)w.tz * w.tx * w.ty;
+    const int64_t stage = (w.mode == 1 || w.mode == 2) ? (int64_t)w.tz * w.ty * (w.tx + 1) : (int64_t)w.tw * w.tz * w.tx * w.ty;
     if (stage > kSmem / es) fail(TN_ERR_ARG, "plan check: tile exceeds shared memory");
-    if ((int64_t)w.tx * w.ty * w.tz > (int64_t)kThreads * kPerThread)
+    if ((int64_t)w.tx * w.ty * w.tz * w.tw > (int64_t)kThreads * kPerThread)
       fail(TN_ERR_ARG, "plan check: tile exceeds thread walk");
     if (w.mode >= 2 && ((int64_t)w.tx * w.ty * w.tz >= (1 << 16) || w.tx > 4096 || w.ty > 4096))
       fail(TN_ERR_ARG, "plan check: tile index exceeds the multiply-high division range");
-    for (int zz = 0; zz < w.nz; zz++)
+    for (int wz = 0; wz < w.nw * w.nz; wz++)
       for (int yy = 0; yy < w.ny; yy++)
         for (int xx = 0; xx < w.nx; xx++) {
-          int64_t so = w.bs + (int64_t)yy * w.sy + (int64_t)xx * w.sx + (int64_t)zz * w.sz;
-          int64_t d = w.bd + (int64_t)yy * w.dy + (int64_t)xx * w.dx + (int64_t)zz * w.dz;
+          const int ww = wz / w.nz, zz = wz % w.nz;
+          int64_t so = w.bs + (int64_t)yy * w.sy + (int64_t)xx * w.sx + (int64_t)zz * w.sz + (int64_t)ww * w.sw;
+          int64_t d = w.bd + (int64_t)yy * w.dy + (int64_t)xx * w.dx + (int64_t)zz * w.dz + (int64_t)ww * w.dw;
           if (so < 0 || so >= n || d < 0 || d >= n) fail(TN_ERR_ARG, "plan check: offset out of range");
           if (hit[d]++) fail(TN_ERR_ARG, "plan check: destination written twice");
           for (int c = 0; c < es; c++) {
@@ -534,26 +588,28 @@ int64_t check_permute_plan_host(const PermPlan& plan, const double* src, double*
   return written;
 }
 
-template <typename T>
+template <typename T, typename Info>
 static void launch_permute_t(const PermSub* subs, const int64_t* tile_start, int nsub, int64_t ntiles, const T* src,
                              T* dst, uint64_t conj, int grid, cudaStream_t s) {
   const size_t smem = (size_t)kStages * kSmem * sizeof(double);
   static bool attr = false;  // once per process and instantiation; the attribute is per function
   if (!attr) {
-    TN_CUDA(cudaFuncSetAttribute(permute_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    TN_CUDA(cudaFuncSetAttribute(permute_kernel<T, Info>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     attr = true;
   }
-  launch_pdl(permute_kernel<T>, dim3(grid), dim3(kThreads), smem, s, subs, tile_start, nsub, ntiles, src, dst, conj);
+  launch_pdl(permute_kernel<T, Info>, dim3(grid), dim3(kThreads), smem, s, subs, tile_start, nsub, ntiles, src, dst, conj);
 }
 
 void launch_permute_kernel(const PermSub* subs, const int64_t* tile_start, int nsub, int64_t ntiles, int esz,
-                           bool conj, const void* src, void* dst, int grid, cudaStream_t s) {
-  if (esz == 8)
-    launch_permute_t<double>(subs, tile_start, nsub, ntiles, (const double*)src, (double*)dst, 0, grid, s);
-  else if (esz == 16)
-    launch_permute_t<double2>(subs, tile_start, nsub, ntiles, (const double2*)src, (double2*)dst,
-                              conj ? 0x8000000000000000ull : 0ull, grid, s);
-  else
+                           bool conj, bool short_rows, const void* src, void* dst, int grid, cudaStream_t s) {
+  const uint64_t c = conj ? 0x8000000000000000ull : 0ull;
+  if (esz == 8) {
+    auto f = short_rows ? launch_permute_t<double, TileInfoW> : launch_permute_t<double, TileInfo>;
+    f(subs, tile_start, nsub, ntiles, (const double*)src, (double*)dst, 0, grid, s);
+  } else if (esz == 16) {
+    auto f = short_rows ? launch_permute_t<double2, TileInfoW> : launch_permute_t<double2, TileInfo>;
+    f(subs, tile_start, nsub, ntiles, (const double2*)src, (double2*)dst, c, grid, s);
+  } else
     fail(TN_ERR_ARG, "permute: element size must be 8 or 16 bytes");
 }
 
