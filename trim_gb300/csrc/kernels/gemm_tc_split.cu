@@ -2,20 +2,28 @@
 // digit images written by tc_slices<6> (gemm_tc.cu) multiplied on the tcgen05
 // tensor cores and recombined exactly.
 //
-// Digits: every FP64 element is rounded to 52 bits below its row's (A) or
+// Digits: every FP64 element is rounded to 53 bits below its row's (A) or
 // column's (B) power-of-two scale 2^e > max and cut into 6 balanced base-512
-// digits, x = 2^(e-7) sum_s d_s 2^(-9s), |d_0| <= 128, d_1..d_5 in
+// digits, x = 2^(e-8) sum_s d_s 2^(-9s), |d_0| <= 256, d_1..d_5 in
 // [-256, 255]: integers that BF16 holds exactly (8 significant bits reach
-// 256).  C = 2^(ea+eb-14) sum_{s+t<=5} 2^(-9(s+t)) A_s B_t: 21 digit products.
-// What is left out (s + t >= 6: five products below 2^-52 of the two maxima
-// per k) and the operands' rounding (2^-53) stay an order of magnitude below
-// the 34 products of 7-bit digits this replaced, whose operands were rounded
-// at 2^-50.  Wider digits than 7 bits are what FP32 accumulation limits: per k
-// the digit products of levels 0..5 (l = s + t) sum to at most 2^14, 2^16,
-// 2^17, 3 2^16, 4 2^16, 5 2^16, so over one 64-k tile levels 0..4 are exact
-// integers below 2^24 and level 5 rounds at 2^-59; the accumulators are
-// therefore drained every 64-k tile, which the digit width pays for only if
-// the drain runs beside the MMAs.
+// 256).  C = 2^(ea+eb-16) sum_{s+t<=5} 2^(-9(s+t)) A_s B_t: 21 digit products.
+// What is left out (s + t >= 6) is five products of, on average, 2^-55.6 of the
+// two maxima per k; the 34 products of 7-bit digits this replaced rounded the
+// operands at 2^-50, 2^-50.8 of a maximum times the other operand.  So the error
+// is below theirs while the root mean squares of a row and a column are above
+// 1/18 of their scales (it is 1/9 .. 1/4 for Gaussian entries, 0.3 .. 0.6 for
+// uniform ones).  With |d_0| <= 128, a bit less of each operand, it was four times
+// as large, and above theirs on Gaussian entries.
+// Measured (Frobenius norm, relative, against 113-bit sums; 34 products / |d_0|
+// <= 128 / now): uniform entries, K = 160000 6.7e-15 / 6.1e-16 / 2.9e-16;
+// Gaussian, K = 2000 3.8e-15 / 3.6e-15 / 8.7e-16, K = 160000 8.5e-15 / 1.1e-14 /
+// 3.0e-15.
+// Wider digits than 7 bits are what FP32 accumulation limits: per k the digit
+// products of levels 0..5 (l = s + t) sum to at most (l + 1) 2^16, so over one
+// 64-k tile levels 0..3 are exact integers up to 2^24; level 4 reaches there only
+// where every digit is at its largest, and rounds by one of 2^-52, level 5 at
+// 2^-60.  The accumulators are therefore drained every 64-k tile, which the
+// digit width pays for only if the drain runs beside the MMAs.
 //
 // Tensor memory is a ring of four 128-column slots, each holding two levels
 // (0/1, 2/3, 4/5) of one 64-k tile at 64 columns: a tile takes three slots,
@@ -35,10 +43,11 @@
 // read from one lane (__shfl_sync), which makes the branches warp-uniform for
 // the compiler.
 //
-// Drain: each level converts to int32 exactly (cvt runs at full rate), and a
-// 64-bit integer per output sums the levels in units of 2^-36 of level 0 (15
-// issue slots per output and tile).  |sum| < K 2^50.03, so it is moved to the
-// FP64 output every 4096 k.
+// Drain: each level converts to int32 exactly (cvt runs at full rate); per
+// output a 32-bit integer sums level 0 and a 64-bit one the others, in units of
+// level 4 (2^-36 of level 0; 15 issue slots per output and tile).  Together, in
+// units of 2^-34 of level 0, |sum| < K 2^50.03, so they are moved to the FP64
+// output every 4096 k.
 //
 // CTA (576 threads, one per SM, 128 x 64 output tile): warp 0 bulk copies
 // (8-slot ring of 16 KB A digit tiles, 2-slot ring of 48 KB B tiles), warp 1
@@ -74,7 +83,7 @@ constexpr int kSlots = 4, kSlotCols = 2 * kTN;  // TMEM ring: two levels per slo
 constexpr int kEpiWarps = 16, kEpiCols = kTN * 4 / kEpiWarps;
 constexpr int kThreadsSplit = 64 + 32 * kEpiWarps;
 constexpr int kSegTiles = 64;  // 4096 k per 64-bit integer sum
-constexpr int kUnit = 50;      // the sum's unit is 2^(ea + eb - 50): level 4
+constexpr int kUnit = 50;      // the sum's unit is 2^(ea + eb - 50)
 
 struct __align__(8) SplitShared {
   uint64_t fullA[kARing], emptyA[kARing], fullB[kBRing], emptyB[kBRing];
@@ -371,9 +380,10 @@ __global__ void __launch_bounds__(kThreadsSplit, 1) tc_gemm_split(const TcSector
       const unsigned long long col_max = (lane & 15) < nc ? __ldg(eb + S.eb_off + j0 + (lane & 15)) : 0;
       for (int k0 = kb; k0 < ke && ok; k0 += kSegTiles) {
         const int k1 = min(ke, k0 + kSegTiles);
+        int top[kEpiCols];  // level 0, and the others in units of level 4
         long long acc[kEpiCols];
 #pragma unroll
-        for (int q = 0; q < kEpiCols; q++) acc[q] = 0;
+        for (int q = 0; q < kEpiCols; q++) top[q] = 0, acc[q] = 0;
         for (int kt = k0; kt < k1 && ok; kt++) {
 #pragma unroll
           for (int j = 0; j < 3; j++) {
@@ -391,8 +401,8 @@ __global__ void __launch_bounds__(kThreadsSplit, 1) tc_gemm_split(const TcSector
             g++;
 #pragma unroll
             for (int q = 0; q < kEpiCols; q++) {
-              if (j == 0)  // |512 L0 + L1| < 2^30
-                acc[q] += (long long)(__float2int_rn(a[q]) * 512 + __float2int_rn(b[q])) * (1 << 27);
+              if (j == 0)
+                top[q] += __float2int_rn(a[q]), acc[q] += (long long)__float2int_rn(b[q]) * (1 << 27);
               else if (j == 1)
                 acc[q] += (long long)__float2int_rn(a[q]) * (1 << 18) + (long long)__float2int_rn(b[q]) * (1 << 9);
               else
@@ -429,7 +439,8 @@ __global__ void __launch_bounds__(kThreadsSplit, 1) tc_gemm_split(const TcSector
             double v[4];
 #pragma unroll
             for (int c = 0; c < 4; c++) {
-              const long long x = acc[8 * (t >> 1) + 2 * (t & 1) + 4 * (c >> 1) + (c & 1)];
+              const int n = 8 * (t >> 1) + 2 * (t & 1) + 4 * (c >> 1) + (c & 1);
+              const long long x = ((long long)top[n] << 34) + ((acc[n] + 2) >> 2);
               // several sums to add: without the scales, which the last addition is
               // followed by (so a result in the subnormal range is rounded once)
               const int q = several ? -kUnit : e_i + ej[c];

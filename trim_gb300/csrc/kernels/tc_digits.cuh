@@ -53,8 +53,8 @@ __device__ __forceinline__ uint32_t scaled_f32_bits(double x, int e) {
 // FP32 from the bit pattern of 1.5 * 2^(23-7s) + d * 2^-7s (integer add into
 // the mantissa, one exact subtraction); it has at most 8 significant bits, so
 // its BF16 pattern is the top half of the FP32 pattern.
-// NS = 6: X = |x| * 2^(52 - e) rounded to the nearest integer (X <= 2^52), V =
-// +-X and its balanced base-512 digits (d_1..d_5 in [-256, 255], |d_0| <= 128)
+// NS = 6: X = |x| * 2^(53 - e) rounded to the nearest integer (X <= 2^53), V =
+// +-X and its balanced base-512 digits (d_1..d_5 in [-256, 255], |d_0| <= 256)
 // read out of Y = V + 256 * (1 + 512 + ... + 512^4) the same way.  They are
 // stored as plain integers (BF16 holds every integer up to 256), so one magic
 // number, 1.5 * 2^23, serves all of them.
@@ -80,7 +80,7 @@ __device__ __forceinline__ void make_slices(const double (&x)[8], int e, uint4 (
           mant |= 1ull << 52;
           E = ef - 1023;
         }
-        const int sh = (NS == 7 ? 3 : 0) + e - E;  // X = mant * 2^(E - 52) * 2^(49 - e), or 2^(52 - e) for 6 digits
+        const int sh = (NS == 7 ? 3 : -1) + e - E;  // X = mant * 2^(E - 52) * 2^(49 - e), or 2^(53 - e) for 6 digits
         const uint64_t X = (sh >= 64) ? 0ull : (sh > 0 ? ((mant + (1ull << (sh - 1))) >> sh) : (mant << (-sh)));
         const long long V = (bits >> 63) ? -(long long)X : (long long)X;
         if constexpr (NS == 6) {
