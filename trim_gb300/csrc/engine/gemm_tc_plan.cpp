@@ -136,14 +136,18 @@ static std::shared_ptr<TcPlan> build_tc_plan(Ctx& ctx, const std::vector<tn_sect
   P->nitems = (int)items.size();
   P->nred = (int)ritems.size();
   if (!P->nsec) return P;
-  // One pass over the operands, an item over all of K, unless that leaves most of
-  // the chip idle on long rows: fewer items than CTAs in flight and K beyond what
-  // an item of A keeps.  There the maxima and the images are made tile by tile
-  // in two launches (as for a list whose items would not number in 32 bits).
+  // One pass over the operands, an item over all of K, or maxima and images
+  // tile by tile in two launches (also for a list whose items would not number
+  // in 32 bits).  The two launches read everything twice, 1.4 times the time of
+  // one pass over a full chip, and take at least 20 us; one pass lasts at least
+  // as long as its longest item, whose CTA slices about 1000 elements a
+  // microsecond.  A 484 x 484 product over K = 234256 has 31 strips of B with
+  // 3.7 M elements each: 1.0 ms in two launches, 3.6 ms in one.
   int64_t nsl = 0;
   for (const auto& s : secs) nsl += cdiv(s.N, 16) + (s.K > kRowWarp ? s.M : cdiv(s.M, 8));
+  const double two_passes = 20 + 1.4 * P->in_bytes / 8 / 330e3, longest_item = 16.0 * P->max_k / 1000;
   std::vector<int2> sitems;
-  if (nsl < INT32_MAX / 2 && (nsl >= 3 * (int64_t)ctx.num_sms || P->max_k <= 8192)) {
+  if (nsl < INT32_MAX / 2 && longest_item <= two_passes) {
     sitems.reserve(nsl);
     for (int g = 0; g < P->nsec; g++)
       for (int64_t c = 0; c < cdiv(secs[g].N, 16); c++) sitems.push_back(make_int2(g, (int)c));
