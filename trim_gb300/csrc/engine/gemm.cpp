@@ -499,7 +499,22 @@ constexpr int kModeFlags = TN_MODE_TC_ONLY | TN_MODE_TC_FUSED | TN_MODE_TC_TILED
 
 // A sector too thin for a 128 x 64 x 16 MMA step to pay: in the tiled form
 // it stays on the exact FP64 kernel (unless TN_MODE_TC_ONLY).
-static bool thin_sector(const tn_sector_gemm& g) { return g.K < 16 || g.N < 16; }
+//
+// In split precision so does one that the FP64 kernel finishes sooner, both in
+// clocks of one SM as grouped launches of small sectors run: 1.6 FMAs a clock
+// there, against 4400 per 64 k of an output tile (3400 more to write it) and 1.9
+// per operand element to slice.  30 x 30 outputs take the tensor cores, 8 x 30
+// do not: on 1024 contractions of bonds 16..256 that moves 1403 of 3007 sectors,
+// 7% of the flop, and the call from 5.4 to 4.8 ms.  The fast modes keep the
+// sizes alone (there a sector's precision hangs on it), and so does a call that
+// asks for the tiled form.
+static bool thin_sector(int mode, const tn_sector_gemm& g) {
+  if (g.K < 16 || g.N < 16) return true;
+  if ((mode & ~kModeFlags) != TN_MODE_SPLIT || (mode & TN_MODE_TC_TILED)) return false;
+  const double m = (double)g.M, n = (double)g.N, k = (double)g.K;
+  const double tiles = std::ceil(m / 128) * std::ceil(n / 64);
+  return m * n * k / 1.6 < tiles * (std::ceil(k / 64) * 4400 + 3400) + 1.9 * (m + n) * k;
+}
 
 // The fused form fits a contraction of a few 128 x 64 output tiles per SM
 // whose sectors all have short K (its CTAs walk K serially).
@@ -527,7 +542,7 @@ static GemmRoute static_route(const Ctx& ctx, int mode, const std::vector<tn_sec
   if (want_tiled) return GemmRoute::Tiled;
   if (want_fused) return GemmRoute::Fused;
   bool all_thin = !tc_only;
-  for (const auto& g : list) all_thin = all_thin && thin_sector(g);
+  for (const auto& g : list) all_thin = all_thin && thin_sector(mode, g);
   if (all_thin) return GemmRoute::Fp64;
   if (mode == TN_MODE_FAST_TF32) return GemmRoute::Tiled;  // TF32 runs in the tiled form only
   // one fused launch for every sector, thin ones included (they cost a CTA
@@ -704,7 +719,7 @@ void run_sector_gemms(Ctx& ctx, int mode, const std::vector<tn_sector_gemm>& lis
   const bool tuned = ctx.route_tuned.count(route_key(mode, list)) > 0;
   auto tiled = [&] {
     std::vector<tn_sector_gemm> tc, f64;
-    for (const auto& g : list) (!tc_only && thin_sector(g) ? f64 : tc).push_back(g);
+    for (const auto& g : list) (!tc_only && thin_sector(mode, g) ? f64 : tc).push_back(g);
     if (!f64.empty()) run_fp64(ctx, f64, A, B, C);
     if (!tc.empty()) run_tc_gemms(ctx, ns == 7 ? kSplitDigits : ns, tc, A, B, C);
   };
