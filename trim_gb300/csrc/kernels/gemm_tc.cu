@@ -2,7 +2,7 @@
 // maxima and digit images in every mode, and the sum over K ranges.  The GEMMs
 // are gemm_tc_split.cu (split precision) and gemm_tc_fast.cu (BF16, TF32).
 //
-// Split precision (TN_MODE_SPLIT): six BF16 digit images per operand tile
+// Split precision (TN_MODE_SPLIT): six FP16 digit images per operand tile
 // (tc_digits.cuh).
 // Fast BF16 (TN_MODE_FAST_BF16): one image, the BF16 rounding of each scaled
 // element.
@@ -131,7 +131,10 @@ __device__ __forceinline__ void store_chunk(uint8_t* img, int img_bytes, int r, 
     *(uint4*)(at + swz_off(r, 2 * (c & 3) + 1)) = o[1];
   } else {
     uint4 o[NS];
-    make_slices<NS>(x, e, o);
+    if constexpr (NS == 6)
+      make_digits(x, e, o);
+    else
+      make_slices<NS>(x, e, o);
     const uint32_t off = swz_off(r, c);
 #pragma unroll
     for (int s = 0; s < NS; s++) *(uint4*)(img + (int64_t)s * img_bytes + off) = o[s];
@@ -220,14 +223,18 @@ __device__ __forceinline__ void slice_b_tile(const TcSector* __restrict__ secs, 
 // each; one row beyond kRowWarp k) or a strip of 16 columns of B, over all of
 // K.  What an item holds in shared memory (74 KB, three CTAs per SM: rows of
 // up to kRowKeep k per warp or 8192 per CTA, strips of up to kWideK) is read from
-// memory once; longer ones are read again, through L2.  Staging is by 8-byte
-// cp.async, consecutive lanes on consecutive addresses whatever a row's
-// alignment; a thread then slices 8 consecutive k.  HBM bound: 8 bytes read and
-// 2 bytes per digit written per element.  Only what the GEMM uses is written:
+// memory once; longer ones are read again, through L2.  Staging is by
+// cp.async, 16 bytes a copy where the row (the strip's rows) starts on 16 bytes,
+// else 8; a thread then slices 8 consecutive k.  8 bytes are read and 2 bytes
+// per digit written per element, 4.9 TB/s on 80000 rows or columns of 400 in
+// split precision (4.2 with 8-byte copies and reads and the digits of
+// make_slices): the instructions per element decide (107 there), not the
+// loads' latency - bringing the next item into L2 ahead made it slower.  Only what the GEMM uses is written:
 // no row past M or column past N (accumulator rows and columns nobody reads),
 // no k past the last 16-k step.
 constexpr int kStageDoubles = 9216, kRowKeep = 1024, kWideK = 576;
-__host__ __device__ constexpr int padded(int k) { return k + (k >> 3); }  // 9 doubles per 8: no bank conflicts
+// 18 doubles per 16: 16-byte reads of 8 consecutive k per lane without bank conflicts
+__host__ __device__ constexpr int padded(int k) { return k + (k >> 4 << 1); }
 static_assert(8 * padded(kRowKeep) <= kStageDoubles && padded(8192) <= kStageDoubles && 16 * kWideK <= kStageDoubles,
               "the staged extents fit");
 
@@ -261,10 +268,26 @@ __device__ __forceinline__ void slice_row(const TcSector& S, int64_t i, int id, 
   const int r = (int)(i % kTM);
   const bool keep = kend <= keep_k;
   // k0 .. k0 + len - 1 (zero past K) on their way into the buffer at `at`
+  const bool wide = ((uintptr_t)src & 15) == 0;  // two doubles a copy
   auto stage = [&](int k0, int len, int at) {
-    for (int k = id; k < min(len, kend - k0); k += n)
-      cp_async8(buf + padded(at + k), k0 + k < S.K ? src + k0 + k : src, k0 + k < S.K);
+    const int end = min(len, kend - k0), left = S.K - k0;
+    if (wide) {
+#pragma unroll 4
+      for (int k = 2 * id; k < end; k += 2 * n)
+        cp_async16(buf + padded(at + k), k < left ? src + k0 + k : src, k < left ? min(16, 8 * (left - k)) : 0);
+    } else {
+      for (int k = id; k < end; k += n)
+        cp_async8(buf + padded(at + k), k < left ? src + k0 + k : src, k < left);
+    }
     cp_async_commit();
+  };
+  auto read8 = [&](int k, double(&x)[8]) {  // k a multiple of 8
+    const double2* p = (const double2*)(buf + padded(k));
+#pragma unroll
+    for (int q = 0; q < 4; q++) {
+      const double2 v = p[q];
+      x[2 * q] = v.x, x[2 * q + 1] = v.y;
+    }
   };
   uint32_t hi = 0;
   if (keep) {
@@ -272,7 +295,12 @@ __device__ __forceinline__ void slice_row(const TcSector& S, int64_t i, int id, 
     stage(0, keep_k, 0);
     cp_async_wait<0>();
     sync();
-    for (int k = id; k < kend; k += n) hi = max(hi, abs_hi(buf[padded(k)]));
+    for (int k = id * 8; k < kend; k += 8 * n) {
+      double x[8];
+      read8(k, x);
+#pragma unroll
+      for (int q = 0; q < 8; q++) hi = max(hi, abs_hi(x[q]));
+    }
   } else {
     sync();
     stage(0, half, 0);  // the first half buffer loads while the maximum is taken
@@ -305,8 +333,7 @@ __device__ __forceinline__ void slice_row(const TcSector& S, int64_t i, int id, 
   auto slice = [&](int k0, int len, int at) {
     for (int k = id * 8; k < min(len, kend - k0); k += 8 * n) {
       double x[8];
-#pragma unroll
-      for (int q = 0; q < 8; q++) x[q] = buf[padded(at + k) + q];
+      read8(at + k, x);
       store_chunk<NS>(img + (int64_t)((k0 + k) / kTK) * NS * kATile, kATile, r, (k / 8) % 8, x, e);
     }
   };
@@ -329,8 +356,8 @@ __device__ __forceinline__ int image_row(int n) {
   return (n & ~15) | ((n & 2) << 2) | ((n & 12) >> 1) | (n & 1);
 }
 
-// 16 columns of B by a CTA: thread (c, g) has column c and the groups g, g +
-// 16, .. of 8 k; it stages the values it slices itself
+// 16 columns of B by a CTA: thread (c, g) slices of column c the groups g, g +
+// 16, .. of 8 k
 template <int NS>
 __device__ __forceinline__ void slice_strip(const TcSector& S, int64_t strip, const double* __restrict__ B,
                                             unsigned long long* __restrict__ eb, uint8_t* __restrict__ ws, double* buf,
@@ -349,12 +376,19 @@ __device__ __forceinline__ void slice_strip(const TcSector& S, int64_t strip, co
   };
   uint32_t hi = 0;
   if (keep) {
-#pragma unroll
-    for (int q = 0; q < 8; q++)
-      for (int k = g * 8 + q; k < kend; k += kPass)
+    const double* s0 = B + S.b_off + strip * W;
+    if (strip * W + W <= S.N && ((uintptr_t)s0 & 15) == 0 && (S.N & 1) == 0) {  // two columns a copy
+      const int p = 2 * (threadIdx.x & 7);
+#pragma unroll 4
+      for (int k = threadIdx.x >> 3; k < kend; k += 32)
+        cp_async16(buf + k * W + p, k < S.K ? s0 + (int64_t)k * S.N + p : s0, k < S.K ? 16 : 0);
+    } else {
+      for (int k = g; k < kend; k += 16)
         cp_async8(buf + at(k), k < cols ? src + (int64_t)k * S.N : B, k < cols);
+    }
     cp_async_commit();
     cp_async_wait<0>();
+    __syncthreads();
     for (int k = g * 8; k < kend; k += kPass)
 #pragma unroll
       for (int q = 0; q < 8; q++) hi = max(hi, abs_hi(buf[at(k + q)]));

@@ -202,7 +202,7 @@ __global__ void __launch_bounds__(kThreadsFast, 1) tc_gemm_fast(const TcSector* 
           if constexpr (NS == 2)
             mma_tf32_elect(d, ad + 2 * kk, bd + 2 * kk, idesc, kk ? 1u : acc0);
           else
-            mma_bf16_elect(d, ad + 2 * kk, bd + 2 * kk, idesc, kk ? 1u : acc0);
+            mma_f16_elect(d, ad + 2 * kk, bd + 2 * kk, idesc, kk ? 1u : acc0);
         }
       mma_commit_elect(&sh.empty[st]);
       if (info & 128) {

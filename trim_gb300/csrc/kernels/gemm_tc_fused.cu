@@ -418,7 +418,7 @@ __global__ void __launch_bounds__(kFThreads, 1) tc_fused(const TcSector* __restr
         if constexpr (NS == 1) {
           for (int kk = 0; kk < nks; kk++)
             // +32 bytes per 16-k step inside the swizzle atom: +2 in the address field
-            mma_bf16_elect(tmem, a0 + 2 * kk, b0 + 2 * kk, idesc1, (carry | (uint32_t)kk) ? 1u : 0u);
+            mma_f16_elect(tmem, a0 + 2 * kk, b0 + 2 * kk, idesc1, (carry | (uint32_t)kk) ? 1u : 0u);
         } else {
           // A digit s with B digits t0 .. t0 + tn - 1 in one MMA (N = 64 tn, at
           // most 4; 7 -> 4 + 3, 6 -> 3 + 3, 5 -> 3 + 2), the group cut where a
@@ -440,7 +440,7 @@ __global__ void __launch_bounds__(kFThreads, 1) tc_fused(const TcSector* __restr
               const uint32_t idesc = idesc1 + ((uint32_t)(tn - 1) * (kFN >> 3) << 17);
               const uint64_t ad = a0 + (uint64_t)(s * (kAImg >> 4)), bd = b0 + (uint64_t)(t0 * (kBImg >> 4));
               for (int kk = 0; kk < nks; kk++)
-                mma_bf16_elect(tmem + l0 * kFN, ad + 2 * kk, bd + 2 * kk, idesc, kk ? 1u : acc);
+                mma_f16_elect(tmem + l0 * kFN, ad + 2 * kk, bd + 2 * kk, idesc, kk ? 1u : acc);
               touched |= ((1u << tn) - 1u) << l0;
               t0 += tn;
             }

@@ -5,8 +5,8 @@
 // Digits: every FP64 element is rounded to 53 bits below its row's (A) or
 // column's (B) power-of-two scale 2^e > max and cut into 6 balanced base-512
 // digits, x = 2^(e-8) sum_s d_s 2^(-9s), |d_0| <= 256, d_1..d_5 in
-// [-256, 255]: integers that BF16 holds exactly (8 significant bits reach
-// 256).  C = 2^(ea+eb-16) sum_{s+t<=5} 2^(-9(s+t)) A_s B_t: 21 digit products.
+// [-256, 255]: integers that FP16 holds exactly.  C = 2^(ea+eb-16)
+// sum_{s+t<=5} 2^(-9(s+t)) A_s B_t: 21 digit products.
 // What is left out (s + t >= 6) is five products of, on average, 2^-55.6 of the
 // two maxima per k; the 34 products of 7-bit digits this replaced rounded the
 // operands at 2^-50, 2^-50.8 of a maximum times the other operand.  So the error
@@ -58,7 +58,7 @@
 // (K = 576, 6.7e11 FP64-equivalent flop) 16.0 -> 9.5 ms, the iPEPS quadrant at
 // chi = 128, D = 8 (K = 4096, 1.4e11) 3.41 -> 1.76 ms, against the 34-product
 // kernel.  21 products per FP64 multiply-add: 80 TFLOP/s FP64-equivalent at
-// K = 4096 is 1 690 of BF16, and the tensor pipe alone (no loads, no drain, no
+// K = 4096 is 1 690 of FP16, and the tensor pipe alone (no loads, no drain, no
 // output) takes 1.51 ms; at K = 576 the FP64 output of every ninth tile (64 KB at
 // the 30 B per clock that an SM stores, whatever the pattern, as long as a row's
 // 128 bytes go together: 17 B per clock with a row per lane) stalls the drain
@@ -137,7 +137,7 @@ template <int M, int S, int L, bool FULL>
 __device__ __forceinline__ bool split_groups(MmaState& st, uint64_t adesc) {
   if constexpr (L < kDigits) {
     constexpr int R = 3 * M % kSlots, n = level_group(R, S, L);
-    constexpr uint32_t idesc = idesc_bf16_f32(kTM, kTN) + ((uint32_t)(n - 1) * (kTN >> 3) << 17);
+    constexpr uint32_t idesc = idesc_fp16_f32(kTM, kTN) + ((uint32_t)(n - 1) * (kTN >> 3) << 17);
     constexpr uint32_t col = level_col(R, L);
     const uint64_t bdesc = desc_sw128(st.bbuf + (M % kBRing) * kDigits * kBTile + (L - S) * kBTile);
     uint64_t* t1 = &st.sh->emptyT[(R + 1) % kSlots];  // the tile's other two slots
@@ -150,9 +150,9 @@ __device__ __forceinline__ bool split_groups(MmaState& st, uint64_t adesc) {
         r1 = mbar_test(t1, p1);
         r2 = mbar_test(t2, p2);
       }
-      // advancing K by 16 bf16 = 32 bytes inside the swizzle atom: +2 in the address field
+      // advancing K by 16 halves = 32 bytes inside the swizzle atom: +2 in the address field
       if (FULL || kk < st.nks)
-        mma_bf16_elect(st.tmem + col, adesc + 2 * kk, bdesc + 2 * kk, idesc, (S > 0 || kk > 0) ? 1u : 0u);
+        mma_f16_elect(st.tmem + col, adesc + 2 * kk, bdesc + 2 * kk, idesc, (S > 0 || kk > 0) ? 1u : 0u);
     }
     if constexpr (S == 0 && L == 0) {
       if (!__all_sync(0xffffffffu, r1 && r2) && !(warp_wait(t1, p1, st.sh) && warp_wait(t2, p2, st.sh))) return false;

@@ -82,6 +82,10 @@ __device__ __forceinline__ void cp_async8(void* smem_dst, const void* src, bool 
                "r"(valid ? 8 : 0)
                : "memory");
 }
+// 16 bytes, of which the first `bytes` (0, 8 or 16) are read and the rest are zero
+__device__ __forceinline__ void cp_async16(void* smem_dst, const void* src, int bytes) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(smem_u32(smem_dst)), "l"(src), "r"(bytes) : "memory");
+}
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
 template <int N>  // all but the last N groups have landed
 __device__ __forceinline__ void cp_async_wait() {
@@ -135,7 +139,7 @@ __device__ __forceinline__ void mma_bf16(uint32_t d_tmem, uint64_t a_desc, uint6
 // warp running the issue loop, the loop's values stay warp-uniform and the
 // per-MMA issue cost drops (one MMA per ~48 clocks at M=128, N=64 against ~58
 // from a single-lane loop).
-__device__ __forceinline__ void mma_bf16_elect(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc,
+__device__ __forceinline__ void mma_f16_elect(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc,
                                                uint32_t accumulate) {
   asm volatile(
       "{\n .reg .pred p, e;\n elect.sync _|e, 0xffffffff;\n setp.ne.b32 p, %4, 0;\n"
@@ -161,7 +165,7 @@ __device__ __forceinline__ void mma_commit(uint64_t* bar) {
                : "memory");
 }
 
-// mma_commit by the lane elect.sync picks (the one that issued mma_bf16_elect)
+// mma_commit by the lane elect.sync picks (the one that issued mma_f16_elect)
 __device__ __forceinline__ void mma_commit_elect(uint64_t* bar) {
   asm volatile(
       "{\n .reg .pred e;\n elect.sync _|e, 0xffffffff;\n"
@@ -203,6 +207,11 @@ __device__ __forceinline__ uint64_t desc_sw128(uint32_t smem_addr) {
 // bits 17-22, M >> 4 in bits 24-28.
 __host__ __device__ constexpr uint32_t idesc_bf16_f32(int M, int N) {
   return (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(N >> 3) << 17) | ((uint32_t)(M >> 4) << 24);
+}
+
+// The same with A and B in FP16 (format 0).
+__host__ __device__ constexpr uint32_t idesc_fp16_f32(int M, int N) {
+  return (1u << 4) | ((uint32_t)(N >> 3) << 17) | ((uint32_t)(M >> 4) << 24);
 }
 
 // Instruction descriptor of kind::tf32: f32 accumulator (bits 4-5 = 1), A and B

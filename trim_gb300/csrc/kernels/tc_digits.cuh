@@ -1,10 +1,11 @@
 // Digit slicing shared by the tensor-core GEMM kernels: the power-of-two
-// row/column scale, the balanced signed digits of an FP64 value as exact BF16
-// values (6 of 9 bits in the tiled form, 7 of 7 bits in the fused form), and
-// the 128-byte swizzled K-major operand layout of tcgen05 shared-memory
-// descriptors.
+// row/column scale, the balanced signed digits of an FP64 value as exact 16-bit
+// values (6 of 9 bits, FP16, in the tiled form; 7 of 7 bits, BF16, in the fused
+// form), and the 128-byte swizzled K-major operand layout of tcgen05
+// shared-memory descriptors.
 #pragma once
 #include <cuda_bf16.h>
+#include <cuda_fp16.h>
 
 #include <cstdint>
 
@@ -53,16 +54,11 @@ __device__ __forceinline__ uint32_t scaled_f32_bits(double x, int e) {
 // FP32 from the bit pattern of 1.5 * 2^(23-7s) + d * 2^-7s (integer add into
 // the mantissa, one exact subtraction); it has at most 8 significant bits, so
 // its BF16 pattern is the top half of the FP32 pattern.
-// NS = 6: X = |x| * 2^(53 - e) rounded to the nearest integer (X <= 2^53), V =
-// +-X and its balanced base-512 digits (d_1..d_5 in [-256, 255], |d_0| <= 256)
-// read out of Y = V + 256 * (1 + 512 + ... + 512^4) the same way.  They are
-// stored as plain integers (BF16 holds every integer up to 256), so one magic
-// number, 1.5 * 2^23, serves all of them.
 // NS = 1 (fast mode): the BF16 rounding of the FP32 rounding of x * 2^(7-e),
 // the scaling done on the exponent field.
 template <int NS>
 __device__ __forceinline__ void make_slices(const double (&x)[8], int e, uint4 (&out)[NS]) {
-  static_assert(NS == 1 || NS == 6 || NS == 7, "6 or 7 digits (split) or one BF16 slice (fast)");
+  static_assert(NS == 1 || NS == 7, "7 digits (split) or one BF16 slice (fast)");
   uint32_t packed[NS][4];
 #pragma unroll
   for (int j = 0; j < 4; j++) {  // pair by pair, so few digits are held at once
@@ -80,24 +76,10 @@ __device__ __forceinline__ void make_slices(const double (&x)[8], int e, uint4 (
           mant |= 1ull << 52;
           E = ef - 1023;
         }
-        const int sh = (NS == 7 ? 3 : -1) + e - E;  // X = mant * 2^(E - 52) * 2^(49 - e), or 2^(53 - e) for 6 digits
+        const int sh = 3 + e - E;  // X = mant * 2^(E - 52) * 2^(49 - e)
         const uint64_t X = (sh >= 64) ? 0ull : (sh > 0 ? ((mant + (1ull << (sh - 1))) >> sh) : (mant << (-sh)));
         const long long V = (bits >> 63) ? -(long long)X : (long long)X;
-        if constexpr (NS == 6) {
-          const uint64_t Y = (uint64_t)(V + 17626613022976ll);  // + 256 * (512^5 - 1) / 511
-          const uint32_t lo = (uint32_t)Y, hi = (uint32_t)(Y >> 32);
-          // the five lower digits plus 256, in the low bits
-          const uint32_t d[6] = {(uint32_t)((int)hi >> 13),
-                                 (hi >> 4) & 511u,
-                                 __funnelshift_r(lo, hi, 27) & 511u,
-                                 (lo >> 18) & 511u,
-                                 (lo >> 9) & 511u,
-                                 lo & 511u};
-          const float magic = __uint_as_float(0x4B400000u);  // 1.5 * 2^23
-#pragma unroll
-          for (int s = 0; s < 6; s++)
-            hbits[s][i] = __float_as_uint(__uint_as_float(0x4B400000u + d[s]) - (s ? magic + 256.f : magic));
-        } else if constexpr (NS == 7) {
+        if constexpr (NS == 7) {
           const uint64_t Y = (uint64_t)(V + 2216338399296ll);  // + 64 * (128^6 - 1) / 127
           const uint32_t lo = (uint32_t)Y, hi = (uint32_t)(Y >> 32);
           int d[7];
@@ -121,6 +103,64 @@ __device__ __forceinline__ void make_slices(const double (&x)[8], int e, uint4 (
   }
 #pragma unroll
   for (int s = 0; s < NS; s++) out[s] = make_uint4(packed[s][0], packed[s][1], packed[s][2], packed[s][3]);
+}
+
+// The six digits of the tiled split form: V = x * 2^(53 - e) rounded to the
+// nearest integer (|V| <= 2^53) and its balanced base-512 digits (d_1..d_5 in
+// [-256, 255], |d_0| <= 256) as FP16 integers.  Y = 512 (V + 256 (1 + 512 + ...
+// + 512^5)), below 2^64, has the digits plus 256 at bits 9, 18, 27, 36, 45 and
+// 54; two elements' worth of one are packed into the mantissas of two FP16 in
+// [1024, 2048) and 1280 subtracted.  About 30 integer instructions an element:
+// the sign goes in as a bit inversion (V's last 2^-9), a shift past the top gives
+// 0 for elements below 2^-62 of the scale and for zeros, and only where the
+// scale itself is near the subnormals does an element's own exponent take the
+// general form.  (The same in BF16, element by element with 64-bit shifts and a
+// rounding of its own, took about 65; slicing 80000 x 400 153 -> 138 us.)
+__device__ __forceinline__ void make_digits(const double (&x)[8], int e, uint4 (&out)[6]) {
+  constexpr uint64_t kBias = (256ull * ((1ull << 54) - 1) / 511) * 512 + 256;  // and half a unit: rounds
+  uint32_t lo[8], hi[8];
+  if (e > -900) {
+#pragma unroll
+    for (int i = 0; i < 8; i++) {
+      const uint32_t h = (uint32_t)__double2hiint(x[i]), l = (uint32_t)__double2loint(x[i]);
+      const uint32_t m = (h & 0xFFFFFu) | 0x100000u, t1 = __funnelshift_l(l, m, 9), t0 = l << 9;  // mantissa * 512
+      const int sh = min(e + 1022 - (int)((h >> 20) & 0x7FFu), 63);
+      const bool far = sh >= 32;
+      const uint32_t a1 = far ? 0u : t1, a0 = far ? t1 : t0, s = (uint32_t)((int)h >> 31);
+      const uint64_t w = ((uint64_t)((a1 >> (sh & 31)) ^ s) << 32) | (__funnelshift_r(a0, a1, sh) ^ s);
+      const uint64_t y = w + kBias;
+      lo[i] = (uint32_t)y, hi[i] = (uint32_t)(y >> 32);
+    }
+  } else {
+#pragma unroll
+    for (int i = 0; i < 8; i++) {
+      const uint64_t bits = (uint64_t)__double_as_longlong(x[i]);
+      const int ef = (int)((bits >> 52) & 0x7FF);
+      const uint64_t mant = (bits & ((1ull << 52) - 1)) | (ef ? 1ull << 52 : 0);
+      const int sh = e + 1022 - max(ef, 1);  // V = mant * 2^-sh
+      const uint64_t X = sh >= 64 ? 0ull : (sh > 0 ? (mant + (1ull << (sh - 1))) >> sh : mant << -sh);
+      const uint64_t y = (((bits >> 63) ? 0ull - X : X) << 9) + kBias;
+      lo[i] = (uint32_t)y, hi[i] = (uint32_t)(y >> 32);
+    }
+  }
+  auto digit = [](uint32_t two, uint32_t mask) {
+    const uint32_t v = (two & mask) | 0x64006400u;
+    const __half2 d = __hsub2(*(const __half2*)&v, __half2(__ushort_as_half(0x6500), __ushort_as_half(0x6500)));
+    return *(const uint32_t*)&d;
+  };
+  uint32_t packed[6][4];
+#pragma unroll
+  for (int j = 0; j < 4; j++) {
+    const uint32_t l0 = lo[2 * j], l1 = lo[2 * j + 1], h0 = hi[2 * j], h1 = hi[2 * j + 1];
+    packed[0][j] = digit(__byte_perm(h0, h1, 0x7632) >> 6, 0x03FF03FFu);  // bits 22..31 of the high words
+    packed[1][j] = digit(__byte_perm(h0, h1, 0x6521) >> 5, 0x01FF01FFu);  // 13..21
+    packed[2][j] = digit(__byte_perm(h0, h1, 0x5410) >> 4, 0x01FF01FFu);  // 4..12
+    packed[3][j] = digit(__byte_perm(__funnelshift_r(l0, h0, 27), __funnelshift_r(l1, h1, 27), 0x5410), 0x01FF01FFu);
+    packed[4][j] = digit(__byte_perm(l0, l1, 0x7632) >> 2, 0x01FF01FFu);  // 18..26 of the low words
+    packed[5][j] = digit(__byte_perm(l0, l1, 0x6521) >> 1, 0x01FF01FFu);  // 9..17
+  }
+#pragma unroll
+  for (int s = 0; s < 6; s++) out[s] = make_uint4(packed[s][0], packed[s][1], packed[s][2], packed[s][3]);
 }
 
 // TF32 fast mode: 8 consecutive-k values of one row as TF32 patterns of
