@@ -490,9 +490,12 @@ void launch_tc_maxima(const TcSector* secs, int nsec, const int64_t* a_ts, int64
                       unsigned long long* bmax, int64_t nmax, int num_sms, cudaStream_t s);
 // both in one pass over the operands; items: (sector, s) for the 16-column
 // strip s of B, (sector, -1 - r) for the rows 8 r .. 8 r + 7 of A, or its row r
-// where K > kRowWarp
-constexpr int kRowWarp = 2000;
-void launch_tc_slice_once(int ns, const TcSector* secs, const int2* items, int nitems, const double* A,
+// where K > kRowWarp.  Strips of more than kSliceWideK rows are shared by
+// slice_group(K) CTAs of a cluster of kSliceCluster; their items come first, one
+// per kSliceCluster / group strips: (sector, the first of them)
+constexpr int kRowWarp = 2000, kSliceWideK = 576, kSliceCluster = 4;
+__host__ __device__ constexpr int slice_group(int K) { return K <= 2 * kSliceWideK ? 2 : 4; }
+void launch_tc_slice_once(int ns, const TcSector* secs, const int2* items, int nshared, int nitems, const double* A,
                           const double* B, unsigned long long* ea, unsigned long long* eb, uint8_t* images,
                           int num_sms, cudaStream_t s);
 void launch_tc_slices(int ns, const TcSector* secs, int nsec, const int64_t* a_ts, int64_t a_tiles,

@@ -24,7 +24,7 @@ struct TcPlan {
   size_t off_secs = 0, off_si = 0, off_at = 0, off_bt = 0, off_it = 0, off_rit = 0;
   int nsec = 0, nitems = 0, nred = 0;
   int wide = 1;    // 64-column tiles per item (fast modes)
-  int nslice = 0;  // items of the one-pass slicing, 0: tile by tile
+  int nslice = 0, nshared = 0;  // items of the one-pass slicing, 0: tile by tile; shared ones before them
   int64_t part_elems = 0;  // FP64 partial tiles of the K-split sectors
   int64_t rows = 0, cols = 0, max_k = 0, a_tiles = 0, b_tiles = 0, img = 0;
   double flops = 0, in_bytes = 0;
@@ -136,26 +136,33 @@ static std::shared_ptr<TcPlan> build_tc_plan(Ctx& ctx, const std::vector<tn_sect
   P->nitems = (int)items.size();
   P->nred = (int)ritems.size();
   if (!P->nsec) return P;
-  // One pass over the operands, an item over all of K, or maxima and images
-  // tile by tile in two launches (also for a list whose items would not number
-  // in 32 bits).  The two launches read everything twice, 1.4 times the time of
-  // one pass over a full chip, and take at least 20 us; one pass lasts at least
-  // as long as its longest item, whose CTA slices about 1000 elements a
-  // microsecond.  A 484 x 484 product over K = 234256 has 31 strips of B with
-  // 3.7 M elements each: 1.0 ms in two launches, 3.6 ms in one.
+  // One pass over the operands, or maxima and images tile by tile in two launches
+  // (also for a list whose items would not number in 32 bits).  The two launches
+  // read everything twice, tiles of 64 k at a time: about 36 us and 127 000
+  // elements a microsecond.  One pass lasts at least as long as its longest item,
+  // a quarter of a strip of 16 columns, whose CTA slices about 530 elements a
+  // microsecond beyond what it stages.  Measured in split precision, one pass and
+  // two launches: 484 x 484 over K = 10648 78 and 97 us, over K = 80000 601 and 623,
+  // 81 x 81 over K = 6561 101 (before strips were shared) and 29 us.
   int64_t nsl = 0;
   for (const auto& s : secs) nsl += cdiv(s.N, 16) + (s.K > kRowWarp ? s.M : cdiv(s.M, 8));
-  const double two_passes = 20 + 1.4 * P->in_bytes / 8 / 330e3, longest_item = 16.0 * P->max_k / 1000;
+  const double two_launches = 36 + P->in_bytes / 8 / 127e3, longest_item = 16.0 / kSliceCluster * P->max_k / 530;
   std::vector<int2> sitems;
-  if (nsl < INT32_MAX / 2 && longest_item <= two_passes) {
+  if (nsl < INT32_MAX / 2 && longest_item <= two_launches) {
     sitems.reserve(nsl);
     for (int g = 0; g < P->nsec; g++)
-      for (int64_t c = 0; c < cdiv(secs[g].N, 16); c++) sitems.push_back(make_int2(g, (int)c));
+      if (secs[g].K > kSliceWideK)
+        for (int64_t c = 0; c < cdiv(secs[g].N, 16); c += kSliceCluster / slice_group(secs[g].K))
+          sitems.push_back(make_int2(g, (int)c));
+    P->nshared = (int)sitems.size();
+    for (int g = 0; g < P->nsec; g++)
+      if (secs[g].K <= kSliceWideK)
+        for (int64_t c = 0; c < cdiv(secs[g].N, 16); c++) sitems.push_back(make_int2(g, (int)c));
     for (int g = 0; g < P->nsec; g++)
       for (int64_t r = 0; r < (secs[g].K > kRowWarp ? secs[g].M : cdiv(secs[g].M, 8)); r++)
         sitems.push_back(make_int2(g, (int)(-1 - r)));
   }
-  P->nslice = (int)sitems.size();
+  P->nslice = (int)sitems.size() - P->nshared;
   const int n1 = P->nsec + 1;
   P->off_secs = 0;
   P->off_at = P->off_secs + P->nsec * sizeof(TcSector);
@@ -217,10 +224,10 @@ void run_tc_gemms(Ctx& ctx, int ns, const std::vector<tn_sector_gemm>& list, con
   int* err = ctx.device_error_word();
   const int64_t* ats = (const int64_t*)(mb + P->off_at);
   const int64_t* bts = (const int64_t*)(mb + P->off_bt);
-  if (P->nslice) {
+  if (P->nslice) {  // rows of A among them
     ProfScope ps(ctx, "tc_slice", P->in_bytes * (1.0 + 0.25 * ns), 0);
-    launch_tc_slice_once(ns, dsecs, (const int2*)(mb + P->off_si), P->nslice, A, B, ea, eb, images, ctx.num_sms,
-                         ctx.stream);
+    launch_tc_slice_once(ns, dsecs, (const int2*)(mb + P->off_si), P->nshared, P->nslice, A, B, ea, eb, images,
+                         ctx.num_sms, ctx.stream);
     ctx.launched();
   } else {
     {

@@ -223,16 +223,22 @@ __device__ __forceinline__ void slice_b_tile(const TcSector* __restrict__ secs, 
 // each; one row beyond kRowWarp k) or a strip of 16 columns of B, over all of
 // K.  What an item holds in shared memory (74 KB, three CTAs per SM: rows of
 // up to kRowKeep k per warp or 8192 per CTA, strips of up to kWideK) is read from
-// memory once; longer ones are read again, through L2.  Staging is by
-// cp.async, 16 bytes a copy where the row (the strip's rows) starts on 16 bytes,
-// else 8; a thread then slices 8 consecutive k.  8 bytes are read and 2 bytes
-// per digit written per element, 4.9 TB/s on 80000 rows or columns of 400 in
-// split precision (4.2 with 8-byte copies and reads and the digits of
-// make_slices): the instructions per element decide (107 there), not the
-// loads' latency - bringing the next item into L2 ahead made it slower.  Only what the GEMM uses is written:
-// no row past M or column past N (accumulator rows and columns nobody reads),
-// no k past the last 16-k step.
-constexpr int kStageDoubles = 9216, kRowKeep = 1024, kWideK = 576;
+// memory once; longer rows are read again, through L2.  A strip of more k is
+// shared by the 2 or 4 CTAs that hold it together (the rest of its k, from 2304
+// on, is read again), which exchange their maxima through distributed shared
+// memory; a cluster of 4 leaves few SM slots empty, one of 8 every ninth.  8192
+// columns of 4096 beside 1024 rows: 225 -> 169 us against a strip per CTA (whose
+// second reads no longer found 240 MB of strips in flight in L2), 1024
+// contractions of bonds 16..256 1507 -> 1061 us.
+// Staging is by cp.async, 16 bytes a copy where the row (the strip's rows) starts
+// on 16 bytes, else 8; a thread then slices 8 consecutive k.  8 bytes are read and
+// 2 bytes per digit written per element, 4.9 TB/s on 80000 rows of 400 in split
+// precision, 5.6 as columns (4.2 with 8-byte copies and reads and a digit at a
+// time): the instructions per element decide (107 there), not the loads' latency
+// - bringing the next item into L2 ahead made it slower.  Only what the GEMM uses
+// is written: no row past M or column past N (accumulator rows and columns nobody
+// reads), no k past the last 16-k step.
+constexpr int kStageDoubles = 9216, kRowKeep = 1024, kWideK = kSliceWideK;
 // 18 doubles per 16: 16-byte reads of 8 consecutive k per lane without bank conflicts
 __host__ __device__ constexpr int padded(int k) { return k + (k >> 4 << 1); }
 static_assert(8 * padded(kRowKeep) <= kStageDoubles && padded(8192) <= kStageDoubles && 16 * kWideK <= kStageDoubles,
@@ -240,6 +246,7 @@ static_assert(8 * padded(kRowKeep) <= kStageDoubles && padded(8192) <= kStageDou
 
 struct SliceShared {
   uint32_t part[8][16];
+  uint32_t peer[2][16];  // this CTA's maxima of a shared strip, for its group
   unsigned long long full[16];
 };
 
@@ -356,51 +363,50 @@ __device__ __forceinline__ int image_row(int n) {
   return (n & ~15) | ((n & 2) << 2) | ((n & 12) >> 1) | (n & 1);
 }
 
-// 16 columns of B by a CTA: thread (c, g) slices of column c the groups g, g +
-// 16, .. of 8 k
-template <int NS>
-__device__ __forceinline__ void slice_strip(const TcSector& S, int64_t strip, const double* __restrict__ B,
-                                            unsigned long long* __restrict__ eb, uint8_t* __restrict__ ws, double* buf,
-                                            SliceShared& sh) {
+// 16 columns of B, their k kb .. ke - 1 (multiples of 16, or the end) by this
+// CTA: thread (c, g) slices of column c the groups g, g + 16, .. of 8 k.  SHARED:
+// the strip's ranges are those of `group` CTAs of the cluster; they exchange
+// their maxima (through buffer `par` in turn, so one barrier an item is enough).
+template <int NS, bool SHARED>
+__device__ __forceinline__ void slice_strip(const TcSector& S, int64_t strip, int kb, int ke, int group, int par,
+                                            const double* __restrict__ B, unsigned long long* __restrict__ eb,
+                                            uint8_t* __restrict__ ws, double* buf, SliceShared& sh) {
   constexpr int W = 16, kPass = 8 * 256 / W;
   const int c = threadIdx.x % W, g = threadIdx.x / W, warp = threadIdx.x >> 5;
   const int64_t n = strip * W + c;
   const int cols = n < S.N ? S.K : 0;  // k values this thread's column has
   const double* src = B + S.b_off + n;
-  const int kend = (S.K + 15) & ~15;
-  const bool keep = kend <= kWideK;
-  auto at = [&](int k) { return k * W + c; };
+  const int ks = SHARED ? min(ke, kb + kWideK) : ke;  // up to here it is staged
+  auto at = [&](int k) { return (k - kb) * W + c; };
   auto load = [&](int k, double(&v)[8]) {
 #pragma unroll
     for (int q = 0; q < 8; q++) v[q] = k + q < cols ? __ldg(src + (int64_t)(k + q) * S.N) : 0.0;
   };
   uint32_t hi = 0;
-  if (keep) {
-    const double* s0 = B + S.b_off + strip * W;
-    if (strip * W + W <= S.N && ((uintptr_t)s0 & 15) == 0 && (S.N & 1) == 0) {  // two columns a copy
-      const int p = 2 * (threadIdx.x & 7);
+  const double* s0 = B + S.b_off + strip * W;
+  if (strip * W + W <= S.N && ((uintptr_t)s0 & 15) == 0 && (S.N & 1) == 0) {  // two columns a copy
+    const int p = 2 * (threadIdx.x & 7);
 #pragma unroll 4
-      for (int k = threadIdx.x >> 3; k < kend; k += 32)
-        cp_async16(buf + k * W + p, k < S.K ? s0 + (int64_t)k * S.N + p : s0, k < S.K ? 16 : 0);
-    } else {
-      for (int k = g; k < kend; k += 16)
-        cp_async8(buf + at(k), k < cols ? src + (int64_t)k * S.N : B, k < cols);
-    }
-    cp_async_commit();
-    cp_async_wait<0>();
-    __syncthreads();
-    for (int k = g * 8; k < kend; k += kPass)
-#pragma unroll
-      for (int q = 0; q < 8; q++) hi = max(hi, abs_hi(buf[at(k + q)]));
+    for (int k = kb + (threadIdx.x >> 3); k < ks; k += 32)
+      cp_async16(buf + (k - kb) * W + p, k < S.K ? s0 + (int64_t)k * S.N + p : s0, k < S.K ? 16 : 0);
   } else {
-    for (int k = g * 8; k < cols; k += 2 * kPass) {  // 16 loads in flight
+    for (int k = kb + g; k < ks; k += 16)
+      cp_async8(buf + at(k), k < cols ? src + (int64_t)k * S.N : B, k < cols);
+  }
+  cp_async_commit();
+  if (SHARED)
+    for (int k = ks + g * 8; k < ke; k += 2 * kPass) {  // 16 loads in flight
       double x[8], y[8];
       load(k, x);
       load(k + kPass, y);
 #pragma unroll
       for (int q = 0; q < 8; q++) hi = max(hi, max(abs_hi(x[q]), abs_hi(y[q])));
     }
-  }
+  cp_async_wait<0>();
+  __syncthreads();
+  for (int k = kb + g * 8; k < ks; k += kPass)
+#pragma unroll
+    for (int q = 0; q < 8; q++) hi = max(hi, abs_hi(buf[at(k + q)]));
 #pragma unroll
   for (int o = W; o < 32; o <<= 1) hi = max(hi, __shfl_xor_sync(0xffffffffu, hi, o));
   __syncthreads();  // the previous item's maxima have been read
@@ -409,6 +415,12 @@ __device__ __forceinline__ void slice_strip(const TcSector& S, int64_t strip, co
   __syncthreads();
 #pragma unroll
   for (int w = 0; w < 8; w++) hi = max(hi, sh.part[w][c]);
+  if (SHARED) {
+    if (threadIdx.x < W) sh.peer[par][c] = hi;
+    cluster_sync();
+    const uint32_t rank = cluster_rank(), first = rank - rank % group;
+    for (int p = 0; p < group; p++) hi = max(hi, ld_cluster(&sh.peer[par][c], first + p));
+  }
   const bool low = (hi >> 20) == 0;  // zero or subnormal column: the full pattern decides
   if (low) {
     unsigned long long m = 0;
@@ -417,21 +429,20 @@ __device__ __forceinline__ void slice_strip(const TcSector& S, int64_t strip, co
   }
   __syncthreads();
   const unsigned long long m = low ? sh.full[c] : (unsigned long long)hi << 32;
-  if (g == 0 && n < S.N) eb[S.eb_off + n] = m;
+  if (g == 0 && n < S.N && kb == 0) eb[S.eb_off + n] = m;
   if (n >= S.N) return;
   const int e = exp_of(m);
   uint8_t* img = ws + S.b_img + (n / kTN) * S.nkt * NS * kBTile;
   const int r = image_row((int)(n % kTN));
   double x[8];
-  if (keep) {
-    for (int k = g * 8; k < kend; k += kPass) {
+  for (int k = kb + g * 8; k < ks; k += kPass) {
 #pragma unroll
-      for (int q = 0; q < 8; q++) x[q] = buf[at(k + q)];
-      store_chunk<NS>(img + (int64_t)(k / kTK) * NS * kBTile, kBTile, r, (k / 8) % 8, x, e);
-    }
-  } else {
-    load(g * 8, x);
-    for (int k = g * 8; k < kend; k += kPass) {  // the next group loads while this one is sliced
+    for (int q = 0; q < 8; q++) x[q] = buf[at(k + q)];
+    store_chunk<NS>(img + (int64_t)(k / kTK) * NS * kBTile, kBTile, r, (k / 8) % 8, x, e);
+  }
+  if (SHARED) {
+    load(ks + g * 8, x);
+    for (int k = ks + g * 8; k < ke; k += kPass) {  // the next group loads while this one is sliced
       double y[8];
       load(k + kPass, y);
       store_chunk<NS>(img + (int64_t)(k / kTK) * NS * kBTile, kBTile, r, (k / 8) % 8, x, e);
@@ -441,25 +452,44 @@ __device__ __forceinline__ void slice_strip(const TcSector& S, int64_t strip, co
   }
 }
 
-// items: (sector, strip of B), or (sector, -1 - row group of A)
-template <int NS>
+// items: the shared ones (sector, first of the strips that a cluster takes at
+// once), then (sector, strip of B), or (sector, -1 - row group of A)
+template <int NS, bool SHARED>
 __global__ void __launch_bounds__(256, 3) tc_slice_once(const TcSector* __restrict__ secs,
-                                                        const int2* __restrict__ items, int nitems,
+                                                        const int2* __restrict__ items, int nshared, int nitems,
                                                         const double* __restrict__ A, const double* __restrict__ B,
                                                         unsigned long long* __restrict__ ea,
                                                         unsigned long long* __restrict__ eb, uint8_t* __restrict__ ws) {
   __shared__ SliceShared sh;
-  extern __shared__ double stage[];  // kStageDoubles
+  extern __shared__ __align__(16) double stage[];  // kStageDoubles
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  int2 next = items[blockIdx.x];
   bool cta = false;  // the last item used the buffer as a CTA
-  for (int t = blockIdx.x; t < nitems; t += gridDim.x) {
+  int t0 = blockIdx.x;
+  if (SHARED) {
+    const int rank = (int)cluster_rank(), clusters = gridDim.x / kSliceCluster;
+    int par = 0;
+    for (int t = blockIdx.x / kSliceCluster; t < nshared; t += clusters, par ^= 1) {
+      const int2 it = items[t];
+      const TcSector& S = secs[it.x];
+      const int kend = (S.K + 15) & ~15, group = slice_group(S.K), kper = ((kend >> 4) + group - 1) / group * 16;
+      const int kb = rank % group * kper;
+      __syncthreads();
+      slice_strip<NS, true>(S, it.y + rank / group, kb, max(kb, min(kend, kb + kper)), group, par, B, eb, ws, stage, sh);
+    }
+    cta = true;
+    cluster_sync();  // the peers have read this CTA's maxima
+    // clusters that had one shared item less take the first of the others
+    t0 = (int)((blockIdx.x + gridDim.x - nshared % clusters * kSliceCluster) % gridDim.x);
+  }
+  items += nshared;
+  int2 next = t0 < nitems ? items[t0] : make_int2(0, 0);
+  for (int t = t0; t < nitems; t += gridDim.x) {
     const int2 it = next;
     if (t + gridDim.x < nitems) next = items[t + gridDim.x];
     const TcSector& S = secs[it.x];
     if (it.y >= 0) {
       __syncthreads();
-      slice_strip<NS>(S, it.y, B, eb, ws, stage, sh);
+      slice_strip<NS, false>(S, it.y, 0, (S.K + 15) & ~15, 1, 0, B, eb, ws, stage, sh);
       cta = true;
     } else if (S.K > kRowWarp) {
       __syncthreads();
@@ -524,20 +554,50 @@ void launch_tc_maxima(const TcSector* secs, int nsec, const int64_t* a_ts, int64
   TN_CUDA(cudaGetLastError());
 }
 
-void launch_tc_slice_once(int ns, const TcSector* secs, const int2* items, int nitems, const double* A,
+template <int NS>
+static void launch_once(const TcSector* secs, const int2* items, int nshared, int nitems, const double* A,
+                        const double* B, unsigned long long* ea, unsigned long long* eb, uint8_t* images, int num_sms,
+                        cudaStream_t s) {
+  constexpr int smem = kStageDoubles * (int)sizeof(double);
+  if (!nshared) {
+    static bool attr = false;
+    if (!attr) {
+      TN_CUDA(cudaFuncSetAttribute(tc_slice_once<NS, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+      attr = true;
+    }
+    tc_slice_once<NS, false>
+        <<<std::min(nitems, num_sms * 3), 256, smem, s>>>(secs, items, 0, nitems, A, B, ea, eb, images);
+    TN_CUDA(cudaGetLastError());
+    return;
+  }
+  cudaLaunchConfig_t cfg{};
+  cfg.blockDim = dim3(256);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = s;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeClusterDimension;
+  at[0].val.clusterDim.x = kSliceCluster;
+  at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = 1;
+  cfg.gridDim = dim3((unsigned)(num_sms * 3 / kSliceCluster * kSliceCluster));
+  static int resident = 0;  // clusters the GPU holds at once
+  if (!resident) {
+    TN_CUDA(cudaFuncSetAttribute(tc_slice_once<NS, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+    int n = 0;
+    TN_CUDA(cudaOccupancyMaxActiveClusters(&n, tc_slice_once<NS, true>, &cfg));
+    resident = std::max(1, n);
+  }
+  const int clusters = std::min(resident, std::max(nshared, (nitems + kSliceCluster - 1) / kSliceCluster));
+  cfg.gridDim = dim3((unsigned)(clusters * kSliceCluster));
+  TN_CUDA(cudaLaunchKernelEx(&cfg, tc_slice_once<NS, true>, secs, items, nshared, nitems, A, B, ea, eb, images));
+}
+
+void launch_tc_slice_once(int ns, const TcSector* secs, const int2* items, int nshared, int nitems, const double* A,
                           const double* B, unsigned long long* ea, unsigned long long* eb, uint8_t* images,
                           int num_sms, cudaStream_t s) {
-  const int grid = std::min(nitems, num_sms * 3);
-  auto k = ns == kSplitDigits ? tc_slice_once<kSplitDigits> : (ns == 2 ? tc_slice_once<2> : tc_slice_once<1>);
-  constexpr int smem = kStageDoubles * (int)sizeof(double);
-  static bool attr[3] = {false, false, false};  // per instantiation
-  bool& done = attr[ns == kSplitDigits ? 0 : ns];
-  if (!done) {
-    TN_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-    done = true;
-  }
-  k<<<grid, 256, smem, s>>>(secs, items, nitems, A, B, ea, eb, images);
-  TN_CUDA(cudaGetLastError());
+  auto launch = ns == kSplitDigits ? launch_once<kSplitDigits> : (ns == 2 ? launch_once<2> : launch_once<1>);
+  launch(secs, items, nshared, nitems, A, B, ea, eb, images, num_sms, s);
 }
 
 void launch_tc_slices(int ns, const TcSector* secs, int nsec, const int64_t* a_ts, int64_t a_tiles,

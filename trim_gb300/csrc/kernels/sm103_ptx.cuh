@@ -93,6 +93,24 @@ __device__ __forceinline__ void cp_async_wait() {
 }
 __device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;" ::: "memory"); }
 
+__device__ __forceinline__ uint32_t cluster_rank() {
+  uint32_t r;
+  asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+  return r;
+}
+// every thread of the cluster: shared-memory writes before it are seen after it
+__device__ __forceinline__ void cluster_sync() {
+  asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+__device__ __forceinline__ uint32_t ld_cluster(const uint32_t* p, uint32_t rank) {  // p in CTA `rank`
+  uint32_t v;
+  asm volatile("{\n .reg .u32 a;\n mapa.shared::cluster.u32 a, %1, %2;\n ld.shared::cluster.u32 %0, [a];\n}\n"
+               : "=r"(v)
+               : "r"(smem_u32(p)), "r"(rank)
+               : "memory");
+  return v;
+}
+
 // 32 bytes in one store (sm_100 and up); four lanes write a row's 128 bytes
 __device__ __forceinline__ void store4(double* p, const double* v) {
   asm volatile("st.global.v4.f64 [%0], {%1, %2, %3, %4};" ::"l"(__cvta_generic_to_global(p)), "d"(v[0]), "d"(v[1]),
