@@ -524,7 +524,7 @@ void launch_tc_fused(int ns, const TcSector* secs, const int4* items, int nitems
                      cudaStream_t s);
 // C tile = sum over the K ranges of its FP64 partial tiles, in range order, scaled
 void launch_tc_reduce(int ns, const TcSector* secs, const int4* ritems, int nred, const double* part, double* C,
-                      const unsigned long long* ea, const unsigned long long* eb, int grid, cudaStream_t s);
+                      const unsigned long long* ea, const unsigned long long* eb, int num_sms, cudaStream_t s);
 void launch_scale(double* p, int64_t n, double a, cudaStream_t s);
 
 // A rows x cols piece of a product with a diagonal factor (RDotR's

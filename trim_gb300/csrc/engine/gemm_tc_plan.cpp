@@ -254,8 +254,7 @@ void run_tc_gemms(Ctx& ctx, int ns, const std::vector<tn_sector_gemm>& list, con
   }
   if (P->nred > 0) {
     ProfScope ps(ctx, "tc_reduce", 0, 0);
-    const int grid = (int)std::min<int64_t>((int64_t)P->nred, (int64_t)ctx.num_sms * 4);
-    launch_tc_reduce(ns, dsecs, (const int4*)(mb + P->off_rit), P->nred, part, C, ea, eb, grid, ctx.stream);
+    launch_tc_reduce(ns, dsecs, (const int4*)(mb + P->off_rit), P->nred, part, C, ea, eb, ctx.num_sms, ctx.stream);
     ctx.launched();
   }
 }

@@ -521,22 +521,29 @@ __global__ void __launch_bounds__(256) tc_slices(const TcSector* __restrict__ se
 }
 
 // ---------------------------------------------------------------- K ranges
-// one CTA per split output tile: C = the sum of its partial tiles in K-range
-// order, scaled by 2^(ea + eb - unit) (the split kernel's partial tiles carry
-// no unit)
+// C = the sum of an output tile's partial tiles in K-range order, scaled by
+// 2^(ea + eb - unit) (the split kernel's partial tiles carry no unit).  A tile is
+// cut into `parts` bands of rows, an item each, as far as it takes to fill the
+// chip: the ranges are summed one after another, and with few tiles (which is
+// where ranges come from) a CTA per tile read up to 64 of them by itself.
+// 32 tiles of 19 ranges 89 -> 13 us, 2 tiles of 53 ranges 270 -> 27.
+constexpr int kReduceParts = 32;  // at most: one output per thread
 __global__ void __launch_bounds__(256) tc_reduce(const TcSector* __restrict__ secs, const int4* __restrict__ ritems,
-                                                 int nred, const double* __restrict__ part, double* __restrict__ C,
-                                                 const unsigned long long* __restrict__ ea,
+                                                 int nred, int parts, const double* __restrict__ part,
+                                                 double* __restrict__ C, const unsigned long long* __restrict__ ea,
                                                  const unsigned long long* __restrict__ eb, int unit) {
-  for (int it = blockIdx.x; it < nred; it += gridDim.x) {
-    const int4 w = ritems[it];
+  const int band = kTM * kTN / parts;
+  for (int it = blockIdx.x; it < nred * parts; it += gridDim.x) {
+    const int4 w = ritems[it / parts];
     const TcSector& S = secs[w.x];
     const double* p = part + S.p_off + ((int64_t)w.y * S.nnt + w.z) * S.nsplit * (kTM * kTN);
-    for (int e = threadIdx.x; e < kTM * kTN; e += blockDim.x) {
+    const int e0 = it % parts * band;
+    for (int e = e0 + threadIdx.x; e < e0 + band; e += 256) {
       const int64_t i = (int64_t)w.y * kTM + e / kTN, j = (int64_t)w.z * kTN + e % kTN;
       if (i >= S.M || j >= S.N) continue;
       double s = 0.0;
-      for (int q = 0; q < S.nsplit; q++) s += p[(int64_t)q * (kTM * kTN) + e];
+#pragma unroll 8
+      for (int q = 0; q < S.nsplit; q++) s += __ldg(p + (int64_t)q * (kTM * kTN) + e);
       C[S.c_off + i * S.N + j] = scale_pow2(s, exp_of(ea[S.ea_off + i]) + exp_of(eb[S.eb_off + j]) - unit);
     }
   }
@@ -615,9 +622,12 @@ void launch_tc_slices(int ns, const TcSector* secs, int nsec, const int64_t* a_t
 }
 
 void launch_tc_reduce(int ns, const TcSector* secs, const int4* ritems, int nred, const double* part, double* C,
-                      const unsigned long long* ea, const unsigned long long* eb, int grid, cudaStream_t s) {
+                      const unsigned long long* ea, const unsigned long long* eb, int num_sms, cudaStream_t s) {
   if (nred <= 0) return;
-  tc_reduce<<<grid, 256, 0, s>>>(secs, ritems, nred, part, C, ea, eb, ns == kSplitDigits ? 0 : 14);
+  int parts = 1;
+  while (parts < kReduceParts && (int64_t)nred * parts < 4 * num_sms) parts *= 2;
+  const int grid = (int)std::min<int64_t>((int64_t)nred * parts, (int64_t)num_sms * 8);
+  tc_reduce<<<grid, 256, 0, s>>>(secs, ritems, nred, parts, part, C, ea, eb, ns == kSplitDigits ? 0 : 14);
   TN_CUDA(cudaGetLastError());
 }
 
