@@ -575,8 +575,8 @@ void launch_svd_qr(const int64_t* tab, int njobs, const double* A, double* ws, s
 void launch_svd_v1(const int64_t* tab, int njobs, double* ws, size_t smem, cudaStream_t s);
 // dst = src^T (n x n) for every (n, src_off, dst_off) triple of tab (device)
 void launch_ns_transpose(const int64_t* tab, int njobs, double* ws, cudaStream_t s);
-void launch_truncate(const int64_t* s_off, const int64_t* s_cnt, int nsec, double* S, int64_t chi, int64_t* kept,
-                     double* norm, cudaStream_t s);
+void launch_truncate(const int64_t* s_off, const int64_t* s_cnt, int nsec, int64_t total, double* S, int64_t chi,
+                     int64_t* kept, double* norm, cudaStream_t s);
 void launch_gather_truncated(const TruncSector* secs, int nsec, const double* U, const double* S, const double* VT,
                              double* Uo, double* So, double* VTo, cudaStream_t s);
 void launch_transpose(const double* src, double* dst, int rows, int cols, cudaStream_t s);

@@ -507,6 +507,8 @@ double run_truncate(Ctx& ctx, const std::vector<int64_t>& s_off, const std::vect
   if (n == 0) return 0.0;
   for (int i = 0; i < n; i++)
     if (s_cnt[i] < 0 || s_off[i] < 0) fail(TN_ERR_ARG, "truncate: negative offset or count");
+  int64_t total = 0;
+  for (int64_t c : s_cnt) total += c;
   std::vector<int64_t> h(2 * (size_t)n);
   std::copy(s_off.begin(), s_off.end(), h.begin());
   std::copy(s_cnt.begin(), s_cnt.end(), h.begin() + n);
@@ -515,7 +517,7 @@ double run_truncate(Ctx& ctx, const std::vector<int64_t>& s_off, const std::vect
   TN_CUDA(cudaMemcpyAsync(d, h.data(), 2 * (size_t)n * sizeof(int64_t), cudaMemcpyHostToDevice, ctx.stream));
   {
     ProfScope ps(ctx, "truncate");
-    launch_truncate(d, d + n, n, S, chi, d + 2 * n, (double*)(d + 3 * n), ctx.stream);
+    launch_truncate(d, d + n, n, total, S, chi, d + 2 * n, (double*)(d + 3 * n), ctx.stream);
     ctx.launched();
   }
   std::vector<int64_t> out((size_t)n + 1);
