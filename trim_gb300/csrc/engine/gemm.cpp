@@ -502,18 +502,20 @@ constexpr int kModeFlags = TN_MODE_TC_ONLY | TN_MODE_TC_FUSED | TN_MODE_TC_TILED
 //
 // In split precision so does one that the FP64 kernel finishes sooner, both in
 // clocks of one SM as grouped launches of small sectors run: 1.6 FMAs a clock
-// there, against 4400 per 64 k of an output tile (3400 more to write it) and 1.9
+// there, against 5200 per 64 k of an output tile (4000 more to write it) and 1.9
 // per operand element to slice.  30 x 30 outputs take the tensor cores, 8 x 30
-// do not: on 1024 contractions of bonds 16..256 that moves 1403 of 3007 sectors,
-// 7% of the flop, and the call from 5.4 to 4.8 ms.  The fast modes keep the
-// sizes alone (there a sector's precision hangs on it), and so does a call that
-// asks for the tiled form.
+// do not: on 1024 contractions of bonds 16..256 that moves 1474 of 3007 sectors,
+// 8% of the flop, and with the size limits alone the call took 12% longer.  Of
+// these constants the sums over four lists (bonds 8..120 to 64..400) came out
+// lowest, 1 to 4% below those with a sixth less or a third less per tile.  The
+// fast modes keep the sizes alone (there a sector's precision hangs on it), and
+// so does a call that asks for the tiled form.
 static bool thin_sector(int mode, const tn_sector_gemm& g) {
   if (g.K < 16 || g.N < 16) return true;
   if ((mode & ~kModeFlags) != TN_MODE_SPLIT || (mode & TN_MODE_TC_TILED)) return false;
   const double m = (double)g.M, n = (double)g.N, k = (double)g.K;
   const double tiles = std::ceil(m / 128) * std::ceil(n / 64);
-  return m * n * k / 1.6 < tiles * (std::ceil(k / 64) * 4400 + 3400) + 1.9 * (m + n) * k;
+  return m * n * k / 1.6 < tiles * (std::ceil(k / 64) * 5200 + 4000) + 1.9 * (m + n) * k;
 }
 
 // The fused form fits a contraction of a few 128 x 64 output tiles per SM
