@@ -20,10 +20,12 @@ struct Dim {
 //         best source dim); y = the next destination dim, several rows/tile.
 // mode 1: 2-D transpose through shared memory: loads run along y (the
 //         source-contiguous dim), stores along x.
-// mode 3: mode-0 rows that are short on both sides (a few elements): tz
-//         row-sets of a third dim stacked into a dense [z][y][x] tile, loaded
-//         in source-stride order and stored in destination-stride order; where
+// mode 3: mode-0 rows whose [y][x] tile is less than half full: tz row-sets of
+//         a third dim stacked into a dense [z][y][x] tile, loaded in
+//         source-stride order and stored in destination-stride order; where
 //         that fills less than half a tile, tw values of a fourth dim repeat it.
+//         From a sixteenth of a tile on the third dim repeats the [y][x] tile
+//         instead (tz = 1).
 // mode 2: when a transpose tile of x and y is small (short bonds, e.g. 24 x
 //         24), a third dim z is stacked into it (tz planes of x by y) so
 //         that each tile still moves thousands of elements; z is the dim
@@ -63,6 +65,24 @@ void choose_tile(PermSub& ps, int es) {
     ps.tx = (int32_t)std::min<int64_t>(ps.dims[x], kRow);
     int64_t ty = std::min<int64_t>(kTile / ps.tx, kStage / (ps.tx + 1));
     ps.ty = (int32_t)std::min<int64_t>(ps.dims[y], std::min<int64_t>(ty, 1024));
+    // Narrower rows where that takes clearly fewer tiles: 96 x 96 as three tiles
+    // of 32 x 96, not 64 + 32 in both directions.  Transposes of 80^4, 96^4 and
+    // 100^4: 250, 360 and 489 us -> 155, 289 and 362 at most.  (16-byte elements
+    // keep their 64 x 32 tiles: 100 x 100 x 8 x 100 ran up to 10% slower in 52 x 34.)
+    auto tiles = [&](int64_t tx, int64_t ty) {
+      return ((ps.dims[x] + tx - 1) / tx) * ((ps.dims[y] + ty - 1) / ty);
+    };
+    int64_t best = tiles(ps.tx, ps.ty) * 7 / 8;
+    for (int64_t nx = (ps.dims[x] + kRow - 1) / kRow; es == 1 && ps.dims[x] / nx >= 32; nx++) {
+      const int64_t tx = std::min<int64_t>(kRow, ((ps.dims[x] + nx - 1) / nx + 3) & ~(int64_t)3);
+      const int64_t cap = std::min<int64_t>({kTile / tx, kStage / (tx + 1), 1024});
+      const int64_t ny = (ps.dims[y] + cap - 1) / cap, ty1 = (ps.dims[y] + ny - 1) / ny;
+      if (tiles(tx, ty1) <= best) {
+        best = tiles(tx, ty1) - 1;
+        ps.tx = (int32_t)tx;
+        ps.ty = (int32_t)ty1;
+      }
+    }
   } else {
     ps.tx = (int32_t)std::min<int64_t>(ps.dims[x], kTile);
     if (n >= 2) {
@@ -82,10 +102,14 @@ void choose_tile(PermSub& ps, int es) {
       ps.ty = 1;
     }
   }
-  // mode 3: rows contiguous on both sides but short (e.g. the charge runs of
-  // a combined bond, 4 elements): a third dim, the one with the smallest
-  // source or destination stride, stacks tz row-sets into one dense tile
-  if (ps.mode == 0 && n >= 3 && (int64_t)ps.tx * ps.ty <= kTile / 16) {
+  // mode 3: rows contiguous on both sides but few to a tile (the charge runs of
+  // a combined bond, 4 elements; 24 rows of 24): a third dim, the one with the
+  // smallest source or destination stride, stacks tz row-sets into one dense
+  // tile.  Where the [y][x] tile has an element or more per thread, the third dim
+  // repeats it with a constant step: a 24^6 permute with the last bond in place
+  // took 1990 us in 576-element tiles, 945 with an index computation per element
+  // (tz), under 650 with one for every 7.
+  if (ps.mode == 0 && n >= 3 && (int64_t)ps.tx * ps.ty <= kTile / 2) {
     int z = -1;
     int64_t best = 0;
     for (int i = 0; i < n - 1; i++) {
@@ -97,7 +121,11 @@ void choose_tile(PermSub& ps, int es) {
       }
     }
     const int64_t tz = std::min<int64_t>((int64_t)ps.dims[z], kTile / ((int64_t)ps.tx * ps.ty));
-    if (tz > 1) {
+    if (tz > 1 && (int64_t)ps.tx * ps.ty > kTile / 16) {
+      ps.mode = 3;
+      ps.wdim = z;
+      ps.tw = (int32_t)tz;
+    } else if (tz > 1) {
       ps.mode = 3;
       ps.zdim = z;
       ps.tz = (int32_t)tz;
