@@ -30,7 +30,8 @@ struct Dim {
 //         24), a third dim z is stacked into it (tz planes of x by y) so
 //         that each tile still moves thousands of elements; z is the dim
 //         with the smallest source or destination stride (it extends a
-//         contiguous run on one side).
+//         contiguous run on one side); of 8-byte elements tw values of a
+//         fourth dim are added where that leaves the tile half empty.
 //
 // Limits are in elements: a tile <= 4096 elements and a transpose tile within
 // 64 x 65 for 8-byte elements; es = 2 (16-byte elements) halves both, so a
@@ -149,6 +150,17 @@ void choose_tile(PermSub& ps, int es) {
       }
     }
   }
+  // A destination row of a few elements beside a long source row: the source run
+  // leaves room for the dim that continues the destination row, to 32 elements.
+  // (The tile of 2 x 1000 wrote 16 bytes at a time: (200, 2, 200, 1000) -> (1000,
+  // 200, 200, 2) 930 -> 400 us.  Complex rows of two fill a sector: no gain.)
+  if (es == 1 && ps.mode == 1 && ps.dims[x] < 16 && n >= 3)
+    for (int i = 0; i < n; i++)
+      if (i != x && i != y && ps.dstride[i] == ps.dims[x]) {
+        const int64_t tz = std::min<int64_t>(ps.dims[i], (32 + ps.tx - 1) / ps.tx);
+        const int64_t cap = std::min(kTile / (ps.tx * tz), kStage / ((ps.tx + 1) * tz)) & ~(int64_t)3;
+        if (cap >= 32 && ps.dims[y] > 2 * cap) ps.ty = (int32_t)cap;
+      }
   if (ps.mode == 1 && (int64_t)ps.tx * ps.ty <= kTile / 2 && n >= 3) {
     int z = -1;
     int64_t best = 0;
@@ -166,6 +178,27 @@ void choose_tile(PermSub& ps, int es) {
       ps.mode = 2;
       ps.zdim = z;
       ps.tz = (int32_t)tz;
+      // and a fourth dim where that leaves the tile half empty: 6^9 transposes
+      // 144 -> 66 us at most (216-element tiles; complex ones, whose tiles hold half
+      // as many and whose single elements fill a 16-byte access, lost up to half)
+      const int64_t tile = (int64_t)ps.tx * ps.ty * tz;
+      int w = -1;
+      if (es == 1 && tile <= kTile / 2)
+        for (int i = 0; i < n; i++) {
+          if (i == x || i == y || i == z) continue;
+          const int64_t c = std::min(ps.sstride[i], ps.dstride[i]);
+          if (w < 0 || c < best) {
+            w = i;
+            best = c;
+          }
+        }
+      if (w >= 0) {
+        const int64_t tw = std::min<int64_t>({(int64_t)ps.dims[w], kStage / (tz * ps.ty * (ps.tx + 1)), kTile / tile});
+        if (tw > 1) {
+          ps.wdim = w;
+          ps.tw = (int32_t)tw;
+        }
+      }
     }
   }
   ps.ntx = (int32_t)((ps.dims[x] + ps.tx - 1) / ps.tx);

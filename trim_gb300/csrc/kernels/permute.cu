@@ -257,7 +257,16 @@ __device__ __forceinline__ void issue_tile(const Info& w, const T* __restrict__ 
         if (xx >= w.nx || yy >= w.ny) continue;
         const T* g = src + w.bs + (int64_t)yy * w.sy + (int64_t)xx * w.sx;
         T* sp = buf + yy * pitch + xx;
-        for (int zz = 0; zz < w.nz; zz++, g += w.sz, sp += plane) cp_async_el(sp, g);
+        if constexpr (Info::kShortRows) {
+          const T* gw = g;
+          for (int ww = 0; ww < w.nw; ww++, gw += w.sw) {
+            sp = buf + yy * pitch + xx + ww * w.tz * plane;
+            g = gw;
+            for (int zz = 0; zz < w.nz; zz++, g += w.sz, sp += plane) cp_async_el(sp, g);
+          }
+        } else {
+          for (int zz = 0; zz < w.nz; zz++, g += w.sz, sp += plane) cp_async_el(sp, g);
+        }
       }
     } else if (w.mode == 3) {
       // [w][z][y][x] dense; elements of a (z, y, x) block in source-stride order,
@@ -339,7 +348,16 @@ __device__ __forceinline__ void store_tile(const Info& w, const T* buf, T* __res
       if (xx >= w.nx || yy >= w.ny) continue;
       const T* sp = buf + yy * pitch + xx;
       T* g = dst + w.bd + (int64_t)yy * w.dy + (int64_t)xx * w.dx;
-      for (int zz = 0; zz < w.nz; zz++, sp += plane, g += w.dz) *g = apply_flip(*sp, f);
+      if constexpr (Info::kShortRows) {
+        T* gw = g;
+        for (int ww = 0; ww < w.nw; ww++, gw += w.dw) {
+          sp = buf + yy * pitch + xx + ww * w.tz * plane;
+          g = gw;
+          for (int zz = 0; zz < w.nz; zz++, sp += plane, g += w.dz) *g = apply_flip(*sp, f);
+        }
+      } else {
+        for (int zz = 0; zz < w.nz; zz++, sp += plane, g += w.dz) *g = apply_flip(*sp, f);
+      }
     }
     return;
   }
@@ -561,9 +579,9 @@ int64_t check_permute_plan_host(const PermPlan& plan, const double* src, double*
     const TileInfoW w = decode_tile<TileInfoW>(P, t - P.tile_begin);
     if (w.nx > w.tx || w.ny > w.ty || w.nz > w.tz || w.nw > w.tw || w.nx <= 0 || w.ny <= 0 || w.nz <= 0 || w.nw <= 0)
       fail(TN_ERR_ARG, "plan check: bad tile extents");
-    if (w.mode != 3 && w.tw != 1) fail(TN_ERR_ARG, "plan check: a fourth tile dim outside mode 3");
+    if (w.mode < 2 && w.tw != 1) fail(TN_ERR_ARG, "plan check: a fourth tile dim outside modes 2 and 3");
     if (w.mode < 2 && w.tz != 1) fail(TN_ERR_ARG, "plan check: stacked planes outside modes 2 and 3");
-    const int64_t stage = (w.mode == 1 || w.mode == 2) ? (int64_t)w.tz * w.ty * (w.tx + 1) : (int64_t)w.tw * w.tz * w.tx * w.ty;
+    const int64_t stage = (w.mode == 1 || w.mode == 2) ? (int64_t)w.tw * w.tz * w.ty * (w.tx + 1) : (int64_t)w.tw * w.tz * w.tx * w.ty;
     if (stage > kSmem / es) fail(TN_ERR_ARG, "plan check: tile exceeds shared memory");
     if ((int64_t)w.tx * w.ty * w.tz * w.tw > (int64_t)kThreads * kPerThread)
       fail(TN_ERR_ARG, "plan check: tile exceeds thread walk");
