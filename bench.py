@@ -9,7 +9,7 @@ whose sector GEMMs are chi^8-sized.  Metric: contract() TFLOP/s counted as
 the FP64-equivalent sum of 2*M*N*K over the sector GEMMs the reference
 issues for these networks and ORDERs (the same count in every precision
 mode).  The headline is the split-precision mode (FP64 operands cut into
-BF16 digit slices multiplied on the tcgen05 tensor cores, FP32 accumulation,
+16-bit digit slices multiplied on the tcgen05 tensor cores, FP32 accumulation,
 FP64 recombination); the plain FP64 GPU form is timed beside it and every
 result states its error against that FP64 output.
 
@@ -89,10 +89,11 @@ def kernels_dtype(names) -> str:
     tc_bf16 = any(n.endswith("_bf16") for n in names if n.startswith("tc_"))
     tc_tf32 = any(n.endswith("_tf32") for n in names if n.startswith("tc_"))
     f64 = "gemm_fp64" in names
+    digits = "7 bf16" if "tc_gemm_split" not in names else "6 fp16"
     if tc_split and f64:
-        return "f64 (split: 7 bf16 digit slices on tcgen05, fp32 accumulation, fp64 recombination; thin sectors on the fp64 kernel)"
+        return f"f64 (split: {digits} digit slices on tcgen05, fp32 accumulation, fp64 recombination; thin sectors on the fp64 kernel)"
     if tc_split:
-        return "f64 (split: 7 bf16 digit slices on tcgen05, fp32 accumulation, fp64 recombination)"
+        return f"f64 (split: {digits} digit slices on tcgen05, fp32 accumulation, fp64 recombination)"
     if tc_bf16:
         return "bf16 (tcgen05, fp32 accumulation)"
     if tc_tf32:
@@ -220,8 +221,9 @@ def measured_fp64_peak(torch, n=4096, reps=5):
 
 def roofline_of(torch, prof, steps_done, peaks, sustained):
     """Roofline of the dominant kernel (most device time) of a profiled run.
-    Tensor-core GEMMs count 34 BF16 digit products per FP64-equivalent flop
-    (split) and are set against the measured cuBLAS BF16 rate (sustained for
+    Tensor-core GEMMs count the 16-bit digit products per FP64-equivalent flop
+    (split: 21 in the tiled form, 34 in the fused one; FP16 and BF16 run at one
+    rate) and are set against the measured cuBLAS BF16 rate (sustained for
     a kernel timed inside a long step, else burst); FP64 GEMMs against a
     cuBLAS DGEMM measured in this run; permute and slicing against the
     measured HBM copy rate."""
@@ -239,13 +241,13 @@ def roofline_of(torch, prof, steps_done, peaks, sustained):
                 "peak_source": "measured in this run: cuBLAS DGEMM 4096^3 (torch.matmul float64), best of 5",
                 "peak_nominal": 1.25, "algorithmic_flops_per_launch": d["flops"] / d["launches"]}
     else:
-        pairs = 34 if "split" in dname else 1
+        pairs = {"tc_gemm_split": 21, "tc_fused_split": 34}.get(dname, 1)
         ach = pairs * d["flops"] / d["launches"] / (avg_ms * 1e-3) / 1e12
         key = "bf16_tflops_sustained" if sustained else "bf16_tflops"
         peak = peaks.get(key, 1700.0 if sustained else 1900.0)
         roof = {"bound": "tensor", "achieved": ach, "peak": peak, "unit": "TFLOP/s",
                 "peak_source": (f"measured (MEASURED_PEAKS.json {key})" if key in peaks else "fallback"),
-                "work": ("BF16 tensor flops: 34 digit products per FP64-equivalent flop" if pairs > 1 else "BF16 flops"),
+                "work": (f"16-bit tensor flops: {pairs} digit products per FP64-equivalent flop" if pairs > 1 else "BF16 flops"),
                 "fp64_equivalent_flops_per_launch": d["flops"] / d["launches"]}
         if "bf16_tflops" in peaks:
             roof["frac_of_burst"] = ach / peaks["bf16_tflops"]
@@ -448,13 +450,13 @@ def mera_section(args, torch, tu, stream, local, world, peaks):
 
 
 # dram__bytes_read.sum + dram__bytes_write.sum of one chi^8 tc_gemm_split
-# launch of the chi=16 diagrams (ncu, 236.9 + 92.4 MB), scaled by the operand
-# elements (24/16)^6 to the chi=24 launch of the same contraction
+# launch at chi=16 (65536 x 256 over K = 256; ncu, 202.8 + 93.7 MB), scaled by
+# the operand elements (24/16)^6 to the chi=24 launch of the same contraction
 TC_GEMM_TRAFFIC_NOTE = {
-    "traffic": 3.75e9, "traffic_unit": "bytes per chi^8 launch (the big-operand contractions)",
-    "traffic_source": "ncu on the chi=16 diagrams (329.3 MB for one chi^8 launch: the digit images read once, "
+    "traffic": 3.38e9, "traffic_unit": "bytes per chi^8 launch (the big-operand contractions)",
+    "traffic_source": "ncu on the chi=16 product (296.5 MB for one chi^8 launch: the digit images read once, "
                       "the output partly still in L2), scaled by (24/16)^6; algorithmic bytes of that launch "
-                      "at chi=24: 4.2 GB (digit images 14 B + FP64 output 8 B per element)"}
+                      "at chi=24: 3.8 GB (digit images 12 B + FP64 output 8 B per element)"}
 
 
 # ----------------------------------------------------------------- iTEBD

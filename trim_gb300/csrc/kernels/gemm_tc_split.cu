@@ -55,14 +55,15 @@
 // columns 16 ((w - 2) >> 2) .. +15 of each level.
 //
 // Measured (GB300, all of a call's launches): the left MERA diagram at chi = 24
-// (K = 576, 6.7e11 FP64-equivalent flop) 16.0 -> 9.5 ms, the iPEPS quadrant at
-// chi = 128, D = 8 (K = 4096, 1.4e11) 3.41 -> 1.76 ms, against the 34-product
-// kernel.  21 products per FP64 multiply-add: 80 TFLOP/s FP64-equivalent at
-// K = 4096 is 1 690 of FP16, and the tensor pipe alone (no loads, no drain, no
-// output) takes 1.51 ms; at K = 576 the FP64 output of every ninth tile (64 KB at
-// the 30 B per clock that an SM stores, whatever the pattern, as long as a row's
-// 128 bytes go together: 17 B per clock with a row per lane) stalls the drain
-// and, through the ring, the MMAs for 1.4 ms of the 9.5.
+// (K = 576, 6.7e11 FP64-equivalent flop) 16.0 -> 10.0 ms, the iPEPS quadrant at
+// chi = 128, D = 8 (K = 4096, 1.4e11) 3.41 -> 1.83 ms, against the 34-product
+// kernel.  21 products per FP64 multiply-add: 77 TFLOP/s FP64-equivalent at
+// K = 4096 is 1 620 of FP16.  What bounds it, from copies with parts left out:
+// 80000 x 576 over K = 576 takes 761 us, 677 without the drain's arithmetic, 596
+// without the output as well (64 KB of FP64 every ninth tile, about 8 000 clocks in
+// which the ring fills and the MMAs stop), 574 without loads; 4096^3 1703, 1619,
+// 1607 and 1505 us.  Converting by magic-number additions instead of cvt changed
+// nothing (its range check cost 10%), nor did loading A two digits at a time.
 #include <cstdint>
 
 #include "../engine/engine.h"
