@@ -51,11 +51,12 @@ enum {
 /* ---- precision of the sector GEMMs ------------------------------------- */
 enum {
   TN_MODE_FP64 = 0,      /* plain FP64 GEMM per sector: the drop-in form */
-  TN_MODE_SPLIT = 1,     /* split-precision: BF16 slices on tcgen05, FP64-level error */
+  TN_MODE_SPLIT = 1,     /* split-precision: 16-bit digit slices on tcgen05, FP64-level error */
   TN_MODE_FAST_BF16 = 2, /* one BF16 slice, FP32 accumulation */
   TN_MODE_FAST_TF32 = 3, /* TF32 operands (tcgen05 kind::tf32, tiled form), FP32 accumulation */
   /* flag: in the tensor-core modes, send every sector to the tensor cores
-   * (by default a sector with K < 16 or N < 16 runs on the exact FP64
+   * (by default a sector with K < 16 or N < 16, and in split precision
+   * one that the FP64 kernel finishes sooner, runs on the exact FP64
    * kernel instead) */
   TN_MODE_TC_ONLY = 0x100,
   /* flags choosing the tensor-core form (by default: where every sector
@@ -64,7 +65,7 @@ enum {
    * kernel, timed once per sector-size histogram; the tiled form above that).
    * Fused: one launch, each CTA slices the operands of its own tile.
    * Tiled: operand maxima and slices once per contraction, then the
-   * pipelined GEMM over pre-sliced tiles (3 launches). */
+   * pipelined GEMM over pre-sliced tiles (2 to 4 launches). */
   TN_MODE_TC_FUSED = 0x200,
   TN_MODE_TC_TILED = 0x400
 };
