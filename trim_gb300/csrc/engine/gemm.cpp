@@ -150,8 +150,11 @@ std::vector<GemmTile> plan_fp64(const std::vector<tn_sector_gemm>& list, int num
 }
 
 // Flat items.  Cost is counted in warp FMAs (slots x K): an SM sub-partition
-// runs one at a time, so items are cut to about a sixteenth of its share (at
+// runs one at a time, so items are cut to about a 24th of its share (at
 // least 64 warp FMAs, below which an item's own latency shows; at most 4096).
+// (Sixteenths were up to 7% slower, on 64 uneven contractions 414 -> 386 us, an
+// iPEPS quadrant at chi = 48, D = 5 460 -> 448; 48ths up to 6% faster still on some
+// lists and 2% slower on others.)
 // Sectors of at least 128 outputs are cut into chunks of at most 4 slots (one
 // slot while an item is small: K ranges, with their partial sums, are the
 // second choice), each with its K ranges as a group; smaller ones deal all
@@ -164,7 +167,7 @@ std::vector<FlatItem> plan_fp64_flat(const std::vector<tn_sector_gemm>& list, in
   double total = 0;
   for (const auto& g : list)
     if (g.M > 0 && g.N > 0 && g.K > 0) total += std::ceil((double)g.M * g.N / 32.0) * (double)g.K;
-  const int64_t target = (int64_t)std::min(4096.0, std::max(64.0, total / (4.0 * num_sms * 16.0)));
+  const int64_t target = (int64_t)std::min(4096.0, std::max(64.0, total / (4.0 * num_sms * 24.0)));
   std::vector<FlatItem> out;
   int64_t ws = 0, ngrp = 0;
   const int64_t most_plain = std::max<int64_t>(1, std::min<int64_t>(kFlatSlots, target / 256));  // slots per chunk
