@@ -13,7 +13,8 @@ from trim_gb300 import workloads as wl
 
 DIMS = [(5, 9, 24, 24), (24, 7, 11, 17), (3, 50, 2, 30), (2, 3, 40, 65), (9, 65, 70), (96, 2, 100), (81, 130, 3), (33, 64, 5, 16),
         (8, 4, 8, 32), (2, 67, 2, 129), (3, 2, 1000), (2, 5, 3, 700),
-        (20, 3, 700, 2), (7, 40, 300, 3), (3, 4, 5, 6, 7), (2, 7, 2, 9, 10), (4, 4, 4, 4, 4, 4)]
+        (20, 3, 700, 2), (7, 40, 300, 3), (3, 4, 5, 6, 7), (2, 7, 2, 9, 10), (4, 4, 4, 4, 4, 4),
+        (9000, 2), (4100, 3), (333, 31), (65, 32), (700, 63), (5, 64)]
 
 
 @pytest.mark.parametrize("dims", DIMS)

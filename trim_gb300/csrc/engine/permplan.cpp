@@ -66,6 +66,15 @@ void choose_tile(PermSub& ps, int es) {
     ps.tx = (int32_t)std::min<int64_t>(ps.dims[x], kRow);
     int64_t ty = std::min<int64_t>(kTile / ps.tx, kStage / (ps.tx + 1));
     ps.ty = (int32_t)std::min<int64_t>(ps.dims[y], std::min<int64_t>(ty, 1024));
+    // A short source row with no third dim to stack: longer destination rows, so
+    // that the tile fills.  (3000, 3000, 3) with the last bond first 782 -> 86 us, 3e6
+    // x 7 268 -> 73, 24^4 x 24 37 -> 29; from half a tile of 64-element rows on the
+    // power of two is worth more, 60 x 60^3 41 -> 46 us, complex 24 x 4e5 60 -> 64.
+    if (n == 2 && ps.dims[y] <= (es == 1 ? 32 : 15)) {
+      const int64_t tx = std::min(kTile / ps.dims[y], kStage / ps.dims[y] - 1) & ~(int64_t)3;
+      ps.tx = (int32_t)std::min<int64_t>(ps.dims[x], tx);
+      ps.ty = (int32_t)ps.dims[y];
+    }
     // Narrower rows where that takes clearly fewer tiles: 96 x 96 as three tiles
     // of 32 x 96, not 64 + 32 in both directions.  Transposes of 80^4, 96^4 and
     // 100^4: 250, 360 and 489 us -> 155, 289 and 362 at most.  (16-byte elements
