@@ -165,7 +165,7 @@ __global__ void __launch_bounds__(kThreadsFast, 1) tc_gemm_fast(const TcSector* 
       // the copies already issued must land before the CTA's shared memory goes away
       for (int i = 0; i < kStages; i++) {
         const uint32_t uses = n / kStages + (i < (int)(n % kStages) ? 1 : 0);
-        if (uses) mbar_wait(&sh.full[i], (uses - 1) & 1, &sh.abort);
+        if (uses) mbar_drain(&sh.full[i], (uses - 1) & 1);
       }
     }
   } else if (warp == 1) {
@@ -214,7 +214,7 @@ __global__ void __launch_bounds__(kThreadsFast, 1) tc_gemm_fast(const TcSector* 
     if (!ok && lane == 0) raise_timeout(sh, err);
     // every MMA issued must complete before the tensor memory is released
     mma_commit_elect(&sh.mma_done);
-    mbar_wait(&sh.mma_done, 0, &sh.abort);
+    mbar_drain(&sh.mma_done, 0);
   } else {
     // ------------------------------------------------ epilogue
     const int quad = warp & 3;         // TMEM lanes 32*quad .. +31
@@ -237,7 +237,7 @@ __global__ void __launch_bounds__(kThreadsFast, 1) tc_gemm_fast(const TcSector* 
         col_max[c] = c < cols && j < S.N ? __ldg(eb + S.eb_off + j) : 0;
       }
       const uint32_t buf = tile & 1;
-      if (!mbar_wait(&sh.acc_full[buf], (tile >> 1) & 1, &sh.abort)) {
+      if (!warp_wait(&sh.acc_full[buf], (tile >> 1) & 1, &sh)) {
         ok = false;
         break;
       }

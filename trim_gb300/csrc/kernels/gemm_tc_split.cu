@@ -329,11 +329,11 @@ __global__ void __launch_bounds__(kThreadsSplit, 1) tc_gemm_split(const TcSector
       // the copies already issued must land before the CTA's shared memory goes away
       for (int i = 0; i < kARing; i++) {
         const uint32_t uses = na / kARing + (i < (int)(na % kARing) ? 1 : 0);
-        if (uses) mbar_wait(&sh.fullA[i], (uses - 1) & 1, &sh.abort);
+        if (uses) mbar_drain(&sh.fullA[i], (uses - 1) & 1);
       }
       for (int i = 0; i < kBRing; i++) {
         const uint32_t uses = nb / kBRing + (i < (int)(nb % kBRing) ? 1 : 0);
-        if (uses) mbar_wait(&sh.fullB[i], (uses - 1) & 1, &sh.abort);
+        if (uses) mbar_drain(&sh.fullB[i], (uses - 1) & 1);
       }
     }
   } else if (warp == 1) {
@@ -358,7 +358,7 @@ __global__ void __launch_bounds__(kThreadsSplit, 1) tc_gemm_split(const TcSector
     if (!ok && lane == 0) raise_timeout(sh, err);
     // every MMA issued must complete before the tensor memory is released
     mma_commit_elect(&sh.mma_done);
-    mbar_wait(&sh.mma_done, 0, &sh.abort);
+    mbar_drain(&sh.mma_done, 0);
   } else {
     // ------------------------------------------------ epilogue
     const int quad = warp & 3;         // TMEM lanes 32*quad .. +31
@@ -389,7 +389,7 @@ __global__ void __launch_bounds__(kThreadsSplit, 1) tc_gemm_split(const TcSector
 #pragma unroll
           for (int j = 0; j < 3; j++) {
             const int slot = g % kSlots;
-            if (!mbar_wait(&sh.fullT[slot], (g / kSlots) & 1, &sh.abort)) {
+            if (!warp_wait(&sh.fullT[slot], (g / kSlots) & 1, &sh)) {
               ok = false;
               break;
             }

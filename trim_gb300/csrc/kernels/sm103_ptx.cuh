@@ -54,9 +54,18 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, volati
     if (mbar_try_wait(bar, parity)) return true;
     if ((i & 255) == 0) {
       if (*abort) return false;
-      if (globaltimer_ns() - t0 > kWaitLimitNs) return false;
+      // signed: a timer that was set back a little between two reads has not run out
+      if ((int64_t)(globaltimer_ns() - t0) > (int64_t)kWaitLimitNs) return false;
     }
   }
+}
+
+// The same for what a kernel has to see finished before it may leave: its own
+// copies (they would land in the next CTA's shared memory) and MMAs (they would
+// write freed tensor memory).  Another thread's abort does not end it.
+__device__ __forceinline__ bool mbar_drain(uint64_t* bar, uint32_t parity) {
+  int never = 0;
+  return mbar_wait(bar, parity, &never);
 }
 
 // Whether a phase completed, without waiting.  The tensor pipe takes few MMAs
