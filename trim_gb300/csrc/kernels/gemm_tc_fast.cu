@@ -62,6 +62,7 @@ __device__ __forceinline__ bool warp_wait(uint64_t* bar, uint32_t parity, FastSh
 // warp: 32 TMEM lanes x 16 columns in the accumulator fragment order (see
 // tmem_ld32x16x2 in gemm_tc_split.cu)
 __device__ __forceinline__ void tmem_ld32x16(uint32_t a, uint32_t (&r)[16]) {
+  __syncwarp();
   asm volatile(
       "tcgen05.ld.sync.aligned.16x256b.x2.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%16];\n"
       "tcgen05.ld.sync.aligned.16x256b.x2.b32 {%8,%9,%10,%11,%12,%13,%14,%15}, [%17];\n"

@@ -212,6 +212,7 @@ __device__ __forceinline__ int split_tile(MmaState& st) {
 // data is in the registers on return.
 __device__ __forceinline__ void tmem_ld32x16x2(uint32_t a, uint32_t b, float (&v)[16], float (&w)[16]) {
   uint32_t r[16], s[16];
+  __syncwarp();
   asm volatile(
       "tcgen05.ld.sync.aligned.16x256b.x2.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%32];\n"
       "tcgen05.ld.sync.aligned.16x256b.x2.b32 {%8,%9,%10,%11,%12,%13,%14,%15}, [%33];\n"

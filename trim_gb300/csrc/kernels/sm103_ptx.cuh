@@ -109,7 +109,8 @@ __device__ __forceinline__ uint32_t cluster_rank() {
 }
 // every thread of the cluster: shared-memory writes before it are seen after it
 __device__ __forceinline__ void cluster_sync() {
-  asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+  __syncwarp();
+  asm volatile("barrier.cluster.arrive.release;\nbarrier.cluster.wait.acquire;" ::: "memory");
 }
 __device__ __forceinline__ uint32_t ld_cluster(const uint32_t* p, uint32_t rank) {  // p in CTA `rank`
   uint32_t v;
@@ -137,18 +138,24 @@ __device__ __forceinline__ void bulk_g2s(void* smem_dst, const void* gmem_src, u
 }
 
 // ---------------------------------------------------------------- tcgen05
+// The .sync.aligned ones want the warp whole.  Lanes that took different ways
+// before (a ragged row, the slow path of a conversion) are not brought together
+// by a CTA barrier or by the end of a loop, so each begins with __syncwarp().
 __device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
 
 // whole warp: allocate ncols tensor-memory columns, address written to *dst
 __device__ __forceinline__ void tmem_alloc(uint32_t* dst, uint32_t ncols) {
+  __syncwarp();
   asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(dst)), "r"(ncols)
                : "memory");
 }
 __device__ __forceinline__ void tmem_relinquish() {
+  __syncwarp();
   asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
 }
 __device__ __forceinline__ void tmem_dealloc(uint32_t taddr, uint32_t ncols) {
+  __syncwarp();
   asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(taddr), "r"(ncols) : "memory");
 }
 
@@ -203,6 +210,7 @@ __device__ __forceinline__ void mma_commit_elect(uint64_t* bar) {
 // warp: 32 lanes x 16 consecutive 32-bit columns starting at taddr
 __device__ __forceinline__ void tmem_ld16(uint32_t taddr, float* v) {
   uint32_t r[16];
+  __syncwarp();
   asm volatile(
       "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
       : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]),
