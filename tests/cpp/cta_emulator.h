@@ -289,6 +289,7 @@ inline int elected() { return (int)meet("elect.sync", 0)[0] * 0; }  // lane 0 of
 #define threadIdx (::emu::cur->tid)
 #define blockIdx (::emu::bid)
 #define gridDim (::emu::gdim)
+#define blockDim (::emu::Idx{::emu::nthreads, 1, 1})
 #define __launch_bounds__(...)
 template <class T>
 T __ldg(const T* p) { return *p; }
@@ -315,6 +316,25 @@ inline void __syncthreads() {
   } else {
     ::emu::block([g] { return ::emu::sync_gen != g; });
   }
+}
+template <class T>
+T __shfl_xor_sync(unsigned, T v, int mask) {
+  uint64_t b = 0;
+  memcpy(&b, &v, sizeof(T));
+  const uint64_t r = ::emu::meet("__shfl_xor_sync", b)[(::emu::tid() & 31) ^ mask];
+  memcpy(&v, &r, sizeof(T));
+  return v;
+}
+inline unsigned __reduce_max_sync(unsigned, unsigned x) {
+  const uint64_t* v = ::emu::meet("__reduce_max_sync", x);
+  uint64_t r = 0;
+  for (int i = 0; i < 32; i++) r = v[i] > r ? v[i] : r;
+  return (unsigned)r;
+}
+inline unsigned long long atomicMax(unsigned long long* p, unsigned long long v) {
+  const unsigned long long o = *p;
+  *p = v > o ? v : o;
+  return o;
 }
 inline int atomicExch(int* p, int v) {
   const int o = *p;
@@ -388,6 +408,25 @@ inline void bulk_g2s(void* dst, const void* src, uint32_t bytes, uint64_t* b) {
   copies.push_back(Copy{(uint8_t*)dst, (const uint8_t*)src, bytes, b, n_copies == hold_copy ? clock_ns + hold_ns : 0});
   n_copies++;
 }
+// cp.async: in order per thread here; an address has to be good even where nothing is read
+inline void cp_async(void* dst, const void* src, int bytes, int size) {
+  using namespace emu;
+  check(((uintptr_t)dst % size) == 0 && ((uintptr_t)src % size) == 0, "a cp.async off its alignment");
+  check((const uint8_t*)src >= gmem0 && (const uint8_t*)src + size_t(bytes ? bytes : 8) <= gmem1, "a cp.async with a bad address");
+  check((uint8_t*)dst >= dyn && (uint8_t*)dst + size <= dyn + dyn_bytes, "a cp.async outside the shared memory");
+  if (!failure.empty()) return;
+  memset(dst, 0, size);
+  memcpy(dst, src, bytes);
+}
+inline void cp_async8(void* dst, const void* src, bool valid) { cp_async(dst, src, valid ? 8 : 0, 8); }
+inline void cp_async16(void* dst, const void* src, int bytes) { cp_async(dst, src, bytes, 16); }
+inline void cp_async_commit() {}
+template <int N>
+void cp_async_wait() {}
+inline void cp_async_wait_all() {}
+inline uint32_t cluster_rank() { return 0; }
+inline void cluster_sync() {}
+inline uint32_t ld_cluster(const uint32_t* p, uint32_t) { return *p; }
 inline void tc_fence_before() {}
 inline void tc_fence_after() {}
 inline void tmem_alloc(uint32_t* dst, uint32_t n) {

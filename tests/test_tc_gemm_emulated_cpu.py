@@ -31,31 +31,39 @@ def _without_ptx(text):
 def _kernel(name):
     text = open(os.path.join(KERNELS, name)).read()
     body = text[text.index("namespace tn {"):]
+    body = re.sub(r"^// -+ launchers\n", "", body, flags=re.M)
     body = body[:re.search(r"^(?:template <int NS>\n)?void launch_", body, re.M).start()]
     body = body[:body.rindex("}  // namespace")] if body.rstrip().endswith("}  // namespace") else body
     body = body.replace("extern __shared__ uint8_t dyn[];", "uint8_t* dyn = ::emu::dyn;")
+    body = body.replace("extern __shared__ __align__(16) double stage[];", "double* stage = (double*)::emu::dyn;")
     return "namespace " + name.split(".")[0] + "_src {}\n" + _without_ptx(body) + "}\n}\n"
+
+
+def _build(d, program, *kernels):
+    if shutil.which("g++") is None:
+        pytest.skip("no g++")
+    cuda = os.environ.get("CUDA_HOME", "/usr/local/cuda")
+    ptx, digits = (open(os.path.join(KERNELS, f)).read().replace("#pragma once", "") for f in ("sm103_ptx.cuh", "tc_digits.cuh"))
+    (d / (program.replace("emulated.cpp", "processed.h"))).write_text('#include "engine/engine.h"\n' + _without_ptx(ptx) + digits + "".join(kernels))
+    for f in ("cta_emulator.h", program):
+        shutil.copy(os.path.join(ROOT, "tests", "cpp", f), d / f)
+    out = str(d / "emu")
+    p = subprocess.run(["g++", "-std=c++17", "-O2", "-w", "-I" + str(d), "-I" + os.path.join(ROOT, "trim_gb300", "csrc"),
+                        "-I" + os.path.join(cuda, "include"), str(d / program), "-o", out], capture_output=True, text=True)
+    assert p.returncode == 0, p.stderr[-4000:]
+    return out
 
 
 @pytest.fixture(scope="session")
 def exe(tmp_path_factory):
-    if shutil.which("g++") is None:
-        pytest.skip("no g++")
-    cuda = os.environ.get("CUDA_HOME", "/usr/local/cuda")
-    d = tmp_path_factory.mktemp("emu")
-    ptx = _without_ptx(open(os.path.join(KERNELS, "sm103_ptx.cuh")).read()).replace("#pragma once", "")
-    digits = open(os.path.join(KERNELS, "tc_digits.cuh")).read().replace("#pragma once", "")
-    split, fast = _kernel("gemm_tc_split.cu"), _kernel("gemm_tc_fast.cu")
     # the two files' anonymous constants side by side
-    fast = re.sub(r"\b(kTM|kTN|kTK|kATile|kBTile|kEpiWarps|kEpiCols|kUnit|raise_timeout|warp_wait)\b", r"\1Fast", fast)
-    (d / "tc_gemm_processed.h").write_text('#include "../engine/engine.h"\n'.replace("../engine", "engine") + ptx + digits + split + fast)
-    for f in ("cta_emulator.h", "tc_gemm_emulated.cpp"):
-        shutil.copy(os.path.join(ROOT, "tests", "cpp", f), d / f)
-    out = str(d / "emu")
-    p = subprocess.run(["g++", "-std=c++17", "-O2", "-w", "-I" + str(d), "-I" + os.path.join(ROOT, "trim_gb300", "csrc"),
-                        "-I" + os.path.join(cuda, "include"), str(d / "tc_gemm_emulated.cpp"), "-o", out], capture_output=True, text=True)
-    assert p.returncode == 0, p.stderr[-4000:]
-    return out
+    fast = re.sub(r"\b(kTM|kTN|kTK|kATile|kBTile|kEpiWarps|kEpiCols|kUnit|raise_timeout|warp_wait)\b", r"\1Fast", _kernel("gemm_tc_fast.cu"))
+    return _build(tmp_path_factory.mktemp("emu"), "tc_gemm_emulated.cpp", _kernel("gemm_tc_split.cu"), fast)
+
+
+@pytest.fixture(scope="session")
+def slice_exe(tmp_path_factory):
+    return _build(tmp_path_factory.mktemp("emu"), "tc_slice_emulated.cpp", _kernel("gemm_tc.cu"))
 
 
 def _run(exe, *args):
@@ -84,3 +92,12 @@ def test_a_wait_that_gives_up(exe, mode, hold):
     for seed in range(2):
         out = _run(exe, mode, 130, 130, 700, 99, 1 if mode == "split" else 2, seed, hold, 3 + 7 * seed)
         assert out == "timeout", out
+
+
+# rows and columns around the strips of 16 and the groups of 8, K around the
+# staged extents (1024 a warp, 8192 a CTA) and odd, from a null base
+@pytest.mark.parametrize("size", [(9, 17, 33), (1, 1, 1), (8, 16, 576), (3, 5, 1041), (2, 3, 2001), (1, 2, 8200), (20, 40, 100)])
+def test_slicing_addresses(slice_exe, size):
+    if size[2] > 576:  # longer strips are a cluster's
+        size = (size[0], 0, size[2])
+    assert _run(slice_exe, *size, 5) == "ok"

@@ -391,7 +391,7 @@ __device__ __forceinline__ void slice_strip(const TcSector& S, int64_t strip, in
       cp_async16(buf + (k - kb) * W + p, k < S.K ? s0 + (int64_t)k * S.N + p : s0, k < S.K ? 16 : 0);
   } else {
     for (int k = kb + g; k < ks; k += 16)
-      cp_async8(buf + at(k), k < cols ? src + (int64_t)k * S.N : B, k < cols);
+      cp_async8(buf + at(k), k < cols ? src + (int64_t)k * S.N : B + S.b_off, k < cols);
   }
   cp_async_commit();
   if (SHARED)

@@ -303,7 +303,7 @@ __global__ void __launch_bounds__(kFThreads, 1) tc_fused(const TcSector* __restr
           for (int j = 0; j < kFK / kGroups; j++) {
             const int k = kb + kGroups * j;
             const bool valid = k < kval && nvalid;
-            cp_async8(bst + k * kStride + bn, valid ? col + (int64_t)(k0 + k) * S.N : B, valid);
+            cp_async8(bst + k * kStride + bn, valid ? col + (int64_t)(k0 + k) * S.N : B + S.b_off, valid);
           }
         } else {
           const int64_t* rs = pool + bv->rs;
@@ -327,7 +327,7 @@ __global__ void __launch_bounds__(kFThreads, 1) tc_fused(const TcSector* __restr
               bbase = B + __ldg(pr) + coff;
               ld = __ldg(pr + 1);
             }
-            cp_async8(bst + k * kStride + bn, valid ? bbase + (k0 + k - r0) * ld : B, valid);
+            cp_async8(bst + k * kStride + bn, valid ? bbase + (k0 + k - r0) * ld : B + S.b_off, valid);
           }
         }
       }
