@@ -5,6 +5,7 @@
 
 #include <cuda_runtime.h>
 
+#include <atomic>
 #include <cstdint>
 #include <map>
 #include <memory>
@@ -30,6 +31,32 @@ void cuda_check(cudaError_t e, const char* what);
 #define TN_CUDA(x) ::tn::cuda_check((x), #x)
 void set_last_error(const std::string& msg);
 const char* last_error();
+
+// What a launcher settles once per device: a kernel's shared-memory attribute
+// (constant for the kernel), the clusters the device holds at once.  0 until
+// set; two threads that both find 0 set the same value twice.
+struct PerDevice {
+  std::atomic<int> value[64] = {};
+  template <class F>
+  int get(F&& make) {
+    int dev = 0;
+    TN_CUDA(cudaGetDevice(&dev));
+    std::atomic<int>& v = value[dev & 63];
+    int x = v.load(std::memory_order_acquire);
+    if (!x || dev > 63) {
+      x = make();
+      v.store(x, std::memory_order_release);
+    }
+    return x;
+  }
+};
+template <class K>
+inline void allow_smem(PerDevice& once, K kernel, size_t bytes) {
+  once.get([&] {
+    TN_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
+    return 1;
+  });
+}
 
 // ---------------------------------------------------------------- charges
 // Qnum (U1, parity, fermionic parity); order by key = U1*4 + prt*2 + prtF

@@ -567,11 +567,8 @@ static void launch_once(const TcSector* secs, const int2* items, int nshared, in
                         cudaStream_t s) {
   constexpr int smem = kStageDoubles * (int)sizeof(double);
   if (!nshared) {
-    static bool attr = false;
-    if (!attr) {
-      TN_CUDA(cudaFuncSetAttribute(tc_slice_once<NS, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-      attr = true;
-    }
+    static PerDevice attr;
+    allow_smem(attr, tc_slice_once<NS, false>, smem);
     tc_slice_once<NS, false>
         <<<std::min(nitems, num_sms * 3), 256, smem, s>>>(secs, items, 0, nitems, A, B, ea, eb, images);
     TN_CUDA(cudaGetLastError());
@@ -588,13 +585,13 @@ static void launch_once(const TcSector* secs, const int2* items, int nshared, in
   cfg.attrs = at;
   cfg.numAttrs = 1;
   cfg.gridDim = dim3((unsigned)(num_sms * 3 / kSliceCluster * kSliceCluster));
-  static int resident = 0;  // clusters the GPU holds at once
-  if (!resident) {
+  static PerDevice fit;  // clusters the GPU holds at once
+  const int resident = fit.get([&] {
     TN_CUDA(cudaFuncSetAttribute(tc_slice_once<NS, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
     int n = 0;
     TN_CUDA(cudaOccupancyMaxActiveClusters(&n, tc_slice_once<NS, true>, &cfg));
-    resident = std::max(1, n);
-  }
+    return std::max(1, n);
+  });
   const int clusters = std::min(resident, std::max(nshared, (nitems + kSliceCluster - 1) / kSliceCluster));
   cfg.gridDim = dim3((unsigned)(clusters * kSliceCluster));
   TN_CUDA(cudaLaunchKernelEx(&cfg, tc_slice_once<NS, true>, secs, items, nshared, nitems, A, B, ea, eb, images));

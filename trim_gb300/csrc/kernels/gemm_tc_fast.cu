@@ -300,11 +300,8 @@ void launch_fast(const TcSector* secs, const int4* items, int nitems, int wide, 
                  const unsigned long long* ea, const unsigned long long* eb, double* C, double* part, int* err, int grid,
                  cudaStream_t s) {
   constexpr size_t smem = (size_t)kStages * kStage + 1024;
-  static bool attr = false;  // per instantiation
-  if (!attr) {
-    TN_CUDA(cudaFuncSetAttribute(tc_gemm_fast<NS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    attr = true;
-  }
+  static PerDevice attr;  // per instantiation
+  allow_smem(attr, tc_gemm_fast<NS>, smem);
   tc_gemm_fast<NS><<<grid, kThreadsFast, smem, s>>>(secs, items, nitems, wide, ws, ea, eb, C, part, err);
   TN_CUDA(cudaGetLastError());
 }

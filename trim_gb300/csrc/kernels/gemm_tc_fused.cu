@@ -546,18 +546,12 @@ void launch_tc_fused(int ns, const TcSector* secs, const int4* items, int nitems
   if (nitems <= 0) return;
   const size_t smem = tc_fused_smem(ns);
   if (ns == 7) {
-    static bool attr = false;
-    if (!attr) {
-      TN_CUDA(cudaFuncSetAttribute(tc_fused<7>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-      attr = true;
-    }
+    static PerDevice attr;
+    allow_smem(attr, tc_fused<7>, smem);
     tc_fused<7><<<grid, kFThreads, smem, s>>>(secs, items, nitems, A, B, C, views, pool, err, rpi);
   } else {
-    static bool attr = false;
-    if (!attr) {
-      TN_CUDA(cudaFuncSetAttribute(tc_fused<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-      attr = true;
-    }
+    static PerDevice attr;
+    allow_smem(attr, tc_fused<1>, smem);
     tc_fused<1><<<grid, kFThreads, smem, s>>>(secs, items, nitems, A, B, C, views, pool, err, rpi);
   }
   TN_CUDA(cudaGetLastError());

@@ -476,11 +476,8 @@ void launch_tc_gemm_split(const TcSector* secs, const int4* items, int nitems, c
                           const unsigned long long* ea, const unsigned long long* eb, double* C, double* part,
                           int* err, int grid, cudaStream_t s) {
   constexpr size_t smem = (size_t)kARing * kATile + (size_t)kBRing * kDigits * kBTile + 1024;
-  static bool attr = false;
-  if (!attr) {
-    TN_CUDA(cudaFuncSetAttribute(tc_gemm_split, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    attr = true;
-  }
+  static PerDevice attr;
+  allow_smem(attr, tc_gemm_split, smem);
   tc_gemm_split<<<grid, kThreadsSplit, smem, s>>>(secs, items, nitems, ws, ea, eb, C, part, err);
   TN_CUDA(cudaGetLastError());
 }

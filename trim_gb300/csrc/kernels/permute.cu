@@ -610,11 +610,8 @@ template <typename T, typename Info>
 static void launch_permute_t(const PermSub* subs, const int64_t* tile_start, int nsub, int64_t ntiles, const T* src,
                              T* dst, uint64_t conj, int grid, cudaStream_t s) {
   const size_t smem = (size_t)kStages * kSmem * sizeof(double);
-  static bool attr = false;  // once per process and instantiation; the attribute is per function
-  if (!attr) {
-    TN_CUDA(cudaFuncSetAttribute(permute_kernel<T, Info>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    attr = true;
-  }
+  static PerDevice attr;  // per instantiation
+  allow_smem(attr, permute_kernel<T, Info>, smem);
   launch_pdl(permute_kernel<T, Info>, dim3(grid), dim3(kThreads), smem, s, subs, tile_start, nsub, ntiles, src, dst, conj);
 }
 

@@ -612,8 +612,9 @@ void launch_truncate(const int64_t* s_off, const int64_t* s_cnt, int nsec, int64
   const size_t all = smem + (size_t)total * sizeof(uint64_t) + ((size_t)nsec + 1) * sizeof(int);
   const bool staged = total > 0 && total < kSvdMaxSmem && all <= (size_t)kSvdMaxSmem;
   if (staged) smem = all;
-  if (smem > 48 * 1024)
-    TN_CUDA(cudaFuncSetAttribute(truncate_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  // the most any call takes, not this one's: another thread's call would lower it
+  static PerDevice attr;
+  allow_smem(attr, truncate_kernel, kSvdMaxSmem);
   truncate_kernel<<<1, 1024, smem, s>>>(s_off, s_cnt, nsec, S, chi, kept, norm, staged ? (int)total : 0);
   TN_CUDA(cudaGetLastError());
 }
