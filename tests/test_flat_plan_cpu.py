@@ -1,0 +1,45 @@
+"""The flat FP64 work list at sizes where it could grow or shrink too far, on
+the CPU: dot products over a long K are spread over the chip."""
+import os
+import subprocess
+
+import pytest
+
+from tests.test_cpp_driver import LIBDIR, ROOT, shutil
+
+SMS = 152
+
+
+@pytest.fixture(scope="module")
+def plan(tmp_path_factory):
+    if shutil.which("g++") is None or not os.path.exists(os.path.join(LIBDIR, "libtrim_gb300.so")):
+        pytest.skip("no g++ or library not built")
+    exe = str(tmp_path_factory.mktemp("flat") / "flat_plan_check")
+    cuda = os.environ.get("CUDA_HOME", "/usr/local/cuda")
+    p = subprocess.run(["g++", "-std=c++17", "-O1", "-I" + os.path.join(ROOT, "trim_gb300", "csrc"), "-I" + os.path.join(cuda, "include"),
+                        os.path.join(ROOT, "tests", "cpp", "flat_plan_check.cpp"), "-L" + LIBDIR, "-ltrim_gb300", "-L" + os.path.join(cuda, "lib64"),
+                        "-lcudart", "-Wl,-rpath," + LIBDIR, "-Wl,-rpath," + os.path.join(cuda, "lib64"), "-o", exe], capture_output=True, text=True)
+    assert p.returncode == 0, p.stderr
+
+    def run(*shapes):
+        out = subprocess.run([exe, str(SMS), *[str(v) for s in shapes for v in s]], capture_output=True, text=True).stdout.split()
+        assert out and out[0] == "ok", out
+        return [int(v) for v in out[1:]]
+
+    return run
+
+
+@pytest.mark.parametrize("shape", [(1, 1, 10 ** 6), (8, 1, 10 ** 5), (2, 2, 3 * 10 ** 5), (1, 2, 10 ** 8)])
+def test_rows_over_a_long_k(plan, shape):
+    """No warp takes more than two items' share: twice a 24th of a
+    sub-partition's (64 warp FMAs at least), or a 1024th of a row."""
+    m, n, k = shape
+    items, _, cost, ranges = plan(shape)
+    share = m * n * k / 32 / (4 * SMS)
+    assert cost <= max(2 * max(64, share / 24) + 5 * n, n * (k / 32 / 1024 + 2))
+    assert items >= min(256, m * n * k // 4096) and ranges <= 1024
+
+
+def test_every_product_once(plan):
+    plan(*[(m, n, k) for m in (1, 3, 33, 130) for n in (1, 2, 3, 32) for k in (1, 31, 32, 700, 40001)])
+    plan((5, 2, 99999), (1, 1, 12345678), (7, 18, 5000), (300, 300, 64))

@@ -221,9 +221,9 @@ struct FlatItem {
   int32_t v0, nv, kc;
   int32_t nsplit, o0, go, gs;
   int32_t grp, cnt;        // group (-1: one K range, written directly) and its number of items
-  int32_t rows;            // 1: entries are rows of a sector of N <= 2 columns, lanes along K
+  int32_t rows;            // 1: entries are rows of a sector of N <= 2 columns, lanes along K (range kq)
   int32_t a_vw, b_vw;      // operand views (ViewHdr index), -1: contiguous row-major
-  int32_t pad;
+  int32_t kq;
 };
 constexpr int kFlatWarps = 4, kFlatCtasPerSm = 5;  // warps per CTA, CTAs an SM holds (registers)
 constexpr int kFlatSlots = 4, kFlatViewSlots = 2;  // slots per item, and with a view

@@ -159,15 +159,24 @@ std::vector<GemmTile> plan_fp64(const std::vector<tn_sector_gemm>& list, int num
 // slot while an item is small: K ranges, with their partial sums, are the
 // second choice), each with its K ranges as a group; smaller ones deal all
 // their (K range, output) pairs to lanes, with the number of ranges raised
-// while more than 1 lane in 16 would stay empty.  An item that reads an operand
+// while more than 1 lane in 16 would stay empty.  One- and two-column sectors (a norm, an expectation value) take
+// rows, lanes along K, and K ranges of a row as soon as one costs two items;
+// with a whole row to a warp 1 x 1 over K = 1e6 took one warp 31 250 steps.  An item that reads an operand
 // through views walks its K range in the views' segments, so its entries share
 // one range.
+constexpr int64_t kRowRanges = 1024;  // K ranges of a row: two for every resident warp of half the chip
 std::vector<FlatItem> plan_fp64_flat(const std::vector<tn_sector_gemm>& list, int num_sms, int64_t* ws_elems,
                                      int64_t* ngroups, const std::vector<std::pair<int, int>>* vw) {
+  auto row_cost = [](int64_t n, int64_t k) { return n * ((k + 31) / 32 + 5); };  // warp FMAs, and 5 to sum the lanes
   double total = 0;
-  for (const auto& g : list)
-    if (g.M > 0 && g.N > 0 && g.K > 0) total += std::ceil((double)g.M * g.N / 32.0) * (double)g.K;
-  const int64_t target = (int64_t)std::min(4096.0, std::max(64.0, total / (4.0 * num_sms * 24.0)));
+  for (size_t gi = 0; gi < list.size(); gi++) {
+    const auto& g = list[gi];
+    if (g.M <= 0 || g.N <= 0 || g.K <= 0) continue;
+    const bool rows = g.N <= 2 && g.K >= 32 && !(vw && ((*vw)[gi].first >= 0 || (*vw)[gi].second >= 0));
+    total += rows ? (double)g.M * (double)row_cost(g.N, g.K) : std::ceil((double)g.M * g.N / 32.0) * (double)g.K;
+  }
+  const double share = total / (4.0 * num_sms);
+  const int64_t target = (int64_t)std::min(4096.0, std::max(64.0, share / 24.0));
   std::vector<FlatItem> out;
   int64_t ws = 0, ngrp = 0;
   const int64_t most_plain = std::max<int64_t>(1, std::min<int64_t>(kFlatSlots, target / 256));  // slots per chunk
@@ -189,11 +198,24 @@ std::vector<FlatItem> plan_fp64_flat(const std::vector<tn_sector_gemm>& list, in
     if (g.N <= 2 && g.K >= 32 && !viewed) {  // lanes along K
       t.rows = 1;
       t.mn = (int32_t)g.M;
-      const int64_t per = std::max<int64_t>(1, std::min<int64_t>(64, target / (g.N * ((g.K + 31) / 32 + 5))));
+      const int64_t row = row_cost(g.N, g.K);
+      const int64_t per = std::max<int64_t>(1, std::min<int64_t>(64, target / row));
+      // a row of more than two items' cost: K ranges, a multiple of the 32 lanes each
+      const int64_t ns = row > 2 * target ? std::min<int64_t>((row + target - 1) / target, kRowRanges) : 1;
+      t.kc = (int32_t)(ns > 1 ? (((g.K + ns - 1) / ns + 31) / 32) * 32 : g.K);
+      t.nsplit = (int32_t)((g.K + t.kc - 1) / t.kc);
       for (int64_t m0 = 0; m0 < g.M; m0 += per) {
         t.v0 = (int32_t)m0;
         t.nv = (int32_t)std::min(per, g.M - m0);
-        out.push_back(t);
+        if (t.nsplit > 1) {
+          t.grp = (int32_t)ngrp++;
+          t.cnt = t.nsplit;
+          t.o0 = (int32_t)(m0 * g.N);
+          t.go = t.gs = (int32_t)(t.nv * g.N);
+          t.ws_off = ws;
+          ws += (int64_t)t.nsplit * t.go;
+        }
+        for (t.kq = 0; t.kq < t.nsplit; t.kq++) out.push_back(t);
       }
       continue;
     }
@@ -254,8 +276,8 @@ std::vector<FlatItem> plan_fp64_flat(const std::vector<tn_sector_gemm>& list, in
   // for the tiles above
   const int64_t grid_items = (int64_t)num_sms * kFlatCtasPerSm * kFlatWarps;
   if ((int64_t)out.size() <= grid_items) return out;
-  auto cost = [](const FlatItem& t) {
-    return t.rows ? (int64_t)t.nv * t.N * ((t.K + 31) / 32 + 5) : (int64_t)((t.nv + 31) / 32) * std::min(t.kc, t.K);
+  auto cost = [&](const FlatItem& t) {
+    return t.rows ? t.nv * row_cost(t.N, std::min(t.kc, t.K)) : (int64_t)((t.nv + 31) / 32) * std::min(t.kc, t.K);
   };
   std::stable_sort(out.begin(), out.end(), [&](const FlatItem& a, const FlatItem& b) { return cost(a) > cost(b); });
   const size_t band = (size_t)grid_items;

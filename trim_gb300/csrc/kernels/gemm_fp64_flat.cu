@@ -23,11 +23,13 @@
 // -> 1.12 TFLOP/s, of 1.26), 64 of its contractions 0.81 -> 0.38 ms, an iPEPS
 // quadrant at chi = 64, D = 6 (sectors of 1152 x 36 .. 648 x 648 outputs) 3.19 ->
 // 3.03 ms, the captured iTEBD network at chi = 512 (operands through views)
-// 42.4 -> 33.7 us.
+// 42.4 -> 33.7 us; one output over K = 1e6 533 -> 23 us, 8 x 1 over 1e5 89 -> 21, 2 x 2
+// over 3e5 248 -> 19, 10 x 10 over 1e6 1169 -> 393.
 //
 // Items that share outputs (K ranges) write partial sums to a workspace; the
-// last one of a group adds them in range order, so the result does not depend
-// on the schedule.  Launched with programmatic dependent launch (pdl.cuh): the
+// last one of a group adds them in a fixed order, so the result does not depend
+// on the schedule: a lane per output in range order, or the lanes along the
+// ranges where outputs are few (a dot product over K = 1e6, 488 ranges).  Launched with programmatic dependent launch (pdl.cuh): the
 // first item and the view tables (plan data) are read before the wait on the
 // previous grid.
 #include "../engine/engine.h"
@@ -197,8 +199,10 @@ __device__ __forceinline__ void flat_body(const FlatItem& t, int lane, const dou
 // sums added by a fixed shuffle butterfly; the item's entries are nv rows.
 template <int NN>
 __device__ __forceinline__ void row_body(const FlatItem& t, int lane, const double* __restrict__ A,
-                                         const double* __restrict__ B, double* __restrict__ C) {
+                                         const double* __restrict__ B, double* __restrict__ C,
+                                         double* __restrict__ ws) {
   const double* __restrict__ b = B + t.b_off;
+  const int k0 = t.kq * t.kc, k1 = min(t.K, k0 + t.kc);
   pdl_wait();
   for (int m = t.v0; m < t.v0 + t.nv; m++) {
     const double* __restrict__ a = A + t.a_off + (int64_t)m * t.K;
@@ -206,7 +210,7 @@ __device__ __forceinline__ void row_body(const FlatItem& t, int lane, const doub
 #pragma unroll
     for (int n = 0; n < NN; n++) acc[n] = 0.0;
 #pragma unroll 4
-    for (int k = lane; k < t.K; k += 32) {
+    for (int k = k0 + lane; k < k1; k += 32) {
       const double av = __ldg(a + k);
 #pragma unroll
       for (int n = 0; n < NN; n++) acc[n] = fma(av, __ldg(b + (int64_t)k * NN + n), acc[n]);
@@ -215,7 +219,12 @@ __device__ __forceinline__ void row_body(const FlatItem& t, int lane, const doub
     for (int n = 0; n < NN; n++) {
 #pragma unroll
       for (int o = 16; o > 0; o >>= 1) acc[n] += __shfl_xor_sync(0xffffffffu, acc[n], o);
-      if (lane == n) C[t.c_off + (int64_t)m * NN + n] = acc[n];
+      if (lane == n) {
+        if (t.grp < 0)
+          C[t.c_off + (int64_t)m * NN + n] = acc[n];
+        else
+          ws[t.ws_off + (int64_t)t.kq * t.gs + (m * NN + n - t.o0)] = acc[n];
+      }
     }
   }
 }
@@ -258,12 +267,10 @@ __global__ void __launch_bounds__(32 * kWarps, kFlatCtasPerSm)
     const FlatItem t = items[it];
     if (t.rows) {
       if (t.N == 1)
-        row_body<1>(t, lane, A, B, C);
+        row_body<1>(t, lane, A, B, C, ws);
       else
-        row_body<2>(t, lane, A, B, C);
-      continue;
-    }
-    if (VIEWS && (t.a_vw >= 0 || t.b_vw >= 0))
+        row_body<2>(t, lane, A, B, C, ws);
+    } else if (VIEWS && (t.a_vw >= 0 || t.b_vw >= 0))
       view_dispatch(t, lane, A, B, C, ws, views, pool);
     else if (t.v0 / t.mn == (t.v0 + t.nv - 1) / t.mn)
       flat_dispatch<true>(t, lane, A, B, C, ws);
@@ -277,10 +284,22 @@ __global__ void __launch_bounds__(32 * kWarps, kFlatCtasPerSm)
       if (__shfl_sync(0xffffffffu, last, 0)) {
         __threadfence();
         const double* p = ws + t.ws_off;
-        for (int o = lane; o < t.go; o += 32) {
-          double s = 0.0;
-          for (int q = 0; q < t.nsplit; q++) s += __ldcg(p + (int64_t)q * t.gs + o);
-          C[t.c_off + t.o0 + o] = s;
+        if (t.go >= 32 || t.nsplit <= 16) {
+          for (int o = lane; o < t.go; o += 32) {
+            double s = 0.0;
+#pragma unroll 8
+            for (int q = 0; q < t.nsplit; q++) s += __ldcg(p + (int64_t)q * t.gs + o);
+            C[t.c_off + t.o0 + o] = s;
+          }
+        } else {  // few outputs of many ranges: lanes along the ranges
+          for (int o = 0; o < t.go; o++) {
+            double s = 0.0;
+#pragma unroll 8
+            for (int q = lane; q < t.nsplit; q += 32) s += __ldcg(p + (int64_t)q * t.gs + o);
+#pragma unroll
+            for (int d = 16; d > 0; d >>= 1) s += __shfl_xor_sync(0xffffffffu, s, d);
+            if (lane == 0) C[t.c_off + t.o0 + o] = s;
+          }
         }
         if (lane == 0) counters[t.grp] = 0;  // for the next launch
       }
