@@ -1,5 +1,5 @@
 """The flat FP64 work list at sizes where it could grow or shrink too far, on
-the CPU: dot products over a long K are spread over the chip."""
+the CPU: dot products and few outputs over a long K are spread over the chip."""
 import os
 import subprocess
 
@@ -38,6 +38,13 @@ def test_rows_over_a_long_k(plan, shape):
     share = m * n * k / 32 / (4 * SMS)
     assert cost <= max(2 * max(64, share / 24) + 5 * n, n * (k / 32 / 1024 + 2))
     assert items >= min(256, m * n * k // 4096) and ranges <= 1024
+
+
+@pytest.mark.parametrize("shape", [(10, 10, 10 ** 6), (3, 4, 10 ** 6), (11, 11, 10 ** 8), (64, 1, 31)])
+def test_few_outputs(plan, shape):
+    _, ws, _, ranges = plan(shape)
+    most = max(256, 8192 // (shape[0] * shape[1]))
+    assert ranges <= most and ws <= most * shape[0] * shape[1]
 
 
 def test_every_product_once(plan):

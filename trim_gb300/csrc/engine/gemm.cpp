@@ -159,7 +159,8 @@ std::vector<GemmTile> plan_fp64(const std::vector<tn_sector_gemm>& list, int num
 // slot while an item is small: K ranges, with their partial sums, are the
 // second choice), each with its K ranges as a group; smaller ones deal all
 // their (K range, output) pairs to lanes, with the number of ranges raised
-// while more than 1 lane in 16 would stay empty.  One- and two-column sectors (a norm, an expectation value) take
+// while more than 1 lane in 16 would stay empty; 256 at most, or
+// 8192 partial sums (one warp adds them up).  One- and two-column sectors (a norm, an expectation value) take
 // rows, lanes along K, and K ranges of a row as soon as one costs two items;
 // with a whole row to a warp 1 x 1 over K = 1e6 took one warp 31 250 steps.  An item that reads an operand
 // through views walks its K range in the views' segments, so its entries share
@@ -247,7 +248,7 @@ std::vector<FlatItem> plan_fp64_flat(const std::vector<tn_sector_gemm>& list, in
       }
     } else {
       const int64_t kc0 = std::max<int64_t>(32, target);
-      int64_t ns = std::max<int64_t>(1, (g.K + kc0 - 1) / kc0);
+      int64_t ns = std::max<int64_t>(1, std::min((g.K + kc0 - 1) / kc0, std::max<int64_t>(256, 8192 / mn)));
       auto waste = [&](int64_t n) { return (double)((mn * n + 31) / 32 * 32) / (double)(mn * n); };
       while (waste(ns) > 1.0625 && ns < 32 && g.K / (ns + 1) >= 32) ns++;
       t.kc = (int32_t)((g.K + ns - 1) / ns);
