@@ -1,5 +1,7 @@
 """The flat FP64 work list at sizes where it could grow or shrink too far, on
-the CPU: dot products and few outputs over a long K are spread over the chip."""
+the CPU: dot products and few outputs over a long K are spread over the chip,
+and large outputs over a long K are not cut into more items and partial sums
+than the chip has use for."""
 import os
 import subprocess
 
@@ -45,6 +47,16 @@ def test_few_outputs(plan, shape):
     _, ws, _, ranges = plan(shape)
     most = max(256, 8192 // (shape[0] * shape[1]))
     assert ranges <= most and ws <= most * shape[0] * shape[1]
+
+
+@pytest.mark.parametrize("shapes", [[(2800, 2800, 10 ** 5)], [(2800, 2800, 10 ** 8)], [(400, 400, 10 ** 6)] * 20, [(130, 1, 10 ** 7), (1000, 1000, 50000)]])
+def test_large_outputs_over_a_long_k(plan, shapes):
+    """Items: 96 a sub-partition and twice that for rounding, and the chunks of
+    128 outputs; partial sums: 128 to an item of a split chunk."""
+    items, ws, _, _ = plan(*shapes)
+    chunks = sum(m * n // 128 + 1 for m, n, _ in shapes)
+    assert items <= 2 * 96 * 4 * SMS + 2 * chunks
+    assert ws <= 128 * 2 * 96 * 4 * SMS
 
 
 def test_every_product_once(plan):

@@ -151,7 +151,9 @@ std::vector<GemmTile> plan_fp64(const std::vector<tn_sector_gemm>& list, int num
 
 // Flat items.  Cost is counted in warp FMAs (slots x K): an SM sub-partition
 // runs one at a time, so items are cut to about a 24th of its share (at
-// least 64 warp FMAs, below which an item's own latency shows; at most 4096).
+// least 64 warp FMAs, below which an item's own latency shows; at most 4096, or
+// a 96th of the share where that is more: a list of 4e10 multiply-adds and up
+// would only grow, items and partial sums by the gigabyte).
 // (Sixteenths were up to 7% slower, on 64 uneven contractions 414 -> 386 us, an
 // iPEPS quadrant at chi = 48, D = 5 460 -> 448; 48ths up to 6% faster still on some
 // lists and 2% slower on others.)
@@ -177,7 +179,7 @@ std::vector<FlatItem> plan_fp64_flat(const std::vector<tn_sector_gemm>& list, in
     total += rows ? (double)g.M * (double)row_cost(g.N, g.K) : std::ceil((double)g.M * g.N / 32.0) * (double)g.K;
   }
   const double share = total / (4.0 * num_sms);
-  const int64_t target = (int64_t)std::min(4096.0, std::max(64.0, share / 24.0));
+  const int64_t target = (int64_t)std::min(std::max(4096.0, share / 96.0), std::max(64.0, share / 24.0));
   std::vector<FlatItem> out;
   int64_t ws = 0, ngrp = 0;
   const int64_t most_plain = std::max<int64_t>(1, std::min<int64_t>(kFlatSlots, target / 256));  // slots per chunk
