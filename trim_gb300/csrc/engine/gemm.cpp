@@ -152,7 +152,7 @@ std::vector<GemmTile> plan_fp64(const std::vector<tn_sector_gemm>& list, int num
 // Flat items.  Cost is counted in warp FMAs (slots x K): an SM sub-partition
 // runs one at a time, so items are cut to about a 24th of its share (at
 // least 64 warp FMAs, below which an item's own latency shows; at most 4096, or
-// a 96th of the share where that is more: a list of 4e10 multiply-adds and up
+// a 96th of the share where that is more: a list of 8e9 multiply-adds and up
 // would only grow, items and partial sums by the gigabyte).
 // (Sixteenths were up to 7% slower, on 64 uneven contractions 414 -> 386 us, an
 // iPEPS quadrant at chi = 48, D = 5 460 -> 448; 48ths up to 6% faster still on some
