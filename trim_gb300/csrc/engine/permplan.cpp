@@ -74,23 +74,26 @@ void choose_tile(PermSub& ps, int es) {
       const int64_t tx = std::min(kTile / ps.dims[y], kStage / ps.dims[y] - 1) & ~(int64_t)3;
       ps.tx = (int32_t)std::min<int64_t>(ps.dims[x], tx);
       ps.ty = (int32_t)ps.dims[y];
-    }
-    // Narrower rows where that takes clearly fewer tiles: 96 x 96 as three tiles
-    // of 32 x 96, not 64 + 32 in both directions.  Transposes of 80^4, 96^4 and
-    // 100^4: 250, 360 and 489 us -> 155, 289 and 362 at most.  (16-byte elements
-    // keep their 64 x 32 tiles: 100 x 100 x 8 x 100 ran up to 10% slower in 52 x 34.)
-    auto tiles = [&](int64_t tx, int64_t ty) {
-      return ((ps.dims[x] + tx - 1) / tx) * ((ps.dims[y] + ty - 1) / ty);
-    };
-    int64_t best = tiles(ps.tx, ps.ty) * 7 / 8;
-    for (int64_t nx = (ps.dims[x] + kRow - 1) / kRow; es == 1 && ps.dims[x] / nx >= 32; nx++) {
-      const int64_t tx = std::min<int64_t>(kRow, ((ps.dims[x] + nx - 1) / nx + 3) & ~(int64_t)3);
-      const int64_t cap = std::min<int64_t>({kTile / tx, kStage / (tx + 1), 1024});
-      const int64_t ny = (ps.dims[y] + cap - 1) / cap, ty1 = (ps.dims[y] + ny - 1) / ny;
-      if (tiles(tx, ty1) <= best) {
-        best = tiles(tx, ty1) - 1;
-        ps.tx = (int32_t)tx;
-        ps.ty = (int32_t)ty1;
+    } else if (es == 1) {
+      // Narrower rows where that takes clearly fewer tiles: 96 x 96 as three tiles
+      // of 32 x 96, not 64 + 32 in both directions.  Transposes of 80^4, 96^4 and
+      // 100^4: 250, 360 and 489 us -> 155, 289 and 362 at most.  (16-byte elements
+      // keep their 64 x 32 tiles: 100 x 100 x 8 x 100 ran up to 10% slower in 52 x 34.)
+      // The widths that an even split of x comes to are few: 64, 60, .., 32.
+      auto tiles = [&](int64_t tx, int64_t ty) {
+        return ((ps.dims[x] + tx - 1) / tx) * ((ps.dims[y] + ty - 1) / ty);
+      };
+      int64_t best = tiles(ps.tx, ps.ty) * 7 / 8;
+      for (int64_t tx = kRow; tx >= kRow / 2; tx -= 4) {
+        const int64_t nx = (ps.dims[x] + tx - 1) / tx;
+        if (ps.dims[x] / nx < kRow / 2 || (((ps.dims[x] + nx - 1) / nx + 3) & ~(int64_t)3) != tx) continue;
+        const int64_t cap = std::min<int64_t>({kTile / tx, kStage / (tx + 1), 1024});
+        const int64_t ny = (ps.dims[y] + cap - 1) / cap, ty1 = (ps.dims[y] + ny - 1) / ny;
+        if (tiles(tx, ty1) <= best) {
+          best = tiles(tx, ty1) - 1;
+          ps.tx = (int32_t)tx;
+          ps.ty = (int32_t)ty1;
+        }
       }
     }
   } else {
