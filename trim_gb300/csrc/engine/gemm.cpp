@@ -650,8 +650,11 @@ bool sectors_take_views(const Ctx& ctx, int mode, const std::vector<tn_sector_ge
   return r == GemmRoute::Fp64 || r == GemmRoute::Fused;
 }
 
-// The views of one contraction's two operands as one device table.
+// The views of one contraction's two operands as one device table.  It holds
+// on to both: the table is found by their addresses, which the view cache would
+// otherwise give to other views once it starts over.
 struct ViewTable {
+  OpViewsP va, vb;
   DevBufP hdrs, pool;
   int na = 0;  // headers of the A operand come first
 };
@@ -669,6 +672,8 @@ static std::shared_ptr<ViewTable> get_view_table(Ctx& ctx, const OpViewsP& va, c
     }
   }
   auto T = std::make_shared<ViewTable>();
+  T->va = va;
+  T->vb = vb;
   std::vector<ViewHdr> hdrs;
   std::vector<int64_t> pool;
   if (va) {
@@ -694,7 +699,7 @@ static std::shared_ptr<ViewTable> get_view_table(Ctx& ctx, const OpViewsP& va, c
                           ctx.stream));
   TN_CUDA(cudaStreamSynchronize(ctx.stream));  // the host copies die here
   std::lock_guard<std::mutex> lk(ctx.mu);
-  ctx.gemm_cache[hk] = T;  // the OpViews behind the two keys are cached for good
+  ctx.gemm_cache[hk] = T;
   ctx.keep_alive(T);
   return T;
 }
