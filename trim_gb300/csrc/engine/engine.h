@@ -168,14 +168,14 @@ struct PermSub {
   int32_t ydim;   // index of the source-contiguous dim used as tile y (-1: none)
   int32_t tx, ty; // tile extents along x (= dims[ndim-1]) and y
   int32_t ntx, nty;
-  int32_t zdim;   // mode 2: a third dim stacked into the tile (-1: none)
+  int32_t zdim;   // modes 2 and 3: a third dim stacked into the tile (-1: none)
   int32_t tz, ntz;
-  int32_t wdim;       // mode 3: a fourth dim whose tw values repeat the tile (-1: none)
+  int32_t wdim;       // modes 2 and 3: a fourth dim whose tw values repeat the tile (-1: none)
   int32_t tw, ntw;
   int64_t nouter;     // product of the dims other than x, y, z and w
   int64_t tile_begin; // first tile index of this sub-block
   double sign;        // +1 (bosonic); a fermionic sign would go here
-  int32_t mode;       // 0: lanes along x; 1: shared-memory transpose (x, y); 2: the same over tz planes (x, y, z);
+  int32_t mode;       // 0: lanes along x; 1: shared-memory transpose (x, y); 2: the same over tz planes (x, y, z, w);
                       // 3: short rows stacked (x, y, z, w)
 };
 struct PermPlan {
@@ -188,7 +188,7 @@ struct PermPlan {
   int64_t elem_num = 0;
   int esz = 8;        // element size in bytes: 8 (real) or 16 (complex pairs)
   bool conj = false;  // 16-byte elements: conjugate on the way (cTranspose)
-  bool short_rows = false;  // some sub-block has tiles with a fourth dim
+  bool fourth_dim = false;  // some sub-block has tiles with a fourth dim
 };
 using PermPlanP = std::shared_ptr<PermPlan>;
 
@@ -481,9 +481,9 @@ std::vector<FlatItem> plan_fp64_flat(const std::vector<tn_sector_gemm>& list, in
                                      int64_t* ngroups, const std::vector<std::pair<int, int>>* vw = nullptr);
 
 // kernel launchers (defined in the .cu files)
-// short_rows: some tile has a fourth dim
+// fourth_dim: some tile has a fourth dim
 void launch_permute_kernel(const PermSub* subs, const int64_t* tile_start, int nsub, int64_t ntiles, int esz,
-                           bool conj, bool short_rows, const void* src, void* dst, int grid, cudaStream_t s);
+                           bool conj, bool fourth_dim, const void* src, void* dst, int grid, cudaStream_t s);
 // counters (one int per split group, zero between launches) may be null: then
 // split tiles need launch_splitk_reduce afterwards; otherwise the last CTA of
 // each split group sums its partial tiles in split order and resets the counter.

@@ -510,14 +510,10 @@ static void run_fp64(Ctx& ctx, const std::vector<tn_sector_gemm>& list, const do
 void run_tc_gemms(Ctx& ctx, int ns, const std::vector<tn_sector_gemm>& list, const double* A, const double* B,
                   double* C);
 
-// Tensor-core modes route work where the tensor-core path cannot pay for its
-// fixed cost (operand slicing + a second launch, ~70 us measured on GB300) --
-// a whole contraction under 5e7 FLOP, or a sector with K < 16 or under 16K
-// multiply-adds -- and sectors the 128 x 64 tensor tiles would pad four-fold
-// or more (M < 32 or N < 16) to the FP64 kernel, which is exact and for those
-// shapes no slower; the rest goes to the tcgen05 kernel.
-// the tensor-core modes' routing rule (see run_sector_gemms): true for a
-// sector the FP64 kernel takes
+// The forms of a tensor-core mode (static_route): a list of thin sectors alone
+// goes to the FP64 kernel; a short list of short K to the fused kernel, or to the
+// FP64 kernel or the tiled form where one of them was faster when first run; every
+// other list is tiled, its thin sectors on the FP64 kernel.
 void run_tc_fused(Ctx& ctx, int ns, const std::vector<tn_sector_gemm>& list, const double* A, const double* B,
                   double* C, const std::vector<std::pair<int, int>>* vw = nullptr, const ViewHdr* views = nullptr,
                   const int64_t* pool = nullptr, const void* table = nullptr);

@@ -1,7 +1,10 @@
-// Planning and dispatch of the tensor-core sector GEMMs (split precision and
-// fast BF16).  Per contraction: the maxima of A's rows and B's columns, the
-// operand slice images (tcgen05 shared-memory layout), then one persistent
-// grouped GEMM launch over all (sector, 128-row tile, 64-column tile) items.
+// Planning and dispatch of the tensor-core sector GEMMs (split precision, fast
+// BF16 and TF32).  Per contraction of the tiled form: the maxima of A's rows and
+// B's columns and the operands' images (tcgen05 shared-memory layout), in one
+// launch or, where its longest item would last longer, in two; one persistent
+// grouped GEMM launch over all (sector, 128-row tile, one to four 64-column tiles,
+// K range) items; and the sum over K ranges where there are any.  The fused form
+// is one launch.
 // Device work lists are built once per sector list and cached on the context,
 // so a repeated contraction (and a captured CUDA graph) uploads nothing.
 #include <algorithm>

@@ -553,7 +553,7 @@ PermPlanP host_plan(std::vector<PermSub> subs, int64_t elem_num, int esz) {
   plan->nsub = (int)subs.size();
   plan->ntiles = tiles;
   plan->elem_num = elem_num;
-  for (const auto& ps : subs) plan->short_rows |= ps.wdim >= 0;
+  for (const auto& ps : subs) plan->fourth_dim |= ps.wdim >= 0;
   plan->host_subs = std::move(subs);
   return plan;
 }
@@ -626,7 +626,7 @@ void run_permute(Ctx& ctx, const PermPlan& plan, const void* src, void* dst) {
   int64_t grid = std::min<int64_t>(plan.ntiles, (int64_t)ctx.num_sms * 2);
   ProfScope ps(ctx, "permute", 2.0 * plan.esz * plan.elem_num, 0);
   launch_permute_kernel((const PermSub*)plan.subs->ptr, (const int64_t*)plan.tile_start->ptr, plan.nsub, plan.ntiles,
-                        plan.esz, plan.conj, plan.short_rows, src, dst, (int)grid, ctx.stream);
+                        plan.esz, plan.conj, plan.fourth_dim, src, dst, (int)grid, ctx.stream);
   ctx.launched();
 }
 

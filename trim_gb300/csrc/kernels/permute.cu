@@ -5,11 +5,12 @@
 // 2-D piece (x, y) of one canonical sub-block copy (see PermSub): x is the
 // destination-contiguous dim, so stores are coalesced; in mode 1 y is the
 // source-contiguous dim and the tile is transposed through shared memory so
-// loads are coalesced too; mode 2 stacks tz planes of a third dim z into a
-// small transpose tile; mode 3 stacks short rows (x contiguous on both sides
-// but only a few elements long) into a dense [w][z][y][x] tile that is loaded in
-// source-stride order and stored in destination-stride order, w a fourth dim
-// stepped with a constant stride.  Remaining dims are decoded once per tile.
+// loads are coalesced too; mode 2 stacks tz planes of a third dim z, and tw
+// values of a fourth dim w, into a small transpose tile; mode 3 stacks short
+// rows (x contiguous on both sides but only a few elements long) into a dense
+// [w][z][y][x] tile that is loaded in source-stride order and stored in
+// destination-stride order, w stepped with a constant stride.  Remaining dims are
+// decoded once per tile.
 //
 // Elements are 8 bytes (real FP64) or 16 bytes (complex FP64 as (re, im)
 // pairs, the cflag twins UniTensorComplex.cpp:447-825): the kernel is the same
@@ -30,17 +31,17 @@ constexpr int kPerThread = 16;  // tile <= 4096 elements: 16 loads in flight per
 constexpr int kSmem = 64 * 65;  // >= ty * (tx + 1) of every transpose tile (checked on the host)
 
 struct TileInfo {
-  static constexpr bool kShortRows = false;
+  static constexpr bool kFourthDim = false;
   int64_t bs, bd;     // base offsets of the tile origin
   int64_t sx, sy, sz, dx, dy, dz;
   int32_t nx, ny, nz; // valid extents of this tile
   int32_t tx, ty, tz; // full tile extents
   int32_t mode, neg;
 };
-// with the fourth tile dim of mode 3; plans that have none run a kernel without
-// it (the longer decode records cost the large transposes 1%)
+// with the fourth tile dim of modes 2 and 3; plans that have none run a kernel
+// without it (the longer decode records cost the large transposes 1%)
 struct TileInfoW : TileInfo {
-  static constexpr bool kShortRows = true;
+  static constexpr bool kFourthDim = true;
   int64_t sw, dw;
   int32_t nw, tw;
 };
@@ -68,13 +69,13 @@ __host__ __device__ inline Info decode_tile(const PermSub& P, int64_t local) {
   if (n == 0) {
     w.nx = w.ny = w.nz = w.tx = w.ty = w.tz = 1;
     w.sx = w.sy = w.sz = w.dx = w.dy = w.dz = 0;
-    if constexpr (Info::kShortRows) {
+    if constexpr (Info::kFourthDim) {
       w.nw = w.tw = 1;
       w.sw = w.dw = 0;
     }
     w.mode = 0;
   } else {
-    const int x = n - 1, y = P.ydim, z = P.zdim, v = Info::kShortRows ? P.wdim : -1;
+    const int x = n - 1, y = P.ydim, z = P.zdim, v = Info::kFourthDim ? P.wdim : -1;
     int64_t xt, yt, zt, wt = 0;
     if (local < 0x7fffffffLL) {  // 32-bit division is several times cheaper
       uint32_t l = (uint32_t)local;
@@ -126,7 +127,7 @@ __host__ __device__ inline Info decode_tile(const PermSub& P, int64_t local) {
       w.sz = w.dz = 0;
       w.tz = w.nz = 1;
     }
-    if constexpr (Info::kShortRows) {
+    if constexpr (Info::kFourthDim) {
       if (v >= 0) {
         const int64_t w0 = wt * P.tw;
         bs += w0 * P.sstride[v];
@@ -257,7 +258,7 @@ __device__ __forceinline__ void issue_tile(const Info& w, const T* __restrict__ 
         if (xx >= w.nx || yy >= w.ny) continue;
         const T* g = src + w.bs + (int64_t)yy * w.sy + (int64_t)xx * w.sx;
         T* sp = buf + yy * pitch + xx;
-        if constexpr (Info::kShortRows) {
+        if constexpr (Info::kFourthDim) {
           const T* gw = g;
           for (int ww = 0; ww < w.nw; ww++, gw += w.sw) {
             sp = buf + yy * pitch + xx + ww * w.tz * plane;
@@ -277,7 +278,7 @@ __device__ __forceinline__ void issue_tile(const Info& w, const T* __restrict__ 
       walk3(a, b, c, [&](int m, int64_t g) {
         const T* p = s0 + g;
         T* sp = buf + m;
-        if constexpr (Info::kShortRows)
+        if constexpr (Info::kFourthDim)
           for (int ww = 0; ww < w.nw; ww++, p += w.sw, sp += w.tx * w.ty * w.tz) cp_async_el(sp, p);
         else
           cp_async_el(sp, p);
@@ -348,7 +349,7 @@ __device__ __forceinline__ void store_tile(const Info& w, const T* buf, T* __res
       if (xx >= w.nx || yy >= w.ny) continue;
       const T* sp = buf + yy * pitch + xx;
       T* g = dst + w.bd + (int64_t)yy * w.dy + (int64_t)xx * w.dx;
-      if constexpr (Info::kShortRows) {
+      if constexpr (Info::kFourthDim) {
         T* gw = g;
         for (int ww = 0; ww < w.nw; ww++, gw += w.dw) {
           sp = buf + yy * pitch + xx + ww * w.tz * plane;
@@ -368,7 +369,7 @@ __device__ __forceinline__ void store_tile(const Info& w, const T* buf, T* __res
     walk3(a, b, c, [&](int m, int64_t g) {
       T* p = d0 + g;
       const T* sp = buf + m;
-      if constexpr (Info::kShortRows)
+      if constexpr (Info::kFourthDim)
         for (int ww = 0; ww < w.nw; ww++, p += w.dw, sp += w.tx * w.ty * w.tz) *p = apply_flip(*sp, f);
       else
         *p = apply_flip(*sp, f);
@@ -616,13 +617,13 @@ static void launch_permute_t(const PermSub* subs, const int64_t* tile_start, int
 }
 
 void launch_permute_kernel(const PermSub* subs, const int64_t* tile_start, int nsub, int64_t ntiles, int esz,
-                           bool conj, bool short_rows, const void* src, void* dst, int grid, cudaStream_t s) {
+                           bool conj, bool fourth_dim, const void* src, void* dst, int grid, cudaStream_t s) {
   const uint64_t c = conj ? 0x8000000000000000ull : 0ull;
   if (esz == 8) {
-    auto f = short_rows ? launch_permute_t<double, TileInfoW> : launch_permute_t<double, TileInfo>;
+    auto f = fourth_dim ? launch_permute_t<double, TileInfoW> : launch_permute_t<double, TileInfo>;
     f(subs, tile_start, nsub, ntiles, (const double*)src, (double*)dst, 0, grid, s);
   } else if (esz == 16) {
-    auto f = short_rows ? launch_permute_t<double2, TileInfoW> : launch_permute_t<double2, TileInfo>;
+    auto f = fourth_dim ? launch_permute_t<double2, TileInfoW> : launch_permute_t<double2, TileInfo>;
     f(subs, tile_start, nsub, ntiles, (const double2*)src, (double2*)dst, c, grid, s);
   } else
     fail(TN_ERR_ARG, "permute: element size must be 8 or 16 bytes");
