@@ -301,6 +301,7 @@ static bool flat_fits(const std::vector<tn_sector_gemm>& list) {
 struct Fp64Plan {
   DevBufP flat;  // FlatItem list (then no tiles)
   int nflat = 0;
+  bool long_k = false;
   std::vector<tn_sector_gemm> list;
   std::vector<std::pair<int, int>> vw;  // operand view ids per sector (empty: contiguous operands)
   const void* table = nullptr;          // the view table the ids index
@@ -348,6 +349,7 @@ static std::shared_ptr<Fp64Plan> get_fp64_plan(Ctx& ctx, const std::vector<tn_se
   if (flat) {
     items = plan_fp64_flat(list, ctx.num_sms, &P->ws_elems, &ngrp, vw);
     P->nflat = (int)items.size();
+    for (const auto& t : items) P->long_k |= t.nsplit > kFlatFewRanges || (t.rows && t.nsplit > 1);
   } else {
     tiles = plan_fp64_split(list, ctx.num_sms, true, &P->ws_elems, pol, vw);
     for (const auto& t : tiles) ngrp = std::max<int64_t>(ngrp, (int64_t)t.grp + 1);
@@ -390,7 +392,7 @@ static void launch_fp64_plan(Ctx& ctx, const Fp64Plan& P, const double* A, const
     grid = (int)std::min<int64_t>(((int64_t)P.nflat + kFlatWarps - 1) / kFlatWarps,
                                   (int64_t)ctx.num_sms * kFlatCtasPerSm);
     launch_gemm_fp64_flat((const FlatItem*)P.flat->ptr, P.nflat, A, B, C, ws,
-                          P.counters ? (int*)P.counters->ptr : nullptr, views, pool, grid, ctx.stream);
+                          P.counters ? (int*)P.counters->ptr : nullptr, views, pool, P.long_k, grid, ctx.stream);
     ctx.launched();
   } else {
     // split tiles are summed by the last CTA of each group (no second launch)

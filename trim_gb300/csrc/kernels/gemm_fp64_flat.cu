@@ -197,12 +197,12 @@ __device__ __forceinline__ void flat_body(const FlatItem& t, int lane, const dou
 // Sectors of one or two columns: lanes along K (A's row and B's rows read
 // coalesced; flat lanes would gather 16 or 32 rows of A per load), the lanes'
 // sums added by a fixed shuffle butterfly; the item's entries are nv rows.
-template <int NN>
+template <int NN, bool LONG>
 __device__ __forceinline__ void row_body(const FlatItem& t, int lane, const double* __restrict__ A,
                                          const double* __restrict__ B, double* __restrict__ C,
                                          double* __restrict__ ws) {
   const double* __restrict__ b = B + t.b_off;
-  const int k0 = t.kq * t.kc, k1 = min(t.K, k0 + t.kc);
+  const int k0 = LONG ? t.kq * t.kc : 0, k1 = LONG ? min(t.K, k0 + t.kc) : t.K;
   pdl_wait();
   for (int m = t.v0; m < t.v0 + t.nv; m++) {
     const double* __restrict__ a = A + t.a_off + (int64_t)m * t.K;
@@ -220,7 +220,7 @@ __device__ __forceinline__ void row_body(const FlatItem& t, int lane, const doub
 #pragma unroll
       for (int o = 16; o > 0; o >>= 1) acc[n] += __shfl_xor_sync(0xffffffffu, acc[n], o);
       if (lane == n) {
-        if (t.grp < 0)
+        if (!LONG || t.grp < 0)
           C[t.c_off + (int64_t)m * NN + n] = acc[n];
         else
           ws[t.ws_off + (int64_t)t.kq * t.gs + (m * NN + n - t.o0)] = acc[n];
@@ -253,8 +253,10 @@ __device__ __forceinline__ void view_dispatch(const FlatItem& t, int lane, const
 
 // VIEWS: some item reads an operand through views (a kernel of its own: with
 // its registers the plain one would hold 4 CTAs per SM instead of 5, 20% slower
-// on the batched workload)
-template <bool VIEWS>
+// on the batched workload).  LONG: some row is cut into K ranges, or some group
+// has more than kFlatFewRanges (a kernel of its own too: in one, lists without
+// such a sector ran 1% longer, the batched workload 5.93 -> 6.01 ms)
+template <bool VIEWS, bool LONG>
 __global__ void __launch_bounds__(32 * kWarps, kFlatCtasPerSm)
     gemm_fp64_flat_kernel(const FlatItem* __restrict__ items, int nitems, const double* __restrict__ A,
                           const double* __restrict__ B, double* __restrict__ C, double* __restrict__ ws,
@@ -267,9 +269,10 @@ __global__ void __launch_bounds__(32 * kWarps, kFlatCtasPerSm)
     const FlatItem t = items[it];
     if (t.rows) {
       if (t.N == 1)
-        row_body<1>(t, lane, A, B, C, ws);
+        row_body<1, LONG>(t, lane, A, B, C, ws);
       else
-        row_body<2>(t, lane, A, B, C, ws);
+        row_body<2, LONG>(t, lane, A, B, C, ws);
+      if (!LONG || t.grp < 0) continue;
     } else if (VIEWS && (t.a_vw >= 0 || t.b_vw >= 0))
       view_dispatch(t, lane, A, B, C, ws, views, pool);
     else if (t.v0 / t.mn == (t.v0 + t.nv - 1) / t.mn)
@@ -284,10 +287,10 @@ __global__ void __launch_bounds__(32 * kWarps, kFlatCtasPerSm)
       if (__shfl_sync(0xffffffffu, last, 0)) {
         __threadfence();
         const double* p = ws + t.ws_off;
-        if (t.go >= 32 || t.nsplit <= 16) {
+        if (!LONG || t.go >= 32 || t.nsplit <= kFlatFewRanges) {
           for (int o = lane; o < t.go; o += 32) {
             double s = 0.0;
-#pragma unroll 8
+#pragma unroll(LONG ? 8 : 1)
             for (int q = 0; q < t.nsplit; q++) s += __ldcg(p + (int64_t)q * t.gs + o);
             C[t.c_off + t.o0 + o] = s;
           }
@@ -310,10 +313,12 @@ __global__ void __launch_bounds__(32 * kWarps, kFlatCtasPerSm)
 }  // namespace
 
 void launch_gemm_fp64_flat(const FlatItem* items, int nitems, const double* A, const double* B, double* C, double* ws,
-                           int* counters, const ViewHdr* views, const int64_t* pool, int grid, cudaStream_t s) {
+                           int* counters, const ViewHdr* views, const int64_t* pool, bool long_k, int grid,
+                           cudaStream_t s) {
   if (nitems <= 0) return;
-  launch_pdl(views ? gemm_fp64_flat_kernel<true> : gemm_fp64_flat_kernel<false>, dim3(grid), dim3(32 * kWarps), 0, s,
-             items, nitems, A, B, C, ws, counters, views, pool);
+  auto kernel = views ? (long_k ? gemm_fp64_flat_kernel<true, true> : gemm_fp64_flat_kernel<true, false>)
+                      : (long_k ? gemm_fp64_flat_kernel<false, true> : gemm_fp64_flat_kernel<false, false>);
+  launch_pdl(kernel, dim3(grid), dim3(32 * kWarps), 0, s, items, nitems, A, B, C, ws, counters, views, pool);
 }
 
 }  // namespace tn
