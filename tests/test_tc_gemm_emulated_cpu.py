@@ -96,7 +96,7 @@ def test_a_wait_that_gives_up(exe, mode, hold):
 
 # rows and columns around the strips of 16 and the groups of 8, K around the
 # staged extents (1024 a warp, 8192 a CTA) and odd, from a null base
-@pytest.mark.parametrize("size", [(9, 17, 33), (1, 1, 1), (8, 16, 576), (3, 5, 1041), (2, 3, 2001), (1, 2, 8200), (20, 40, 100)])
+@pytest.mark.parametrize("size", [(9, 17, 33), (1, 1, 1), (8, 16, 576), (3, 5, 1041), (9, 3, 1100), (2, 3, 1101), (2, 3, 2001), (1, 2, 8200), (20, 40, 100)])
 def test_slicing_addresses(slice_exe, size):
     if size[2] > 576:  # longer strips are a cluster's
         size = (size[0], 0, size[2])

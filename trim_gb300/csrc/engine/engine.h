@@ -523,7 +523,13 @@ void launch_tc_maxima(const TcSector* secs, int nsec, const int64_t* a_ts, int64
 // where K > kRowWarp.  Strips of more than kSliceWideK rows are shared by
 // slice_group(K) CTAs of a cluster of kSliceCluster; their items come first, one
 // per kSliceCluster / group strips: (sector, the first of them)
-constexpr int kRowWarp = 2000, kSliceWideK = 576, kSliceCluster = 4;
+// kRowWarp is where the two ways to take a row of A cost the same: a warp keeps
+// 1024 k in shared memory and reads longer rows twice, a CTA keeps 8192 but pays
+// its barriers row by row.  Split precision, 80e6 elements, warp / CTA: K = 1040 452 /
+// 479 us, 1200 453 / 429, 1500 451 / 394, 2048 456 / 354, 4096 535 / 290; BF16 1040 378 /
+// 402, 1200 375 / 355; 300 rows of 1500 24 / 14.  With the line at 2000 the slicing of
+// 1024 contractions of bonds 16..256 took 936 us, at 1500 863, at 1100 843.
+constexpr int kRowWarp = 1100, kSliceWideK = 576, kSliceCluster = 4;
 __host__ __device__ constexpr int slice_group(int K) { return K <= 2 * kSliceWideK ? 2 : 4; }
 void launch_tc_slice_once(int ns, const TcSector* secs, const int2* items, int nshared, int nitems, const double* A,
                           const double* B, unsigned long long* ea, unsigned long long* eb, uint8_t* images,
