@@ -209,10 +209,10 @@ __device__ __forceinline__ int split_tile(MmaState& st) {
 // warp: 32 TMEM lanes x 16 columns at a and at b, as four 16-lane x 16-column
 // loads in the accumulator fragment order: with r = lane / 4 and p = lane % 4,
 // value 8 h + 4 g + 2 u + i is row 16 h + 8 u + r, column 8 g + 2 p + i.  The
-// data is in the registers on return.
+// data is in the registers on return.  The caller's warp_wait has brought the warp
+// together (a __syncwarp here as well took 0.2 to 0.5% of the call).
 __device__ __forceinline__ void tmem_ld32x16x2(uint32_t a, uint32_t b, float (&v)[16], float (&w)[16]) {
   uint32_t r[16], s[16];
-  __syncwarp();
   asm volatile(
       "tcgen05.ld.sync.aligned.16x256b.x2.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%32];\n"
       "tcgen05.ld.sync.aligned.16x256b.x2.b32 {%8,%9,%10,%11,%12,%13,%14,%15}, [%33];\n"
