@@ -38,9 +38,7 @@ const char* last_error();
 struct PerDevice {
   std::atomic<int> value[64] = {};
   template <class F>
-  int get(F&& make) {
-    int dev = 0;
-    TN_CUDA(cudaGetDevice(&dev));
+  int get(int dev, F&& make) {
     std::atomic<int>& v = value[dev & 63];
     int x = v.load(std::memory_order_acquire);
     if (!x || dev > 63) {
@@ -50,9 +48,14 @@ struct PerDevice {
     return x;
   }
 };
+inline int current_device() {
+  int dev = 0;
+  TN_CUDA(cudaGetDevice(&dev));
+  return dev;
+}
 template <class K>
-inline void allow_smem(PerDevice& once, K kernel, size_t bytes) {
-  once.get([&] {
+inline void allow_smem(PerDevice& once, int device, K kernel, size_t bytes) {
+  once.get(device, [&] {
     TN_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
     return 1;
   });
@@ -83,24 +86,30 @@ struct BondSig {
   BondSig changed(int t) const;  // Bond::change (data-structure/lib/Bond.cpp:150-157)
   bool operator==(const BondSig& o) const { return type == o.type && q == o.q && deg == o.deg; }
 };
-// The cache key of a bond signature: its numbers as raw 32-bit words, each bond
-// and the whole preceded by its count, so that keys are self-delimiting.  (As
-// decimal text, a dozen small strings per bond, the keys were a third of the
-// host time of an eager contraction of small tensors.)
+// The cache key of a bond signature: its numbers seven bits to a byte (the top
+// bit set where more follow), each bond and the whole preceded by its count, so
+// that keys are self-delimiting.  (As decimal text, a dozen small strings per bond,
+// the keys were a third of the host time of an eager contraction of small tensors;
+// as 32-bit words a permute of dense bonds spent longer hashing them.)
 struct SigKey {
   std::string s;
   explicit SigKey(size_t nbonds) {
-    s.reserve(4 + nbonds * 96);
+    s.reserve(4 + nbonds * 32);
     word((int32_t)nbonds);
   }
-  void word(int32_t v) { s.append((const char*)&v, sizeof(v)); }
+  void word(int32_t v) {
+    uint32_t u = ((uint32_t)v << 1) ^ (uint32_t)(v >> 31);  // small magnitudes of either sign first
+    for (; u >= 128; u >>= 7) s.push_back((char)(u | 128));
+    s.push_back((char)u);
+  }
   void bond(int type, size_t runs) {
     word(type);
     word((int32_t)runs);
   }
   void run(int u1, int prt, int prtf, int deg) {
-    const int32_t w[3] = {u1, prt + 2 * prtf, deg};
-    s.append((const char*)w, sizeof(w));
+    word(u1);
+    word(prt + 2 * prtf);
+    word(deg);
   }
 };
 std::string sig_key(const std::vector<BondSig>& bonds);
@@ -481,9 +490,9 @@ std::vector<GemmTile> plan_fp64(const std::vector<tn_sector_gemm>& list, int num
 std::vector<FlatItem> plan_fp64_flat(const std::vector<tn_sector_gemm>& list, int num_sms, int64_t* ws_elems,
                                      int64_t* ngroups, const std::vector<std::pair<int, int>>* vw = nullptr);
 
-// kernel launchers (defined in the .cu files)
+// kernel launchers (defined in the .cu files); device: the context's
 // fourth_dim: some tile has a fourth dim
-void launch_permute_kernel(const PermSub* subs, const int64_t* tile_start, int nsub, int64_t ntiles, int esz,
+void launch_permute_kernel(int device, const PermSub* subs, const int64_t* tile_start, int nsub, int64_t ntiles, int esz,
                            bool conj, bool fourth_dim, const void* src, void* dst, int grid, cudaStream_t s);
 // counters (one int per split group, zero between launches) may be null: then
 // split tiles need launch_splitk_reduce afterwards; otherwise the last CTA of

@@ -625,7 +625,7 @@ void run_permute(Ctx& ctx, const PermPlan& plan, const void* src, void* dst) {
   // persistent: two resident CTAs per SM (100 KB of staging shared memory each)
   int64_t grid = std::min<int64_t>(plan.ntiles, (int64_t)ctx.num_sms * 2);
   ProfScope ps(ctx, "permute", 2.0 * plan.esz * plan.elem_num, 0);
-  launch_permute_kernel((const PermSub*)plan.subs->ptr, (const int64_t*)plan.tile_start->ptr, plan.nsub, plan.ntiles,
+  launch_permute_kernel(ctx.device, (const PermSub*)plan.subs->ptr, (const int64_t*)plan.tile_start->ptr, plan.nsub, plan.ntiles,
                         plan.esz, plan.conj, plan.fourth_dim, src, dst, (int)grid, ctx.stream);
   ctx.launched();
 }

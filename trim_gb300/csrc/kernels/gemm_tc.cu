@@ -568,7 +568,7 @@ static void launch_once(const TcSector* secs, const int2* items, int nshared, in
   constexpr int smem = kStageDoubles * (int)sizeof(double);
   if (!nshared) {
     static PerDevice attr;
-    allow_smem(attr, tc_slice_once<NS, false>, smem);
+    allow_smem(attr, current_device(), tc_slice_once<NS, false>, smem);
     tc_slice_once<NS, false>
         <<<std::min(nitems, num_sms * 3), 256, smem, s>>>(secs, items, 0, nitems, A, B, ea, eb, images);
     TN_CUDA(cudaGetLastError());
@@ -586,7 +586,7 @@ static void launch_once(const TcSector* secs, const int2* items, int nshared, in
   cfg.numAttrs = 1;
   cfg.gridDim = dim3((unsigned)(num_sms * 3 / kSliceCluster * kSliceCluster));
   static PerDevice fit;  // clusters the GPU holds at once
-  const int resident = fit.get([&] {
+  const int resident = fit.get(current_device(), [&] {
     TN_CUDA(cudaFuncSetAttribute(tc_slice_once<NS, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
     int n = 0;
     TN_CUDA(cudaOccupancyMaxActiveClusters(&n, tc_slice_once<NS, true>, &cfg));

@@ -301,7 +301,7 @@ void launch_fast(const TcSector* secs, const int4* items, int nitems, int wide, 
                  cudaStream_t s) {
   constexpr size_t smem = (size_t)kStages * kStage + 1024;
   static PerDevice attr;  // per instantiation
-  allow_smem(attr, tc_gemm_fast<NS>, smem);
+  allow_smem(attr, current_device(), tc_gemm_fast<NS>, smem);
   tc_gemm_fast<NS><<<grid, kThreadsFast, smem, s>>>(secs, items, nitems, wide, ws, ea, eb, C, part, err);
   TN_CUDA(cudaGetLastError());
 }

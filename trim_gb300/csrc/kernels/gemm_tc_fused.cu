@@ -547,11 +547,11 @@ void launch_tc_fused(int ns, const TcSector* secs, const int4* items, int nitems
   const size_t smem = tc_fused_smem(ns);
   if (ns == 7) {
     static PerDevice attr;
-    allow_smem(attr, tc_fused<7>, smem);
+    allow_smem(attr, current_device(), tc_fused<7>, smem);
     tc_fused<7><<<grid, kFThreads, smem, s>>>(secs, items, nitems, A, B, C, views, pool, err, rpi);
   } else {
     static PerDevice attr;
-    allow_smem(attr, tc_fused<1>, smem);
+    allow_smem(attr, current_device(), tc_fused<1>, smem);
     tc_fused<1><<<grid, kFThreads, smem, s>>>(secs, items, nitems, A, B, C, views, pool, err, rpi);
   }
   TN_CUDA(cudaGetLastError());

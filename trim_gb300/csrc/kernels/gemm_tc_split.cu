@@ -477,7 +477,7 @@ void launch_tc_gemm_split(const TcSector* secs, const int4* items, int nitems, c
                           int* err, int grid, cudaStream_t s) {
   constexpr size_t smem = (size_t)kARing * kATile + (size_t)kBRing * kDigits * kBTile + 1024;
   static PerDevice attr;
-  allow_smem(attr, tc_gemm_split, smem);
+  allow_smem(attr, current_device(), tc_gemm_split, smem);
   tc_gemm_split<<<grid, kThreadsSplit, smem, s>>>(secs, items, nitems, ws, ea, eb, C, part, err);
   TN_CUDA(cudaGetLastError());
 }

@@ -608,23 +608,23 @@ int64_t check_permute_plan_host(const PermPlan& plan, const double* src, double*
 }
 
 template <typename T, typename Info>
-static void launch_permute_t(const PermSub* subs, const int64_t* tile_start, int nsub, int64_t ntiles, const T* src,
-                             T* dst, uint64_t conj, int grid, cudaStream_t s) {
+static void launch_permute_t(int device, const PermSub* subs, const int64_t* tile_start, int nsub, int64_t ntiles,
+                             const T* src, T* dst, uint64_t conj, int grid, cudaStream_t s) {
   const size_t smem = (size_t)kStages * kSmem * sizeof(double);
   static PerDevice attr;  // per instantiation
-  allow_smem(attr, permute_kernel<T, Info>, smem);
+  allow_smem(attr, device, permute_kernel<T, Info>, smem);
   launch_pdl(permute_kernel<T, Info>, dim3(grid), dim3(kThreads), smem, s, subs, tile_start, nsub, ntiles, src, dst, conj);
 }
 
-void launch_permute_kernel(const PermSub* subs, const int64_t* tile_start, int nsub, int64_t ntiles, int esz,
+void launch_permute_kernel(int device, const PermSub* subs, const int64_t* tile_start, int nsub, int64_t ntiles, int esz,
                            bool conj, bool fourth_dim, const void* src, void* dst, int grid, cudaStream_t s) {
   const uint64_t c = conj ? 0x8000000000000000ull : 0ull;
   if (esz == 8) {
     auto f = fourth_dim ? launch_permute_t<double, TileInfoW> : launch_permute_t<double, TileInfo>;
-    f(subs, tile_start, nsub, ntiles, (const double*)src, (double*)dst, 0, grid, s);
+    f(device, subs, tile_start, nsub, ntiles, (const double*)src, (double*)dst, 0, grid, s);
   } else if (esz == 16) {
     auto f = fourth_dim ? launch_permute_t<double2, TileInfoW> : launch_permute_t<double2, TileInfo>;
-    f(subs, tile_start, nsub, ntiles, (const double2*)src, (double2*)dst, c, grid, s);
+    f(device, subs, tile_start, nsub, ntiles, (const double2*)src, (double2*)dst, c, grid, s);
   } else
     fail(TN_ERR_ARG, "permute: element size must be 8 or 16 bytes");
 }

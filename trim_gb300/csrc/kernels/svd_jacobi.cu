@@ -614,7 +614,7 @@ void launch_truncate(const int64_t* s_off, const int64_t* s_cnt, int nsec, int64
   if (staged) smem = all;
   // the most any call takes, not this one's: another thread's call would lower it
   static PerDevice attr;
-  allow_smem(attr, truncate_kernel, kSvdMaxSmem);
+  allow_smem(attr, current_device(), truncate_kernel, kSvdMaxSmem);
   truncate_kernel<<<1, 1024, smem, s>>>(s_off, s_cnt, nsec, S, chi, kept, norm, staged ? (int)total : 0);
   TN_CUDA(cudaGetLastError());
 }
