@@ -31,15 +31,24 @@ struct Dim {
 //         that each tile still moves thousands of elements; z is the dim
 //         with the smallest source or destination stride (it extends a
 //         contiguous run on one side); of 8-byte elements tw values of a
-//         fourth dim are added where that leaves the tile half empty.
+//         fourth dim are added where that leaves the tile nearly empty.
 //
 // Limits are in elements: a tile <= 4096 elements and a transpose tile within
 // 64 x 65 for 8-byte elements; es = 2 (16-byte elements) halves both, so a
 // tile fills the same shared memory.  Transpose rows stay up to 64 elements
 // wide either way (64 x 32 complex tiles: 86% of the copy rate against 69%
 // for 32 x 63 ones).
-void choose_tile(PermSub& ps, int es) {
+//
+// The rules that fill tiles further (longer destination rows, another y, a
+// fourth dim) are for plans with a full tile for each of the 304 resident CTAs
+// (`full`).  Smaller ones are one round of tiles whatever their size, and end
+// with their slowest: 49 560 elements in 14 tiles of 3540 took 13.9 us, in 826 of
+// 60 4.4.
+void choose_tile(PermSub& ps, int es, int64_t elem_num) {
   const int64_t kTile = 4096 / es, kStage = (64 * 65) / es, kRow = 64;
+  const bool full = elem_num >= 304 * kTile;
+  // at most `most` of ext values in a tile, the tiles alike (12 as 6 + 6, not 9 + 3)
+  auto even = [](int64_t ext, int64_t most) { return (int32_t)((ext + (ext + most - 1) / most - 1) / ((ext + most - 1) / most)); };
   const int n = ps.ndim;
   ps.ydim = -1;
   ps.zdim = ps.wdim = -1;
@@ -70,20 +79,23 @@ void choose_tile(PermSub& ps, int es) {
     // that the tile fills.  (3000, 3000, 3) with the last bond first 782 -> 86 us, 3e6
     // x 7 268 -> 73, 24^4 x 24 37 -> 29; from half a tile of 64-element rows on the
     // power of two is worth more, 60 x 60^3 41 -> 46 us, complex 24 x 4e5 60 -> 64.
-    if (n == 2 && ps.dims[y] <= (es == 1 ? 32 : 15)) {
+    if (n == 2 && ps.dims[y] <= (es == 1 ? 32 : 15) && full) {
       const int64_t tx = std::min(kTile / ps.dims[y], kStage / ps.dims[y] - 1) & ~(int64_t)3;
       ps.tx = (int32_t)std::min<int64_t>(ps.dims[x], tx);
       ps.ty = (int32_t)ps.dims[y];
-    } else if (es == 1) {
-      // Narrower rows where that takes clearly fewer tiles: 96 x 96 as three tiles
+    } else if (es == 1 && elem_num >= (int64_t)1 << 23) {
+      // Narrower rows where that takes clearly fewer tiles, in plans that come from
+      // memory (below about 8e6 elements L2 holds both sides, and the tiles' uneven
+      // steps cost more: 133^3 8.7 -> 10.4 us): 96 x 96 as three tiles
       // of 32 x 96, not 64 + 32 in both directions.  Transposes of 80^4, 96^4 and
       // 100^4: 250, 360 and 489 us -> 155, 289 and 362 at most.  (16-byte elements
-      // keep their 64 x 32 tiles: 100 x 100 x 8 x 100 ran up to 10% slower in 52 x 34.)
+      // keep their 64 x 32 tiles: 100 x 100 x 8 x 100 ran up to 10% slower in 52 x 34.
+      // A seventh fewer tiles is not enough: 329579 x 212 240 -> 263 us.)
       // The widths that an even split of x comes to are few: 64, 60, .., 32.
       auto tiles = [&](int64_t tx, int64_t ty) {
         return ((ps.dims[x] + tx - 1) / tx) * ((ps.dims[y] + ty - 1) / ty);
       };
-      int64_t best = tiles(ps.tx, ps.ty) * 7 / 8;
+      int64_t best = tiles(ps.tx, ps.ty) * 3 / 4;
       for (int64_t tx = kRow; tx >= kRow / 2; tx -= 4) {
         const int64_t nx = (ps.dims[x] + tx - 1) / tx;
         if (ps.dims[x] / nx < kRow / 2 || (((ps.dims[x] + nx - 1) / nx + 3) & ~(int64_t)3) != tx) continue;
@@ -107,7 +119,7 @@ void choose_tile(PermSub& ps, int es) {
       // took 71 us, now 31.)
       const int64_t rows = std::max<int64_t>(1, kTile / ps.tx);
       ps.ydim = n - 2;
-      if (ps.tx >= 32)
+      if (ps.tx >= 32 && full)
         for (int i = n - 3; i >= 0; i--)
           if (std::min<int64_t>(ps.dims[i], rows) > std::min<int64_t>(ps.dims[ps.ydim], rows)) ps.ydim = i;
       ps.ty = (int32_t)std::min<int64_t>(ps.dims[ps.ydim], rows);
@@ -133,12 +145,13 @@ void choose_tile(PermSub& ps, int es) {
         best = c;
       }
     }
-    const int64_t tz = std::min<int64_t>((int64_t)ps.dims[z], kTile / ((int64_t)ps.tx * ps.ty));
-    if (tz > 1 && (int64_t)ps.tx * ps.ty > kTile / 16) {
+    const int64_t xy = (int64_t)ps.tx * ps.ty;
+    const int64_t tz = std::min<int64_t>((int64_t)ps.dims[z], kTile / xy);
+    if (tz > 1 && xy > kTile / 16 && full) {
       ps.mode = 3;
       ps.wdim = z;
-      ps.tw = (int32_t)tz;
-    } else if (tz > 1) {
+      ps.tw = even(ps.dims[z], tz);
+    } else if (tz > 1 && xy <= kTile / 16) {
       ps.mode = 3;
       ps.zdim = z;
       ps.tz = (int32_t)tz;
@@ -147,7 +160,7 @@ void choose_tile(PermSub& ps, int es) {
       // 215 us, with 4 values of the second chi bond in a tile 118 us.
       const int64_t tile = (int64_t)ps.tx * ps.ty * tz;
       int w = -1;
-      if (tile <= kTile / 2)
+      if (tile <= kTile / 2 && full)
         for (int i = 0; i < n - 1; i++) {
           if (i == ps.ydim || i == z) continue;
           const int64_t c = std::min(ps.sstride[i], ps.dstride[i]);
@@ -158,7 +171,7 @@ void choose_tile(PermSub& ps, int es) {
         }
       if (w >= 0) {
         ps.wdim = w;
-        ps.tw = (int32_t)std::min<int64_t>(ps.dims[w], kTile / tile);
+        ps.tw = even(ps.dims[w], kTile / tile);
       }
     }
   }
@@ -166,7 +179,7 @@ void choose_tile(PermSub& ps, int es) {
   // leaves room for the dim that continues the destination row, to 32 elements.
   // (The tile of 2 x 1000 wrote 16 bytes at a time: (200, 2, 200, 1000) -> (1000,
   // 200, 200, 2) 930 -> 400 us.  Complex rows of two fill a sector: no gain.)
-  if (es == 1 && ps.mode == 1 && ps.dims[x] < 16 && n >= 3)
+  if (es == 1 && ps.mode == 1 && ps.dims[x] < 16 && n >= 3 && full)
     for (int i = 0; i < n; i++)
       if (i != x && i != y && ps.dstride[i] == ps.dims[x]) {
         const int64_t tz = std::min<int64_t>(ps.dims[i], (32 + ps.tx - 1) / ps.tx);
@@ -190,12 +203,13 @@ void choose_tile(PermSub& ps, int es) {
       ps.mode = 2;
       ps.zdim = z;
       ps.tz = (int32_t)tz;
-      // and a fourth dim where that leaves the tile half empty: 6^9 transposes
-      // 144 -> 66 us at most (216-element tiles; complex ones, whose tiles hold half
-      // as many and whose single elements fill a 16-byte access, lost up to half)
+      // and a fourth dim where that leaves the tile nearly empty: 6^9 transposes
+      // 144 -> 66 us at most (216-element tiles; of 900 and more elements they lost up
+      // to 27%; complex ones, whose tiles hold half as many and whose single elements
+      // fill a 16-byte access, up to half)
       const int64_t tile = (int64_t)ps.tx * ps.ty * tz;
       int w = -1;
-      if (es == 1 && tile <= kTile / 2)
+      if (es == 1 && tile <= kTile / 8 && full)
         for (int i = 0; i < n; i++) {
           if (i == x || i == y || i == z) continue;
           const int64_t c = std::min(ps.sstride[i], ps.dstride[i]);
@@ -208,7 +222,7 @@ void choose_tile(PermSub& ps, int es) {
         const int64_t tw = std::min<int64_t>({(int64_t)ps.dims[w], kStage / (tz * ps.ty * (ps.tx + 1)), kTile / tile});
         if (tw > 1) {
           ps.wdim = w;
-          ps.tw = (int32_t)tw;
+          ps.tw = even(ps.dims[w], tw);
         }
       }
     }
@@ -357,7 +371,7 @@ std::vector<PermSub> build_perm_subs(const SectorMap& src, const SectorMap& dst,
       ps.sstride[i] = dims[i].s;
       ps.dstride[i] = dims[i].d;
     }
-    choose_tile(ps, esz / 8);
+    choose_tile(ps, esz / 8, src.elem_num);
     subs.push_back(ps);
   }
   return subs;
@@ -532,7 +546,7 @@ PermPlanP get_transpose_plan(Ctx& ctx, const SectorMap& src, const SectorMap& ds
       ps.sstride[i] = dims[i].s;
       ps.dstride[i] = dims[i].d;
     }
-    choose_tile(ps, esz / 8);
+    choose_tile(ps, esz / 8, src.elem_num);
     subs.push_back(ps);
   }
   return finish_plan(ctx, key, subs, src.elem_num, esz, conj);

@@ -252,22 +252,22 @@ __device__ __forceinline__ void issue_tile(const Info& w, const T* __restrict__ 
       // [z][y][x] with pitch tx + 1.  A thread takes (y, x) pairs with lanes
       // along y (source-contiguous) and walks the tile's z planes for each
       // with a constant source step: one division per pair, not per element.
+      // With a fourth dim the threads take (w, y, x) triples.
       const int pitch = w.tx + 1, plane = w.ty * pitch, pairs = w.ty * w.tx;
-      for (int p = threadIdx.x; p < pairs; p += kThreads) {
+      int units = pairs;
+      if constexpr (Info::kFourthDim) units *= w.nw;
+      for (int u = threadIdx.x; u < units; u += kThreads) {
+        int ww = 0, p = u;
+        if constexpr (Info::kFourthDim) ww = u / pairs, p = u - ww * pairs;
         const int xx = p / w.ty, yy = p - xx * w.ty;
         if (xx >= w.nx || yy >= w.ny) continue;
         const T* g = src + w.bs + (int64_t)yy * w.sy + (int64_t)xx * w.sx;
         T* sp = buf + yy * pitch + xx;
         if constexpr (Info::kFourthDim) {
-          const T* gw = g;
-          for (int ww = 0; ww < w.nw; ww++, gw += w.sw) {
-            sp = buf + yy * pitch + xx + ww * w.tz * plane;
-            g = gw;
-            for (int zz = 0; zz < w.nz; zz++, g += w.sz, sp += plane) cp_async_el(sp, g);
-          }
-        } else {
-          for (int zz = 0; zz < w.nz; zz++, g += w.sz, sp += plane) cp_async_el(sp, g);
+          g += ww * w.sw;
+          sp += ww * w.tz * plane;
         }
+        for (int zz = 0; zz < w.nz; zz++, g += w.sz, sp += plane) cp_async_el(sp, g);
       }
     } else if (w.mode == 3) {
       // [w][z][y][x] dense; elements of a (z, y, x) block in source-stride order,
@@ -344,21 +344,20 @@ __device__ __forceinline__ void store_tile(const Info& w, const T* buf, T* __res
   const Flip f{flip, flip ^ conj};
   if (w.mode == 2) {  // (x, y) pairs with lanes along x; the z planes with a constant step
     const int pitch = w.tx + 1, plane = w.ty * pitch, pairs = w.ty * w.tx;
-    for (int p = threadIdx.x; p < pairs; p += kThreads) {
+    int units = pairs;
+    if constexpr (Info::kFourthDim) units *= w.nw;
+    for (int u = threadIdx.x; u < units; u += kThreads) {
+      int ww = 0, p = u;
+      if constexpr (Info::kFourthDim) ww = u / pairs, p = u - ww * pairs;
       const int yy = p / w.tx, xx = p - yy * w.tx;
       if (xx >= w.nx || yy >= w.ny) continue;
       const T* sp = buf + yy * pitch + xx;
       T* g = dst + w.bd + (int64_t)yy * w.dy + (int64_t)xx * w.dx;
       if constexpr (Info::kFourthDim) {
-        T* gw = g;
-        for (int ww = 0; ww < w.nw; ww++, gw += w.dw) {
-          sp = buf + yy * pitch + xx + ww * w.tz * plane;
-          g = gw;
-          for (int zz = 0; zz < w.nz; zz++, sp += plane, g += w.dz) *g = apply_flip(*sp, f);
-        }
-      } else {
-        for (int zz = 0; zz < w.nz; zz++, sp += plane, g += w.dz) *g = apply_flip(*sp, f);
+        g += ww * w.dw;
+        sp += ww * w.tz * plane;
       }
+      for (int zz = 0; zz < w.nz; zz++, sp += plane, g += w.dz) *g = apply_flip(*sp, f);
     }
     return;
   }
