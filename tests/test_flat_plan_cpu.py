@@ -59,6 +59,20 @@ def test_large_outputs_over_a_long_k(plan, shapes):
     assert ws <= 128 * 2 * 96 * 4 * SMS
 
 
+@pytest.mark.parametrize("shapes", [[(1, 1, 562)], [(4, 4, 105)] * 2, [(3, 7, 14786)], [(4460, 1, 59)], [(281, 1, 55)] * 100, [(2, 39, 895)], [(9, 16, 320)] * 20])
+def test_lists_that_leave_warps_idle(plan, shapes):
+    """The longest item costs at most two of the least (64 warp FMAs), and a
+    warp adds up no more ranges than the square root of K, or 8, unless the lanes
+    run along them."""
+    items, _, cost, ranges = plan(*shapes)
+    m, n, k = shapes[0]
+    assert cost <= 2 * 64
+    assert ranges <= max(8, k ** 0.5) or n <= 8 or m * n >= 128
+    if n <= 8 and k >= 32:  # rows: spread over the resident warps, four to a warp at most beyond that
+        rows = m * len(shapes)
+        assert items >= min(rows, rows // 12)
+
+
 def test_every_product_once(plan):
     plan(*[(m, n, k) for m in (1, 3, 33, 130) for n in (1, 2, 3, 32) for k in (1, 31, 32, 700, 40001)])
     plan((5, 2, 99999), (1, 1, 12345678), (7, 18, 5000), (300, 300, 64))

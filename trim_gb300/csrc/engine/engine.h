@@ -236,7 +236,7 @@ struct FlatItem {
 };
 constexpr int kFlatWarps = 4, kFlatCtasPerSm = 5;  // warps per CTA, CTAs an SM holds (registers)
 constexpr int kFlatSlots = 4, kFlatViewSlots = 2;  // slots per item, and with a view
-constexpr int kFlatFewRanges = 32;  // K ranges that a lane adds up by itself
+constexpr int kFlatFewRanges = 32;  // K ranges that the plain kernel adds up one after another
 
 // Planning choices of the FP64 grouped GEMM (the autotuner's search space):
 // flat items, or tiles with a width rule (0: the
@@ -503,7 +503,8 @@ void launch_permute_kernel(int device, const PermSub* subs, const int64_t* tile_
 void launch_gemm_fp64(const GemmTile* tiles, int ntiles, const double* A, const double* B, double* C,
                       double* ws, int* counters, const ViewHdr* views, const int64_t* pool, int grid,
                       cudaStream_t s, bool dependent_launch = true);
-// long_k: some item is a row over a part of K, or of a group of more than kFlatFewRanges
+// long_k: some item is a row over a part of K or of a group of more than
+// kFlatFewRanges, or the list has fewer items than the GPU holds warps
 void launch_gemm_fp64_flat(const FlatItem* items, int nitems, const double* A, const double* B, double* C, double* ws,
                            int* counters, const ViewHdr* views, const int64_t* pool, bool long_k, int grid,
                            cudaStream_t s);

@@ -154,7 +154,7 @@ std::vector<GemmTile> plan_fp64(const std::vector<tn_sector_gemm>& list, int num
 // least 64 warp FMAs, below which an item's own latency shows; at most 4096, or
 // a 96th of the share where that is more: a list of 8e9 multiply-adds and up
 // would only grow, items and partial sums by the gigabyte).
-// (Sixteenths were up to 7% slower, on 64 uneven contractions 414 -> 386 us, an
+// (Sixteenths were up to 7% slower, on 64 uneven contractions 404 -> 376 us, an
 // iPEPS quadrant at chi = 48, D = 5 460 -> 448; 48ths up to 6% faster still on some
 // lists and 2% slower on others.)
 // Sectors of at least 128 outputs are cut into chunks of at most 4 slots (one
@@ -162,24 +162,35 @@ std::vector<GemmTile> plan_fp64(const std::vector<tn_sector_gemm>& list, int num
 // second choice), each with its K ranges as a group; smaller ones deal all
 // their (K range, output) pairs to lanes, with the number of ranges raised
 // while more than 1 lane in 16 would stay empty; 256 at most, or
-// 8192 partial sums (one warp adds them up).  One- and two-column sectors (a norm, an expectation value) take
-// rows, lanes along K, and K ranges of a row as soon as one costs two items;
-// with a whole row to a warp 1 x 1 over K = 1e6 took one warp 31 250 steps.  An item that reads an operand
-// through views walks its K range in the views' segments, so its entries share
-// one range.
+// 8192 partial sums (one warp adds them up).  One- and two-column sectors (a norm, an
+// expectation value) take rows, lanes along K, and K ranges of a row as soon as
+// one costs two items; with a whole row to a warp 1 x 1 over K = 1e6 took one warp
+// 31 250 steps.  An item that reads an operand through views walks its K range in
+// the views' segments, so its entries share one range.
+constexpr double kFlatFloor = 64.0;   // warp FMAs of an item, at least
 constexpr int64_t kRowRanges = 1024;  // K ranges of a row: two for every resident warp of half the chip
 std::vector<FlatItem> plan_fp64_flat(const std::vector<tn_sector_gemm>& list, int num_sms, int64_t* ws_elems,
                                      int64_t* ngroups, const std::vector<std::pair<int, int>>* vw) {
   auto row_cost = [](int64_t n, int64_t k) { return n * ((k + 31) / 32 + 5); };  // warp FMAs, and 5 to sum the lanes
-  double total = 0;
+  auto viewed = [&](size_t gi) { return vw && ((*vw)[gi].first >= 0 || (*vw)[gi].second >= 0); };
+  double total = 0, rows8 = 0;
   for (size_t gi = 0; gi < list.size(); gi++) {
     const auto& g = list[gi];
     if (g.M <= 0 || g.N <= 0 || g.K <= 0) continue;
-    const bool rows = g.N <= 2 && g.K >= 32 && !(vw && ((*vw)[gi].first >= 0 || (*vw)[gi].second >= 0));
-    total += rows ? (double)g.M * (double)row_cost(g.N, g.K) : std::ceil((double)g.M * g.N / 32.0) * (double)g.K;
+    const bool rows = g.K >= 32 && !viewed(gi);
+    total += rows && g.N <= 2 ? (double)g.M * (double)row_cost(g.N, g.K) : std::ceil((double)g.M * g.N / 32.0) * (double)g.K;
+    if (rows && g.N <= 8) rows8 += (double)g.M;
   }
   const double share = total / (4.0 * num_sms);
-  const int64_t target = (int64_t)std::min(std::max(4096.0, share / 96.0), std::max(64.0, share / 24.0));
+  const int64_t target = (int64_t)std::min(std::max(4096.0, share / 96.0), std::max(kFlatFloor, share / 24.0));
+  // A list so small that items are at their least leaves warps idle and lasts as
+  // long as its longest item: up to 8 columns are rows there (a lane's chain is K /
+  // 32 long, not K), and no more rows to an item than leave every resident warp one.
+  const bool idle = share / 24.0 < kFlatFloor;
+  const int64_t warps = (int64_t)num_sms * kFlatCtasPerSm * kFlatWarps;
+  const int64_t row_cols = idle && rows8 <= (double)warps ? 8 : 2;
+  int64_t most_rows = idle ? std::max<int64_t>(1, (int64_t)std::ceil(rows8 / (double)warps)) : 64;
+  if (most_rows > 2) most_rows = (most_rows + 3) & ~(int64_t)3;  // rows are taken four at a time
   std::vector<FlatItem> out;
   int64_t ws = 0, ngrp = 0;
   const int64_t most_plain = std::max<int64_t>(1, std::min<int64_t>(kFlatSlots, target / 256));  // slots per chunk
@@ -197,12 +208,12 @@ std::vector<FlatItem> plan_fp64_flat(const std::vector<tn_sector_gemm>& list, in
     t.nsplit = 1;
     t.a_vw = vw ? (*vw)[gi].first : -1;
     t.b_vw = vw ? (*vw)[gi].second : -1;
-    const bool viewed = t.a_vw >= 0 || t.b_vw >= 0;
-    if (g.N <= 2 && g.K >= 32 && !viewed) {  // lanes along K
+    if (g.N <= row_cols && g.K >= 32 && !viewed(gi)) {  // lanes along K
       t.rows = 1;
       t.mn = (int32_t)g.M;
       const int64_t row = row_cost(g.N, g.K);
-      const int64_t per = std::max<int64_t>(1, std::min<int64_t>(64, target / row));
+      int64_t per = std::max<int64_t>(1, std::min<int64_t>(most_rows, idle ? 2 * target / row : target / row));
+      if (per > 4) per &= ~(int64_t)3;
       // a row of more than two items' cost: K ranges, a multiple of the 32 lanes each
       const int64_t ns = row > 2 * target ? std::min<int64_t>((row + target - 1) / target, kRowRanges) : 1;
       t.kc = (int32_t)(ns > 1 ? (((g.K + ns - 1) / ns + 31) / 32) * 32 : g.K);
@@ -224,8 +235,8 @@ std::vector<FlatItem> plan_fp64_flat(const std::vector<tn_sector_gemm>& list, in
     }
     const int64_t mn = g.M * g.N, slots = (mn + 31) / 32;
     t.mn = (int32_t)mn;
-    if (mn >= 128 || viewed) {
-      const int64_t most = viewed ? std::min<int64_t>(most_plain, kFlatViewSlots) : most_plain;
+    if (mn >= 128 || viewed(gi)) {
+      const int64_t most = viewed(gi) ? std::min<int64_t>(most_plain, kFlatViewSlots) : most_plain;
       const int64_t nch = (slots + most - 1) / most;
       const int64_t kc0 = std::max<int64_t>(32, target * nch / slots);
       const int64_t ns = std::max<int64_t>(1, std::min<int64_t>((g.K + kc0 / 2) / kc0, 256));
@@ -250,7 +261,10 @@ std::vector<FlatItem> plan_fp64_flat(const std::vector<tn_sector_gemm>& list, in
       }
     } else {
       const int64_t kc0 = std::max<int64_t>(32, target);
-      int64_t ns = std::max<int64_t>(1, std::min((g.K + kc0 - 1) / kc0, std::max<int64_t>(256, 8192 / mn)));
+      int64_t most = std::max<int64_t>(256, 8192 / mn);
+      if (idle)  // a range's chain and the chain of sums come out alike
+        most = std::min(most, std::max<int64_t>(8, (int64_t)std::sqrt((double)(g.K / slots))));
+      int64_t ns = std::max<int64_t>(1, std::min((g.K + kc0 - 1) / kc0, most));
       auto waste = [&](int64_t n) { return (double)((mn * n + 31) / 32 * 32) / (double)(mn * n); };
       while (waste(ns) > 1.0625 && ns < 32 && g.K / (ns + 1) >= 32) ns++;
       t.kc = (int32_t)((g.K + ns - 1) / ns);
@@ -349,7 +363,8 @@ static std::shared_ptr<Fp64Plan> get_fp64_plan(Ctx& ctx, const std::vector<tn_se
   if (flat) {
     items = plan_fp64_flat(list, ctx.num_sms, &P->ws_elems, &ngrp, vw);
     P->nflat = (int)items.size();
-    for (const auto& t : items) P->long_k |= t.nsplit > kFlatFewRanges || (t.rows && t.nsplit > 1);
+    P->long_k = P->nflat <= ctx.num_sms * kFlatCtasPerSm * kFlatWarps;
+    for (const auto& t : items) P->long_k |= t.nsplit > kFlatFewRanges || (t.rows && (t.nsplit > 1 || t.N > 2));
   } else {
     tiles = plan_fp64_split(list, ctx.num_sms, true, &P->ws_elems, pol, vw);
     for (const auto& t : tiles) ngrp = std::max<int64_t>(ngrp, (int64_t)t.grp + 1);

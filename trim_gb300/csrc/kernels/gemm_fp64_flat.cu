@@ -56,7 +56,7 @@ __device__ __forceinline__ int find_start(const int64_t* __restrict__ st, int n,
 template <int R>
 __device__ __forceinline__ void fma_run(double (&acc)[R], const double* const (&pa)[R], const double* (&pb)[R],
                                         const int64_t (&ldb)[R], int len) {
-  constexpr int U = R <= 2 ? 4 : 2;
+  constexpr int U = R == 1 ? 8 : (R == 2 ? 4 : 2);  // loads in flight: a small item is their latency
   int k = 0;
   for (; k + U <= len; k += U) {
     double a[R][U], b[R][U];
@@ -194,38 +194,92 @@ __device__ __forceinline__ void flat_body(const FlatItem& t, int lane, const dou
     }
 }
 
-// Sectors of one or two columns: lanes along K (A's row and B's rows read
-// coalesced; flat lanes would gather 16 or 32 rows of A per load), the lanes'
-// sums added by a fixed shuffle butterfly; the item's entries are nv rows.
+// The sums over the lanes of V values, P = V rounded up to a power of two: while
+// there are several, a lane keeps half of them and gives the other half away, so
+// that four values cost 6 additions, not 20 (an addition holds the FP64 pipe as
+// long as an FMA).  Lane j 32 / P returns the sum of value j.
+template <int V, int P>
+__device__ __forceinline__ double lane_sums(const double (&x)[V], int lane) {
+  double v[P];
+#pragma unroll
+  for (int i = 0; i < P; i++) v[i] = i < V ? x[i] : 0.0;
+  int o = 16;
+#pragma unroll
+  for (int s = P / 2; s > 0; s >>= 1, o >>= 1) {
+    const bool high = lane & o;
+#pragma unroll
+    for (int i = 0; i < s; i++) {
+      const double give = high ? v[i] : v[i + s], keep = high ? v[i + s] : v[i];
+      v[i] = keep + __shfl_xor_sync(0xffffffffu, give, o);
+    }
+  }
+  for (; o > 0; o >>= 1) v[0] += __shfl_xor_sync(0xffffffffu, v[0], o);
+  return v[0];
+}
+
+// Sectors of few columns: lanes along K (A's row and B's rows read coalesced;
+// flat lanes would gather 16 or 32 rows of A per load), the lanes' sums added by
+// fixed shuffles; the item's entries are nv rows, RB of them at a time where there
+// are as many (one row's loads and shuffles leave the warp waiting).
+template <int NN, int RB, bool LONG>
+__device__ __forceinline__ void row_block(const FlatItem& t, int m, int lane, const double* __restrict__ A,
+                                          const double* __restrict__ B, double* __restrict__ C,
+                                          double* __restrict__ ws) {
+  const double* __restrict__ a = A + t.a_off + (int64_t)m * t.K;
+  const double* __restrict__ b = B + t.b_off;
+  const int k0 = LONG ? t.kq * t.kc : 0, k1 = LONG ? min(t.K, k0 + t.kc) : t.K;
+  constexpr int V = RB * NN, P = V <= 2 ? V : (V <= 4 ? 4 : 8);
+  double acc[V];
+#pragma unroll
+  for (int i = 0; i < V; i++) acc[i] = 0.0;
+#pragma unroll 4
+  for (int k = k0 + lane; k < k1; k += 32) {
+    double bv[NN];
+#pragma unroll
+    for (int n = 0; n < NN; n++) bv[n] = __ldg(b + (int64_t)k * NN + n);
+#pragma unroll
+    for (int r = 0; r < RB; r++) {
+      const double av = __ldg(a + (int64_t)r * t.K + k);
+#pragma unroll
+      for (int n = 0; n < NN; n++) acc[r * NN + n] = fma(av, bv[n], acc[r * NN + n]);
+    }
+  }
+  const double s = lane_sums<V, P>(acc, lane);
+  const int j = lane / (32 / P);  // the rows of the block lie one after another
+  if (lane % (32 / P) == 0 && j < V) {
+    if (!LONG || t.grp < 0)
+      C[t.c_off + (int64_t)m * NN + j] = s;
+    else
+      ws[t.ws_off + (int64_t)t.kq * t.gs + (m * NN + j - t.o0)] = s;
+  }
+}
+
 template <int NN, bool LONG>
 __device__ __forceinline__ void row_body(const FlatItem& t, int lane, const double* __restrict__ A,
                                          const double* __restrict__ B, double* __restrict__ C,
                                          double* __restrict__ ws) {
-  const double* __restrict__ b = B + t.b_off;
-  const int k0 = LONG ? t.kq * t.kc : 0, k1 = LONG ? min(t.K, k0 + t.kc) : t.K;
+  constexpr int RB = NN == 1 ? 4 : (NN == 2 ? 2 : 1);
   pdl_wait();
-  for (int m = t.v0; m < t.v0 + t.nv; m++) {
-    const double* __restrict__ a = A + t.a_off + (int64_t)m * t.K;
-    double acc[NN];
-#pragma unroll
-    for (int n = 0; n < NN; n++) acc[n] = 0.0;
-#pragma unroll 4
-    for (int k = k0 + lane; k < k1; k += 32) {
-      const double av = __ldg(a + k);
-#pragma unroll
-      for (int n = 0; n < NN; n++) acc[n] = fma(av, __ldg(b + (int64_t)k * NN + n), acc[n]);
-    }
-#pragma unroll
-    for (int n = 0; n < NN; n++) {
-#pragma unroll
-      for (int o = 16; o > 0; o >>= 1) acc[n] += __shfl_xor_sync(0xffffffffu, acc[n], o);
-      if (lane == n) {
-        if (!LONG || t.grp < 0)
-          C[t.c_off + (int64_t)m * NN + n] = acc[n];
-        else
-          ws[t.ws_off + (int64_t)t.kq * t.gs + (m * NN + n - t.o0)] = acc[n];
-      }
-    }
+  int m = t.v0;
+  const int end = t.v0 + t.nv;
+  for (; m + RB <= end; m += RB) row_block<NN, RB, LONG>(t, m, lane, A, B, C, ws);
+  if (RB > 1)
+    for (; m < end; m++) row_block<NN, 1, LONG>(t, m, lane, A, B, C, ws);
+}
+
+template <bool LONG>
+__device__ __forceinline__ void row_dispatch(const FlatItem& t, int lane, const double* __restrict__ A,
+                                             const double* __restrict__ B, double* __restrict__ C,
+                                             double* __restrict__ ws) {
+  if (t.N == 1) return row_body<1, LONG>(t, lane, A, B, C, ws);
+  if (!LONG || t.N == 2) return row_body<2, LONG>(t, lane, A, B, C, ws);
+  switch (t.N) {  // small lists only (plan_fp64_flat)
+    case 3: return row_body<3, LONG>(t, lane, A, B, C, ws);
+    case 4: return row_body<4, LONG>(t, lane, A, B, C, ws);
+    case 5: return row_body<5, LONG>(t, lane, A, B, C, ws);
+    case 6: return row_body<6, LONG>(t, lane, A, B, C, ws);
+    case 7: return row_body<7, LONG>(t, lane, A, B, C, ws);
+    default: return row_body<8, LONG>(t, lane, A, B, C, ws);
   }
 }
 
@@ -253,9 +307,10 @@ __device__ __forceinline__ void view_dispatch(const FlatItem& t, int lane, const
 
 // VIEWS: some item reads an operand through views (a kernel of its own: with
 // its registers the plain one would hold 4 CTAs per SM instead of 5, 20% slower
-// on the batched workload).  LONG: some row is cut into K ranges, or some group
-// has more than kFlatFewRanges (a kernel of its own too: in one, lists without
-// such a sector ran 1% longer, the batched workload 5.93 -> 6.01 ms)
+// on the batched workload).  LONG: some row is cut into K ranges, some group has
+// more than kFlatFewRanges, or the list leaves warps idle, so that a group's sum
+// is seen (a kernel of its own too: in one, lists without such a sector ran 1%
+// longer, the batched workload 5.93 -> 6.01 ms)
 template <bool VIEWS, bool LONG>
 __global__ void __launch_bounds__(32 * kWarps, kFlatCtasPerSm)
     gemm_fp64_flat_kernel(const FlatItem* __restrict__ items, int nitems, const double* __restrict__ A,
@@ -268,10 +323,7 @@ __global__ void __launch_bounds__(32 * kWarps, kFlatCtasPerSm)
   for (int it = blockIdx.x * kWarps + warp; it < nitems; it += gridDim.x * kWarps) {
     const FlatItem t = items[it];
     if (t.rows) {
-      if (t.N == 1)
-        row_body<1, LONG>(t, lane, A, B, C, ws);
-      else
-        row_body<2, LONG>(t, lane, A, B, C, ws);
+      row_dispatch<LONG>(t, lane, A, B, C, ws);
       if (!LONG || t.grp < 0) continue;
     } else if (VIEWS && (t.a_vw >= 0 || t.b_vw >= 0))
       view_dispatch(t, lane, A, B, C, ws, views, pool);
@@ -287,22 +339,23 @@ __global__ void __launch_bounds__(32 * kWarps, kFlatCtasPerSm)
       if (__shfl_sync(0xffffffffu, last, 0)) {
         __threadfence();
         const double* p = ws + t.ws_off;
-        if (!LONG || t.go >= 32 || t.nsplit <= kFlatFewRanges) {
+        if (!LONG || t.go > 16 || t.nsplit <= 4) {
           for (int o = lane; o < t.go; o += 32) {
             double s = 0.0;
 #pragma unroll(LONG ? 8 : 1)
             for (int q = 0; q < t.nsplit; q++) s += __ldcg(p + (int64_t)q * t.gs + o);
             C[t.c_off + t.o0 + o] = s;
           }
-        } else {  // few outputs of many ranges: lanes along the ranges
-          for (int o = 0; o < t.go; o++) {
-            double s = 0.0;
+        } else {  // few outputs of many ranges: 32 / w lanes along the ranges of each
+          int w = 1;
+          while (w < t.go) w *= 2;
+          const int o = lane & (w - 1);
+          double s = 0.0;
+          if (o < t.go)
 #pragma unroll 8
-            for (int q = lane; q < t.nsplit; q += 32) s += __ldcg(p + (int64_t)q * t.gs + o);
-#pragma unroll
-            for (int d = 16; d > 0; d >>= 1) s += __shfl_xor_sync(0xffffffffu, s, d);
-            if (lane == 0) C[t.c_off + t.o0 + o] = s;
-          }
+            for (int q = lane / w; q < t.nsplit; q += 32 / w) s += __ldcg(p + (int64_t)q * t.gs + o);
+          for (int d = 16; d >= w; d >>= 1) s += __shfl_xor_sync(0xffffffffu, s, d);
+          if (lane < t.go) C[t.c_off + t.o0 + lane] = s;
         }
         if (lane == 0) counters[t.grp] = 0;  // for the next launch
       }
