@@ -159,17 +159,29 @@ static std::shared_ptr<TcPlan> build_tc_plan(Ctx& ctx, const std::vector<tn_sect
   if (!P->nsec) return P;
   // One pass over the operands, or maxima and images tile by tile in two launches
   // (also for a list whose items would not number in 32 bits).  The two launches
-  // read everything twice, tiles of 64 k at a time: about 36 us and 127 000
-  // elements a microsecond.  One pass lasts at least as long as its longest item,
-  // a quarter of a strip of 16 columns, whose CTA slices about 530 elements a
+  // read everything twice, tiles of 64 k at a time: 36 us, 400 000 elements a
+  // microsecond for the maxima and 270 000, those of the last tile's padding among
+  // them, for the images.  One pass takes 600 000 elements a microsecond and 0.70 ns
+  // for every row of A that is a warp's, 4.2 for every 16 columns of B: rows below
+  // about 120 k are not long enough for it.  Nor does it end before its longest
+  // item, a quarter of a strip of 16 columns, whose CTA slices about 530 elements a
   // microsecond beyond what it stages.  Measured in split precision, one pass and
-  // two launches: 484 x 484 over K = 10648 78 and 97 us, over K = 80000 601 and 623,
-  // 81 x 81 over K = 6561 101 (before strips were shared) and 29 us.
+  // two launches: 30e6 elements of A in rows of 16 k 1314 and 403 us, 64 339 and 179, 128
+  // 183 and 180, 200 146 and 237; 1e6 columns of 41 328 and 501; 484 x 484 over K = 10648 78
+  // and 97, over K = 80000 601 and 623, 81 x 81 over K = 6561 101 (before strips were
+  // shared) and 29.
   int64_t nsl = 0;
-  for (const auto& s : secs) nsl += cdiv(s.N, 16) + (s.K > kRowWarp ? s.M : cdiv(s.M, 8));
-  const double two_launches = 36 + P->in_bytes / 8 / 127e3, longest_item = 16.0 / kSliceCluster * P->max_k / 530;
+  double rows = 0, strips = 0, padded = 0;
+  for (const auto& s : secs) {
+    nsl += cdiv(s.N, 16) + (s.K > kRowWarp ? s.M : cdiv(s.M, 8));
+    rows += s.K > kRowWarp ? 0 : s.M;
+    strips += (double)cdiv(s.N, 16);
+    padded += ((double)s.M + s.N) * s.nkt * kTK;
+  }
+  const double elems = P->in_bytes / 8, two_launches = 36 + elems / 400e3 + padded / 270e3;
+  const double one_pass = std::max(rows * 0.70e-3 + strips * 4.2e-3 + elems / 600e3, 16.0 / kSliceCluster * P->max_k / 530);
   std::vector<int2> sitems;
-  if (nsl < INT32_MAX / 2 && longest_item <= two_launches) {
+  if (nsl < INT32_MAX / 2 && one_pass <= two_launches) {
     sitems.reserve(nsl);
     for (int g = 0; g < P->nsec; g++)
       if (secs[g].K > kSliceWideK)
