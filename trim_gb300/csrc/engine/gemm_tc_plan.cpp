@@ -165,7 +165,8 @@ static std::shared_ptr<TcPlan> build_tc_plan(Ctx& ctx, const std::vector<tn_sect
   // for every row of A that is a warp's, 4.2 for every 16 columns of B: rows below
   // about 120 k are not long enough for it.  Nor does it end before its longest
   // item, a quarter of a strip of 16 columns, whose CTA slices about 530 elements a
-  // microsecond beyond what it stages.  Measured in split precision, one pass and
+  // microsecond beyond what it stages; of operands of such a K the two launches take
+  // about 127 000 elements a microsecond in all.  Measured in split precision, one pass and
   // two launches: 30e6 elements of A in rows of 16 k 1314 and 403 us, 64 339 and 179, 128
   // 183 and 180, 200 146 and 237; 1e6 columns of 41 328 and 501; 484 x 484 over K = 10648 78
   // and 97, over K = 80000 601 and 623, 81 x 81 over K = 6561 101 (before strips were
@@ -178,10 +179,11 @@ static std::shared_ptr<TcPlan> build_tc_plan(Ctx& ctx, const std::vector<tn_sect
     strips += (double)cdiv(s.N, 16);
     padded += ((double)s.M + s.N) * s.nkt * kTK;
   }
-  const double elems = P->in_bytes / 8, two_launches = 36 + elems / 400e3 + padded / 270e3;
-  const double one_pass = std::max(rows * 0.70e-3 + strips * 4.2e-3 + elems / 600e3, 16.0 / kSliceCluster * P->max_k / 530);
+  const double elems = P->in_bytes / 8, longest_item = 16.0 / kSliceCluster * P->max_k / 530;
+  const bool once = longest_item <= 36 + elems / 127e3 &&
+                    rows * 0.70e-3 + strips * 4.2e-3 + elems / 600e3 <= 36 + elems / 400e3 + padded / 270e3;
   std::vector<int2> sitems;
-  if (nsl < INT32_MAX / 2 && one_pass <= two_launches) {
+  if (nsl < INT32_MAX / 2 && once) {
     sitems.reserve(nsl);
     for (int g = 0; g < P->nsec; g++)
       if (secs[g].K > kSliceWideK)
