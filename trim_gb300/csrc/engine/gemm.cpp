@@ -312,22 +312,6 @@ static bool flat_fits(const std::vector<tn_sector_gemm>& list) {
   return true;
 }
 
-// Sectors that the tiles fill: there a tile's 1.25 loads an FMA beat the flat
-// form's two by 4%, which a few empty lanes cost again (1889 x 887 x 590, 98% full, 1638 us
-// in tiles, 1708 flat; 802 x 2284 x 890, 97%, 2716 and 2810; two of 2048 x 648 x 648, 96%, 3.0
-// ms in tiles, 2.85 flat).
-static bool tiles_full(const std::vector<tn_sector_gemm>& list, int num_sms) {
-  double wanted = 0, padded = 0, tiles = 0;
-  for (const auto& g : list) {
-    if (g.M <= 0 || g.N <= 0 || g.K <= 0) continue;
-    const double t = std::ceil((double)g.M / 16) * std::ceil((double)g.N / 32);
-    wanted += (double)g.M * (double)g.N * (double)g.K;
-    padded += t * 512 * (double)g.K;
-    tiles += t;
-  }
-  return tiles >= 4.0 * num_sms && wanted >= 0.97 * padded;
-}
-
 struct Fp64Plan {
   DevBufP flat;  // FlatItem list (then no tiles)
   int nflat = 0;
@@ -372,7 +356,7 @@ static std::shared_ptr<Fp64Plan> get_fp64_plan(Ctx& ctx, const std::vector<tn_se
     P->vw = *vw;
     P->table = table;
   }
-  const bool flat = pol.flat && flat_fits(list) && (vw || !tiles_full(list, ctx.num_sms));
+  const bool flat = pol.flat && flat_fits(list);
   int64_t ngrp = 0;
   std::vector<FlatItem> items;
   std::vector<GemmTile> tiles;
