@@ -343,7 +343,6 @@ __global__ void __launch_bounds__(32 * kWarps, kFlatCtasPerSm)
         if (!LONG || t.go > 16 || t.nsplit <= 4) {
           for (int o = lane; o < t.go; o += 32) {
             double s = 0.0;
-#pragma unroll(LONG ? 8 : 1)
             for (int q = 0; q < t.nsplit; q++) s += __ldcg(p + (int64_t)q * t.gs + o);
             C[t.c_off + t.o0 + o] = s;
           }
