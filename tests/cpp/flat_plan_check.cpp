@@ -1,8 +1,9 @@
 // The FP64 grouped GEMM's flat work list on the host: flat_plan_check SMS
 // M N K [M N K ...] plans the list and walks it as the kernel does, checking
 // that every product is taken once and every index lies in its range; prints
-// the items, the partial sums (elements), the warp FMAs of the costliest item
-// and the most ranges that one warp adds up.
+// the items, the partial sums (elements), the warp FMAs of the costliest item,
+// the most ranges that one warp adds up and the most products of one sum (0 where
+// the kernel breaks them off at kFlatChain).
 #include <algorithm>
 #include <cstdio>
 #include <cstdlib>
@@ -28,8 +29,9 @@ int main(int argc, char** argv) {
     a += g.M * g.K, b += g.K * g.N, c += g.M * g.N;
     list.push_back(g);
   }
-  int64_t ws = 0, ngrp = 0, most_cost = 0, most_ranges = 0;
-  const std::vector<FlatItem> items = plan_fp64_flat(list, atoi(argv[1]), &ws, &ngrp);
+  int64_t ws = 0, ngrp = 0, most_cost = 0, most_ranges = 0, chain = 0;
+  int form = kFlatPlain;
+  const std::vector<FlatItem> items = plan_fp64_flat(list, atoi(argv[1]), &ws, &ngrp, &form);
   std::map<int64_t, int64_t> k_of;  // output -> products taken
   std::vector<int> arrived(ngrp, 0), cnt(ngrp, 0);
   const bool small = c < 100000;
@@ -43,6 +45,7 @@ int main(int argc, char** argv) {
       if (t.nv > 128) return bad("more entries than slots");
       most_cost = std::max<int64_t>(most_cost, (int64_t)((t.nv + 31) / 32) * std::min(t.kc, t.K));
     }
+    if (!t.rows && form != kFlatHuge) chain = std::max<int64_t>(chain, std::min(t.kc, t.K));
     if ((t.grp >= 0) != (t.nsplit > 1)) return bad("ranges without a group");
     if (t.grp >= 0) {
       if (t.grp >= ngrp) return bad("a group out of range");
@@ -71,6 +74,7 @@ int main(int argc, char** argv) {
     for (const auto& g : list)
       for (int64_t o = 0; o < g.M * g.N; o++)
         if (done[g.c_off + o] != g.K) return bad("a product left out or taken twice");
-  printf("ok %zu %lld %lld %lld\n", items.size(), (long long)ws, (long long)most_cost, (long long)most_ranges);
+  printf("ok %zu %lld %lld %lld %lld\n", items.size(), (long long)ws, (long long)most_cost, (long long)most_ranges,
+         (long long)chain);
   return 0;
 }

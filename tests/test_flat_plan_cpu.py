@@ -36,7 +36,7 @@ def test_rows_over_a_long_k(plan, shape):
     """No warp takes more than two items' share: twice a 24th of a
     sub-partition's (64 warp FMAs at least), or a 1024th of a row."""
     m, n, k = shape
-    items, _, cost, ranges = plan(shape)
+    items, _, cost, ranges, _ = plan(shape)
     share = m * n * k / 32 / (4 * SMS)
     assert cost <= max(2 * max(64, share / 24) + 5 * n, n * (k / 32 / 1024 + 2))
     assert items >= min(256, m * n * k // 4096) and ranges <= 1024
@@ -44,19 +44,21 @@ def test_rows_over_a_long_k(plan, shape):
 
 @pytest.mark.parametrize("shape", [(10, 10, 10 ** 6), (3, 4, 10 ** 6), (11, 11, 10 ** 8), (64, 1, 31)])
 def test_few_outputs(plan, shape):
-    _, ws, _, ranges = plan(shape)
+    _, ws, _, ranges, _ = plan(shape)
     most = max(256, 8192 // (shape[0] * shape[1]))
     assert ranges <= most and ws <= most * shape[0] * shape[1]
 
 
-@pytest.mark.parametrize("shapes", [[(2800, 2800, 10 ** 5)], [(2800, 2800, 10 ** 8)], [(400, 400, 10 ** 6)] * 20, [(130, 1, 10 ** 7), (1000, 1000, 50000)]])
+@pytest.mark.parametrize("shapes", [[(2800, 2800, 10 ** 5)], [(2800, 2800, 10 ** 8)], [(400, 400, 10 ** 6)] * 20, [(130, 1, 10 ** 7), (1000, 1000, 50000)], [(576, 576, 331776)], [(1000, 1000, 10 ** 5)], [(10, 10, 10 ** 5), (2000, 2000, 50000)]])
 def test_large_outputs_over_a_long_k(plan, shapes):
-    """Items: 96 a sub-partition and twice that for rounding, and the chunks of
-    128 outputs; partial sums: 128 to an item of a split chunk."""
-    items, ws, _, _ = plan(*shapes)
+    """Items: 768 a sub-partition and twice that for rounding, and the chunks of
+    128 outputs; partial sums: 128 to an item of a split chunk.  No sum of more than
+    4096 products that the kernel does not break off."""
+    items, ws, _, _, chain = plan(*shapes)
     chunks = sum(m * n // 128 + 1 for m, n, _ in shapes)
-    assert items <= 2 * 96 * 4 * SMS + 2 * chunks
-    assert ws <= 128 * 2 * 96 * 4 * SMS
+    assert items <= 2 * 768 * 4 * SMS + 2 * chunks
+    assert ws <= 128 * 2 * 768 * 4 * SMS
+    assert chain <= 4096
 
 
 @pytest.mark.parametrize("shapes", [[(1, 1, 562)], [(4, 4, 105)] * 2, [(3, 7, 14786)], [(4460, 1, 59)], [(281, 1, 55)] * 100, [(2, 39, 895)], [(9, 16, 320)] * 20])
@@ -64,7 +66,7 @@ def test_lists_that_leave_warps_idle(plan, shapes):
     """The longest item costs at most two of the least (64 warp FMAs), and a
     warp adds up no more ranges than the square root of K, or 8, unless the lanes
     run along them."""
-    items, _, cost, ranges = plan(*shapes)
+    items, _, cost, ranges, _ = plan(*shapes)
     m, n, k = shapes[0]
     assert cost <= 2 * 64
     assert ranges <= max(8, k ** 0.5) or n <= 8 or m * n >= 128

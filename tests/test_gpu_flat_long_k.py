@@ -39,3 +39,53 @@ def test_long_k(together):
             x, y = a[oa:oa + m * k].reshape(m, k), b[ob:ob + k * n].reshape(k, n)
             err = np.abs(outs[0][oc:oc + m * n].reshape(m, n) - x @ y)
             assert np.all(err <= 2 * (k + 1) * 2.0 ** -53 * (np.abs(x) @ np.abs(y))), (m, n, k)
+
+
+def test_sums_stay_short_in_large_lists():
+    """Equal products round the same way at every step, so a sum's error grows
+    with its length: with sums of 1024 products, and sums of those, it stays
+    within (1024 + K / 1024 + 256) 2^-53 (relative; 1.1 rounds to 1937 of these units
+    in sums of 13400).  Beside it few outputs, whose lanes hold several ranges, and
+    rows."""
+    torch = pytest.importorskip("torch")
+    if not torch.cuda.is_available():
+        pytest.skip("no CUDA device")
+    from fractions import Fraction
+    from trim_gb300 import uni10 as tu
+
+    tu.set_stream(torch.cuda.current_stream().cuda_stream)
+    gemms, ao, bo, co = [], 0, 0, 0
+    k = 100000
+    for m, n in [(1000, 1000), (9, 10), (3, 2)]:
+        gemms.append((m, n, k, ao, bo, co))
+        ao, bo, co = ao + m * k, bo + k * n, co + m * n
+    A = torch.ones(ao, dtype=torch.float64, device="cuda")
+    B = torch.full((bo,), 1.1, dtype=torch.float64, device="cuda")
+    C = torch.full((co,), float("nan"), dtype=torch.float64, device="cuda")
+    torch.cuda.synchronize()
+    tu.contract_sectors("fp64", gemms, A.data_ptr(), B.data_ptr(), C.data_ptr())
+    tu.sync()
+    want = Fraction(1.1) * k
+    worst = max(abs(Fraction(v) - want) / want for v in set(C.cpu().tolist()))
+    assert worst <= Fraction(1024 + k // 1024 + 256, 2 ** 53)
+
+
+def test_sums_stay_short_through_views():
+    """The same with A read through a view of its unpermuted source."""
+    torch = pytest.importorskip("torch")
+    if not torch.cuda.is_available():
+        pytest.skip("no CUDA device")
+    from fractions import Fraction
+    from trim_gb300 import uni10 as tu
+    from trim_gb300 import workloads as wl
+
+    tu.set_stream(torch.cuda.current_stream().cuda_stream)
+    m, n, k0, k1 = 800, 800, 2, 60000  # two segments of 60000 k where the view has them
+    a = tu.UniTensor([wl.dense_bond(wl.IN, m), wl.dense_bond(wl.IN, k0), wl.dense_bond(wl.IN, k1)], [0, 1, 2])
+    b = tu.UniTensor([wl.dense_bond(wl.IN, k0), wl.dense_bond(wl.IN, k1), wl.dense_bond(wl.OUT, n)], [1, 2, 3])
+    a.set_elem(np.ones(m * k0 * k1))
+    b.set_elem(np.full(n * k0 * k1, 1.1))
+    c = tu.contract(a, b).get_elem()
+    want = Fraction(1.1) * k0 * k1
+    worst = max(abs(Fraction(float(v)) - want) / want for v in set(c.tolist()))
+    assert worst <= Fraction(1024 + k0 * k1 // 1024 + 256, 2 ** 53)

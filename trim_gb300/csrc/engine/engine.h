@@ -237,6 +237,8 @@ struct FlatItem {
 constexpr int kFlatWarps = 4, kFlatCtasPerSm = 5;  // warps per CTA, CTAs an SM holds (registers)
 constexpr int kFlatSlots = 4, kFlatViewSlots = 2;  // slots per item, and with a view
 constexpr int kFlatFewRanges = 32;  // K ranges that the plain kernel adds up one after another
+constexpr int kFlatChain = 1024;    // products that one sum takes in the items of a huge list
+enum { kFlatPlain = 0, kFlatLong = 1, kFlatHuge = 2 };  // instances of the kernel (plan_fp64_flat)
 
 // Planning choices of the FP64 grouped GEMM (the autotuner's search space):
 // flat items, or tiles with a width rule (0: the
@@ -488,7 +490,8 @@ std::vector<GemmTile> plan_fp64(const std::vector<tn_sector_gemm>& list, int num
 // Flat work list: ws_elems / ngroups receive the partial sums' workspace and
 // the number of split groups; vw (may be null): (A view, B view) per sector.
 std::vector<FlatItem> plan_fp64_flat(const std::vector<tn_sector_gemm>& list, int num_sms, int64_t* ws_elems,
-                                     int64_t* ngroups, const std::vector<std::pair<int, int>>* vw = nullptr);
+                                     int64_t* ngroups, int* form,
+                                     const std::vector<std::pair<int, int>>* vw = nullptr);
 
 // kernel launchers (defined in the .cu files); device: the context's
 // fourth_dim: some tile has a fourth dim
@@ -503,10 +506,9 @@ void launch_permute_kernel(int device, const PermSub* subs, const int64_t* tile_
 void launch_gemm_fp64(const GemmTile* tiles, int ntiles, const double* A, const double* B, double* C,
                       double* ws, int* counters, const ViewHdr* views, const int64_t* pool, int grid,
                       cudaStream_t s, bool dependent_launch = true);
-// long_k: some item is a row over a part of K or of a group of more than
-// kFlatFewRanges, or the list has fewer items than the GPU holds warps
+// form: from the planner (plan_fp64_flat)
 void launch_gemm_fp64_flat(const FlatItem* items, int nitems, const double* A, const double* B, double* C, double* ws,
-                           int* counters, const ViewHdr* views, const int64_t* pool, bool long_k, int grid,
+                           int* counters, const ViewHdr* views, const int64_t* pool, int form, int grid,
                            cudaStream_t s);
 void launch_splitk_reduce(const GemmTile* tiles, int ntiles, const double* ws, double* C, int grid,
                           cudaStream_t s);

@@ -152,8 +152,9 @@ std::vector<GemmTile> plan_fp64(const std::vector<tn_sector_gemm>& list, int num
 // Flat items.  Cost is counted in warp FMAs (slots x K): an SM sub-partition
 // runs one at a time, so items are cut to about a 24th of its share (at
 // least 64 warp FMAs, below which an item's own latency shows; at most 4096, or
-// a 96th of the share where that is more: a list of 8e9 multiply-adds and up
-// would only grow, items and partial sums by the gigabyte).
+// a 768th of the share where that is more: a list of 6e10 multiply-adds and up
+// would only grow, items and partial sums by gigabytes; the kernel sums such an
+// item's K range kFlatChain products at a time, so that sums stay short).
 // (Sixteenths were up to 7% slower, on 64 uneven contractions 404 -> 376 us, an
 // iPEPS quadrant at chi = 48, D = 5 460 -> 448; 48ths up to 6% faster still on some
 // lists and 2% slower on others.)
@@ -167,10 +168,13 @@ std::vector<GemmTile> plan_fp64(const std::vector<tn_sector_gemm>& list, int num
 // one costs two items; with a whole row to a warp 1 x 1 over K = 1e6 took one warp
 // 31 250 steps.  An item that reads an operand through views walks its K range in
 // the views' segments, so its entries share one range.
+// *form: the kernel's instance, kFlatLong for rows over a part of K, groups of more
+// than kFlatFewRanges and lists that leave warps idle, kFlatHuge for those items.
 constexpr double kFlatFloor = 64.0;   // warp FMAs of an item, at least
 constexpr int64_t kRowRanges = 1024;  // K ranges of a row: two for every resident warp of half the chip
 std::vector<FlatItem> plan_fp64_flat(const std::vector<tn_sector_gemm>& list, int num_sms, int64_t* ws_elems,
-                                     int64_t* ngroups, const std::vector<std::pair<int, int>>* vw) {
+                                     int64_t* ngroups, int* form,
+                                     const std::vector<std::pair<int, int>>* vw) {
   auto row_cost = [](int64_t n, int64_t k) { return n * ((k + 31) / 32 + 5); };  // warp FMAs, and 5 to sum the lanes
   auto viewed = [&](size_t gi) { return vw && ((*vw)[gi].first >= 0 || (*vw)[gi].second >= 0); };
   double total = 0, rows8 = 0;
@@ -182,7 +186,7 @@ std::vector<FlatItem> plan_fp64_flat(const std::vector<tn_sector_gemm>& list, in
     if (rows && g.N <= 8) rows8 += (double)g.M;
   }
   const double share = total / (4.0 * num_sms);
-  const int64_t target = (int64_t)std::min(std::max(4096.0, share / 96.0), std::max(kFlatFloor, share / 24.0));
+  const int64_t target = (int64_t)std::min(std::max(4096.0, share / 768.0), std::max(kFlatFloor, share / 24.0));
   // A list so small that items are at their least leaves warps idle and lasts as
   // long as its longest item: up to 8 columns are rows there (a lane's chain is K /
   // 32 long, not K), and no more rows to an item than leave every resident warp one.
@@ -288,16 +292,21 @@ std::vector<FlatItem> plan_fp64_flat(const std::vector<tn_sector_gemm>& list, in
   }
   *ws_elems = ws;
   *ngroups = ngrp;
+  *form = (int64_t)out.size() <= warps ? kFlatLong : kFlatPlain;
+  for (const auto& t : out)
+    if (!t.rows && target > 4096 && t.kc > kFlatChain)
+      *form = kFlatHuge;
+    else if (*form == kFlatPlain && (t.nsplit > kFlatFewRanges || (t.rows && (t.nsplit > 1 || t.N > 2))))
+      *form = kFlatLong;
   // the warps of a CTA take kWarps consecutive items; with more items than the
   // grid holds at once, costly ones first, in bands alternately reversed, as
   // for the tiles above
-  const int64_t grid_items = (int64_t)num_sms * kFlatCtasPerSm * kFlatWarps;
-  if ((int64_t)out.size() <= grid_items) return out;
+  if ((int64_t)out.size() <= warps) return out;
   auto cost = [&](const FlatItem& t) {
     return t.rows ? t.nv * row_cost(t.N, std::min(t.kc, t.K)) : (int64_t)((t.nv + 31) / 32) * std::min(t.kc, t.K);
   };
   std::stable_sort(out.begin(), out.end(), [&](const FlatItem& a, const FlatItem& b) { return cost(a) > cost(b); });
-  const size_t band = (size_t)grid_items;
+  const size_t band = (size_t)warps;
   for (size_t b0 = band; b0 < out.size(); b0 += 2 * band)
     std::reverse(out.begin() + b0, out.begin() + std::min(out.size(), b0 + band));
   return out;
@@ -315,7 +324,7 @@ static bool flat_fits(const std::vector<tn_sector_gemm>& list) {
 struct Fp64Plan {
   DevBufP flat;  // FlatItem list (then no tiles)
   int nflat = 0;
-  bool long_k = false;
+  int form = kFlatPlain;
   std::vector<tn_sector_gemm> list;
   std::vector<std::pair<int, int>> vw;  // operand view ids per sector (empty: contiguous operands)
   const void* table = nullptr;          // the view table the ids index
@@ -361,10 +370,8 @@ static std::shared_ptr<Fp64Plan> get_fp64_plan(Ctx& ctx, const std::vector<tn_se
   std::vector<FlatItem> items;
   std::vector<GemmTile> tiles;
   if (flat) {
-    items = plan_fp64_flat(list, ctx.num_sms, &P->ws_elems, &ngrp, vw);
+    items = plan_fp64_flat(list, ctx.num_sms, &P->ws_elems, &ngrp, &P->form, vw);
     P->nflat = (int)items.size();
-    P->long_k = P->nflat <= ctx.num_sms * kFlatCtasPerSm * kFlatWarps;
-    for (const auto& t : items) P->long_k |= t.nsplit > kFlatFewRanges || (t.rows && (t.nsplit > 1 || t.N > 2));
   } else {
     tiles = plan_fp64_split(list, ctx.num_sms, true, &P->ws_elems, pol, vw);
     for (const auto& t : tiles) ngrp = std::max<int64_t>(ngrp, (int64_t)t.grp + 1);
@@ -407,7 +414,7 @@ static void launch_fp64_plan(Ctx& ctx, const Fp64Plan& P, const double* A, const
     grid = (int)std::min<int64_t>(((int64_t)P.nflat + kFlatWarps - 1) / kFlatWarps,
                                   (int64_t)ctx.num_sms * kFlatCtasPerSm);
     launch_gemm_fp64_flat((const FlatItem*)P.flat->ptr, P.nflat, A, B, C, ws,
-                          P.counters ? (int*)P.counters->ptr : nullptr, views, pool, P.long_k, grid, ctx.stream);
+                          P.counters ? (int*)P.counters->ptr : nullptr, views, pool, P.form, grid, ctx.stream);
     ctx.launched();
   } else {
     // split tiles are summed by the last CTA of each group (no second launch)

@@ -83,10 +83,28 @@ __device__ __forceinline__ void fma_run(double (&acc)[R], const double* const (&
     }
 }
 
+// fma_run over a long range, kFlatChain products to a sum
+template <int R>
+__device__ __forceinline__ void fma_long(double (&acc)[R], const double* const (&pa)[R], const double* (&pb)[R],
+                                         const int64_t (&ldb)[R], int len) {
+  for (int k = 0; k < len; k += kFlatChain) {
+    const double* pk[R];
+    double part[R];
+#pragma unroll
+    for (int i = 0; i < R; i++) {
+      pk[i] = pa[i] + k;
+      part[i] = 0.0;
+    }
+    fma_run<R>(part, pk, pb, ldb, min(kFlatChain, len - k));
+#pragma unroll
+    for (int i = 0; i < R; i++) acc[i] += part[i];
+  }
+}
+
 // Operands read through views of their unpermuted source (ViewHdr): the K range
 // is walked in segments (the contracted bonds' charge tuples), each a plain
 // row-major view per row (column) tuple.
-template <int R>
+template <int R, bool HUGE>
 __device__ __forceinline__ void view_body(const FlatItem& t, int lane, const double* __restrict__ A,
                                           const double* __restrict__ B, double* __restrict__ C,
                                           double* __restrict__ ws, const ViewHdr* __restrict__ views,
@@ -107,13 +125,13 @@ __device__ __forceinline__ void view_body(const FlatItem& t, int lane, const dou
   const int64_t* seg = av ? pool + av->cs : pool + bv->rs;
   const int nseg = av ? av->nc : bv->nr;
   const int kb = slice * t.kc, ke = min(t.K, kb + t.kc);
-  double acc[R];
+  double acc[R], sum[R];
 #pragma unroll
-  for (int i = 0; i < R; i++) acc[i] = 0.0;
+  for (int i = 0; i < R; i++) acc[i] = sum[i] = 0.0;
   int s = find_start(seg, nseg, kb);
   pdl_wait();  // A, B, C and ws may be written by the previous grid
-  for (int k0 = kb; k0 < ke; s++) {
-    const int s0 = (int)seg[s], k1 = (int)min((int64_t)ke, seg[s + 1]);
+  for (int k0 = kb, chain0 = kb; k0 < ke;) {
+    const int s0 = (int)seg[s], s1 = (int)min((int64_t)ke, seg[s + 1]), k1 = HUGE ? min(s1, chain0 + kFlatChain) : s1;
     const double *pa[R], *pb[R];
     int64_t ldb[R];
 #pragma unroll
@@ -135,7 +153,19 @@ __device__ __forceinline__ void view_body(const FlatItem& t, int lane, const dou
     }
     fma_run<R>(acc, pa, pb, ldb, k1 - k0);
     k0 = k1;
+    s += k1 == s1;
+    if (HUGE && k1 == chain0 + kFlatChain) {  // short segments share a sum
+#pragma unroll
+      for (int i = 0; i < R; i++) {
+        sum[i] += acc[i];
+        acc[i] = 0.0;
+      }
+      chain0 = k1;
+    }
   }
+  if (HUGE)
+#pragma unroll
+    for (int i = 0; i < R; i++) acc[i] += sum[i];
 #pragma unroll
   for (int i = 0; i < R; i++)
     if (lane + 32 * i < t.nv) {
@@ -147,7 +177,7 @@ __device__ __forceinline__ void view_body(const FlatItem& t, int lane, const dou
 }
 
 // R slots of 32 entries; UNI: all entries of the item in one K range
-template <int R, bool UNI>
+template <int R, bool UNI, bool HUGE>
 __device__ __forceinline__ void flat_body(const FlatItem& t, int lane, const double* __restrict__ A,
                                           const double* __restrict__ B, double* __restrict__ C,
                                           double* __restrict__ ws) {
@@ -173,10 +203,16 @@ __device__ __forceinline__ void flat_body(const FlatItem& t, int lane, const dou
   for (int i = 0; i < R; i++) ldb[i] = t.N;
   pdl_wait();  // A, B, C and ws may be written by the previous grid
   if (UNI) {
-    fma_run<R>(acc, pa, pb, ldb, len[0]);
+    if (HUGE)
+      fma_long<R>(acc, pa, pb, ldb, len[0]);
+    else
+      fma_run<R>(acc, pa, pb, ldb, len[0]);
   } else {  // the last K range may be shorter
     const int kmin = min(t.kc, t.K - (int)((uint32_t)(t.v0 + t.nv - 1) / (uint32_t)t.mn) * t.kc);
-    fma_run<R>(acc, pa, pb, ldb, kmin);
+    if (HUGE)
+      fma_long<R>(acc, pa, pb, ldb, kmin);
+    else
+      fma_run<R>(acc, pa, pb, ldb, kmin);
     for (int k = kmin; k < t.kc; k++) {
 #pragma unroll
       for (int i = 0; i < R; i++) {
@@ -284,26 +320,27 @@ __device__ __forceinline__ void row_dispatch(const FlatItem& t, int lane, const 
   }
 }
 
-template <bool UNI>
+template <bool UNI, bool HUGE>
 __device__ __forceinline__ void flat_dispatch(const FlatItem& t, int lane, const double* __restrict__ A,
                                               const double* __restrict__ B, double* __restrict__ C,
                                               double* __restrict__ ws) {
   switch ((t.nv + 31) >> 5) {
-    case 1: flat_body<1, UNI>(t, lane, A, B, C, ws); break;
-    case 2: flat_body<2, UNI>(t, lane, A, B, C, ws); break;
-    case 3: flat_body<3, UNI>(t, lane, A, B, C, ws); break;
-    default: flat_body<4, UNI>(t, lane, A, B, C, ws); break;
+    case 1: flat_body<1, UNI, HUGE>(t, lane, A, B, C, ws); break;
+    case 2: flat_body<2, UNI, HUGE>(t, lane, A, B, C, ws); break;
+    case 3: flat_body<3, UNI, HUGE>(t, lane, A, B, C, ws); break;
+    default: flat_body<4, UNI, HUGE>(t, lane, A, B, C, ws); break;
   }
 }
 
+template <bool HUGE>
 __device__ __forceinline__ void view_dispatch(const FlatItem& t, int lane, const double* __restrict__ A,
                                               const double* __restrict__ B, double* __restrict__ C,
                                               double* __restrict__ ws, const ViewHdr* __restrict__ views,
                                               const int64_t* __restrict__ pool) {
   if (t.nv <= 32)  // the planner gives these items at most kFlatViewSlots = 2 slots
-    view_body<1>(t, lane, A, B, C, ws, views, pool);
+    view_body<1, HUGE>(t, lane, A, B, C, ws, views, pool);
   else
-    view_body<2>(t, lane, A, B, C, ws, views, pool);
+    view_body<2, HUGE>(t, lane, A, B, C, ws, views, pool);
 }
 
 // VIEWS: some item reads an operand through views (a kernel of its own: with
@@ -311,8 +348,12 @@ __device__ __forceinline__ void view_dispatch(const FlatItem& t, int lane, const
 // on the batched workload).  LONG: some row is cut into K ranges, some group has
 // more than kFlatFewRanges, or the list leaves warps idle, so that a group's sum
 // is seen (a kernel of its own too: in one, lists without such a sector ran 1%
-// longer, the batched workload 5.93 -> 6.01 ms)
-template <bool VIEWS, bool LONG>
+// longer, the batched workload 5.93 -> 6.01 ms).  HUGE: a list of 6e10
+// multiply-adds and up with K ranges of more than kFlatChain, which are summed
+// kFlatChain products at a time: with one sum to a range the relative error of 576
+// x 576 over K = 331776 was 1.2e-15 -> 1.5e-14, now 1.0e-15 in the same 203 ms (in
+// the LONG instance the breaks cost 100 x 300 over 20000 4%).
+template <bool VIEWS, bool LONG, bool HUGE>
 __global__ void __launch_bounds__(32 * kWarps, kFlatCtasPerSm)
     gemm_fp64_flat_kernel(const FlatItem* __restrict__ items, int nitems, const double* __restrict__ A,
                           const double* __restrict__ B, double* __restrict__ C, double* __restrict__ ws,
@@ -327,11 +368,11 @@ __global__ void __launch_bounds__(32 * kWarps, kFlatCtasPerSm)
       row_dispatch<LONG>(t, lane, A, B, C, ws);
       if (!LONG || t.grp < 0) continue;
     } else if (VIEWS && (t.a_vw >= 0 || t.b_vw >= 0))
-      view_dispatch(t, lane, A, B, C, ws, views, pool);
+      view_dispatch<HUGE>(t, lane, A, B, C, ws, views, pool);
     else if (t.v0 / t.mn == (t.v0 + t.nv - 1) / t.mn)
-      flat_dispatch<true>(t, lane, A, B, C, ws);
+      flat_dispatch<true, HUGE>(t, lane, A, B, C, ws);
     else
-      flat_dispatch<false>(t, lane, A, B, C, ws);
+      flat_dispatch<false, HUGE>(t, lane, A, B, C, ws);
     if (t.grp >= 0) {
       __threadfence();  // this lane's partial sums are visible device-wide
       __syncwarp();
@@ -366,11 +407,15 @@ __global__ void __launch_bounds__(32 * kWarps, kFlatCtasPerSm)
 }  // namespace
 
 void launch_gemm_fp64_flat(const FlatItem* items, int nitems, const double* A, const double* B, double* C, double* ws,
-                           int* counters, const ViewHdr* views, const int64_t* pool, bool long_k, int grid,
+                           int* counters, const ViewHdr* views, const int64_t* pool, int form, int grid,
                            cudaStream_t s) {
   if (nitems <= 0) return;
-  auto kernel = views ? (long_k ? gemm_fp64_flat_kernel<true, true> : gemm_fp64_flat_kernel<true, false>)
-                      : (long_k ? gemm_fp64_flat_kernel<false, true> : gemm_fp64_flat_kernel<false, false>);
+  auto kernel = views ? (form == kFlatHuge   ? gemm_fp64_flat_kernel<true, true, true>
+                         : form == kFlatLong ? gemm_fp64_flat_kernel<true, true, false>
+                                             : gemm_fp64_flat_kernel<true, false, false>)
+                      : (form == kFlatHuge   ? gemm_fp64_flat_kernel<false, true, true>
+                         : form == kFlatLong ? gemm_fp64_flat_kernel<false, true, false>
+                                             : gemm_fp64_flat_kernel<false, false, false>);
   launch_pdl(kernel, dim3(grid), dim3(32 * kWarps), 0, s, items, nitems, A, B, C, ws, counters, views, pool);
 }
 
